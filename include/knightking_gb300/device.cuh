@@ -37,6 +37,9 @@ struct GraphView
      * vertex cursor}, so a uniform pick yields the next vertex and where its
      * adjacency lies in one 16 B read */
     const uint4 *adjc = nullptr;
+    /* the offsets as 32-bit words (a graph of fewer than 2^32 edges; nullptr:
+     * read off), the copy the walks' random reads go to */
+    const uint32_t *off32 = nullptr;
 };
 
 /* An edge as the hooks see it (AdjUnit, include/graph.hpp:49-61): its
@@ -145,6 +148,21 @@ struct Sampler
         step = s;
         stream = st;
         draw = 0;
+    }
+
+    /* enter() with the step's first block computed now: a walk that knows it
+     * will draw evaluates the next step's block while this step's reads are
+     * in flight (the block depends on the walker and the step only) */
+    __device__ __forceinline__ void prime(walker_id_t w, step_t s, uint32_t st)
+    {
+        enter(w, s, st);
+        buf = philox4x32_10(make_uint4(w, s, 0u, st), k0, k1);
+    }
+    /* word() of a step entered by prime(), for its first four draws */
+    __device__ __forceinline__ uint32_t primed_word()
+    {
+        const uint32_t slot = draw++;
+        return slot == 0 ? buf.x : (slot == 1 ? buf.y : (slot == 2 ? buf.z : buf.w));
     }
 
     __device__ __forceinline__ uint32_t word()

@@ -41,6 +41,7 @@ void kk_engine::free_graph()
     vcur_valid = false;
     edge_set_valid = false;
     adjc_valid = false;
+    off32_valid = false;
     dead_ends_valid = false;
     alias_cached = -1;
     n_hub = n_nz = 0;
@@ -734,6 +735,7 @@ void kk_engine_destroy(kk_engine *e)
     e->order.release();
     e->rows.release();
     e->adjc.release();
+    e->off32.release();
     if (e->h_status)
         cudaFreeHost(e->h_status);
     for (int r = 0; r < kk_engine::kReaders; r++)
@@ -852,6 +854,8 @@ kk_status kk_engine_set_option(kk_engine *e, const char *name, int64_t value)
             e->into_stream = (int)value;
         else if (n == "cursor_adjacency" && (value == 0 || value == 1))
             e->cursor_adjacency = (int)value;
+        else if (n == "compact_offsets" && (value == 0 || value == 1))
+            e->compact_offsets = (int)value;
         else if (n == "alias_hub_grid" && value >= 0 && value <= 4096)
             e->alias_hub_grid = (int)value;
         else if (n == "walk_park" && value >= 0 && value <= 32)

@@ -176,6 +176,17 @@ __global__ void deg_to_u64_kernel(const unsigned int *deg, uint64_t *out, uint32
 
 } // namespace
 
+void graph_offsets32(kk_engine *e)
+{
+    if (e->E > 0xffffffffull)
+        return;
+    uint32_t *o = e->off32.as<uint32_t>((uint64_t)e->V + 1);
+    offsets32_kernel<<<grid_for(e, (uint64_t)e->V + 1, 256), 256, 0, e->stream>>>(e->d_off, e->V, o);
+    count_launch(e);
+    KK_CUDA_CHECK(cudaGetLastError());
+    e->off32_valid = true;
+}
+
 const uint32_t *vertex_order(kk_engine *e)
 {
     if (e->order_valid)
@@ -400,9 +411,10 @@ void graph_upload(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, cons
         KK_CUDA_CHECK(cudaMalloc(&e->d_type, E + 4));
         KK_CUDA_CHECK(cudaMemcpyAsync(e->d_type, type, E, cudaMemcpyHostToDevice, e->stream));
     }
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->V = V;
     e->E = E;
+    graph_offsets32(e);
+    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->has_graph = true;
     e->sorted = -1;
 }
@@ -558,9 +570,10 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
                                                                              weighted ? e->d_w : nullptr);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->V = V;
     e->E = m;
+    graph_offsets32(e);
+    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->has_graph = true;
     e->sorted = -1;
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -632,9 +645,10 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->V = V;
     e->E = m;
+    graph_offsets32(e);
+    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->has_graph = true;
     e->sorted = -1;
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1088,13 +1102,14 @@ void graph_generate_rmat(kk_engine *e, uint32_t scale, uint32_t ef, double a, do
     count_launch(e);
     KK_CUDA_CHECK(cudaMalloc(&e->d_off, ((size_t)V + 1) * 8));
     exclusive_scan_u64(e, deg64, (uint64_t *)e->d_off, (uint64_t)V + 1);
+    e->V = V;
+    e->E = E;
+    graph_offsets32(e);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     cudaFree(mir_sorted);
     cudaFree(deg);
     cudaFree(deg64);
     cudaFree(d_count);
-    e->V = V;
-    e->E = E;
     e->has_graph = true;
     e->sorted = 1;
 }
