@@ -19,6 +19,7 @@ namespace apps
 template <typename S>
 struct FixedLengthExt
 {
+    static constexpr bool any_vertex = true;
     step_t walk_length;
     __device__ __forceinline__ real_t operator()(const Walker<S> &w, vertex_id_t) const
     {
@@ -122,7 +123,8 @@ struct Node2vecRespond
     {
         if (set.keys != nullptr)
         {
-            resp = edge_set_slot(set, target, query) != ~0ull;
+            const int64_t e0 = gather(set.off + target);
+            resp = edge_set_find(set, target, e0, (uint32_t)(gather(set.off + target + 1) - e0), query, nullptr);
             return;
         }
         uint32_t deg = adj.degree();
@@ -155,38 +157,20 @@ struct Node2vecDyn
  * overflow * w(return edge) (weighted), one outlier.  Where the previous
  * vertex is not a neighbour (directed graphs) the reference reads past the
  * adjacency; here the area is empty. */
-/* The return edge std::lower_bound(N(v), x) of node2vec.hpp:71-78 / :91-97:
- * its local index i (deg if none) and, when want_weight, its weight.  x = 0
- * (the value-initialised state of step 0) is at or below every neighbour, so
- * its position is 0 with no lookup; a neighbour x comes from the edge set,
- * index and weight in one access; anything else by binary search. */
-__device__ __forceinline__ uint32_t n2v_return_edge(const uint32_t *nbr, const float *w, const EdgeSetView &set,
-                                                    vertex_id_t v, const AdjList &adj, vertex_id_t x, bool want_weight,
-                                                    float &weight, bool &is_x)
+/* The weight of the return edge std::lower_bound(N(v), x) of
+ * node2vec.hpp:71-78; false where there is none.  x = 0 (the value-initialised
+ * state of step 0) is at or below every neighbour, so it is the first edge; a
+ * neighbour x's comes from the edge set; anything else by binary search. */
+__device__ __forceinline__ bool n2v_return_weight(const uint32_t *nbr, const float *w, const EdgeSetView &set,
+                                                  vertex_id_t v, const AdjList &adj, vertex_id_t x, float &weight)
 {
     const uint32_t deg = adj.degree();
-    uint32_t i;
-    is_x = false;
-    if (x == 0)
-    {
-        i = 0;
-    }
-    else
-    {
-        if (set.keys != nullptr)
-        {
-            uint32_t pos;
-            if (edge_set_find(set, v, x, pos, weight))
-            {
-                is_x = true; /* the edge at pos leads to x */
-                return pos;
-            }
-        }
-        i = lower_bound_adj(nbr, adj.begin, deg, x);
-    }
-    if (want_weight && i < deg)
+    if (x != 0 && set.keys != nullptr && edge_set_find(set, v, (int64_t)adj.begin, deg, x, &weight))
+        return true;
+    const uint32_t i = x == 0 ? 0 : lower_bound_adj(nbr, adj.begin, deg, x);
+    if (i < deg)
         weight = gather(w + adj.begin + i);
-    return i;
+    return i < deg;
 }
 
 template <bool Weighted>
@@ -210,9 +194,7 @@ struct Node2vecOutlierUB
                 return;
             }
             float rw = 0.0f;
-            bool is_x;
-            const uint32_t i = n2v_return_edge(nbr, w, set, v, adj, wk.data.previous_vertex, true, rw, is_x);
-            area = i < adj.degree() ? fmul(rw, overflow) : 0.0f;
+            area = n2v_return_weight(nbr, w, set, v, adj, wk.data.previous_vertex, rw) ? fmul(rw, overflow) : 0.0f;
         }
         else
         {
@@ -225,17 +207,15 @@ struct Node2vecOutlierUB
 struct Node2vecOutlierSearch
 {
     const uint32_t *nbr;
-    EdgeSetView set;
-    __device__ __forceinline__ bool operator()(const Walker<Node2vecState> &wk, vertex_id_t v, const AdjList &adj,
+    __device__ __forceinline__ bool operator()(const Walker<Node2vecState> &wk, vertex_id_t, const AdjList &adj,
                                                vertex_id_t, AdjUnit &out) const
     {
-        float unused = 0.0f;
-        bool is_x;
+        const uint32_t deg = adj.degree();
         const vertex_id_t x = wk.data.previous_vertex;
-        const uint32_t i = n2v_return_edge(nbr, nullptr, set, v, adj, x, false, unused, is_x);
-        if (i >= adj.degree())
+        const uint32_t i = x == 0 ? 0 : lower_bound_adj(nbr, adj.begin, deg, x);
+        if (i >= deg)
             return false;
-        out = AdjUnit{is_x ? x : gather(nbr + adj.begin + i), adj.begin + i};
+        out = AdjUnit{gather(nbr + adj.begin + i), adj.begin + i};
         return true;
     }
 };
@@ -281,6 +261,7 @@ struct MetaSchemes
 /* extension: 0 at the length or when no out-edge has an allowed type (metapath.hpp:102-105) */
 struct MetapathExt
 {
+    static constexpr bool any_vertex = true;
     const uint8_t *vertex_mask;
     step_t walk_length;
     const MetaSchemes *sc;
@@ -392,7 +373,7 @@ struct Node2vecBatch
         tc.dcomp_upperbound = ConstBound{j.c[0]};
         tc.dcomp_lowerbound = ConstBound{j.c[1]};
         tc.outlier_upperbound = Node2vecOutlierUB<Weighted>{nbr, w, j.c[2], set};
-        tc.outlier_search = Node2vecOutlierSearch{nbr, set};
+        tc.outlier_search = Node2vecOutlierSearch{nbr};
     }
 };
 

@@ -135,6 +135,7 @@ struct Sampler
     uint32_t k0, k1;
     uint32_t walker, step, stream, draw;
     uint4 buf;
+    bool fresh; /* draw & 3 == 0, and buf holds that draw's block already */
 
     __device__ __forceinline__ void init(uint64_t seed)
     {
@@ -148,6 +149,12 @@ struct Sampler
         step = s;
         stream = st;
         draw = 0;
+        fresh = false;
+    }
+
+    __device__ __forceinline__ void block()
+    {
+        buf = philox4x32_10(make_uint4(walker, step, draw >> 2, stream), k0, k1);
     }
 
     /* enter() with the step's first block computed now: a walk that knows it
@@ -156,7 +163,8 @@ struct Sampler
     __device__ __forceinline__ void prime(walker_id_t w, step_t s, uint32_t st)
     {
         enter(w, s, st);
-        buf = philox4x32_10(make_uint4(w, s, 0u, st), k0, k1);
+        block();
+        fresh = true;
     }
     /* word() of a step entered by prime(), for its first four draws */
     __device__ __forceinline__ uint32_t primed_word()
@@ -167,13 +175,41 @@ struct Sampler
 
     __device__ __forceinline__ uint32_t word()
     {
-        uint32_t slot = draw & 3u;
-        if (slot == 0)
-        {
-            buf = philox4x32_10(make_uint4(walker, step, draw >> 2, stream), k0, k1);
-        }
+        const uint32_t slot = draw & 3u;
+        if (slot == 0 && !fresh)
+            block();
+        fresh = false;
         draw++;
         return slot == 0 ? buf.x : (slot == 1 ? buf.y : (slot == 2 ? buf.z : buf.w));
+    }
+
+    /* The next four words without drawing them, from one evaluation of the
+     * generator: a rejection trial draws at most four, and asking for them one
+     * by one makes a warp whose lanes stand at different draws evaluate the
+     * generator at each of them.  nxt: for take(). */
+    __device__ __forceinline__ uint4 quad(uint4 &nxt)
+    {
+        const uint32_t slot = draw & 3u;
+        if (slot != 0 || !fresh)
+            nxt = philox4x32_10(make_uint4(walker, step, (draw + 3u) >> 2, stream), k0, k1);
+        if (slot == 0 && !fresh)
+        {
+            buf = nxt;
+            fresh = true;
+        }
+        const bool s1 = slot & 1u, s2 = slot & 2u;
+        const uint32_t a0 = s1 ? buf.y : buf.x, a1 = s1 ? buf.z : buf.y, a2 = s1 ? buf.w : buf.z,
+                       a3 = s1 ? nxt.x : buf.w, a4 = s1 ? nxt.y : nxt.x, a5 = s1 ? nxt.z : nxt.y;
+        return make_uint4(s2 ? a2 : a0, s2 ? a3 : a1, s2 ? a4 : a2, s2 ? a5 : a3);
+    }
+    /* Draws n (at most four) of the words quad() returned. */
+    __device__ __forceinline__ void take(uint32_t n, const uint4 &nxt)
+    {
+        const uint32_t slot = draw & 3u;
+        draw += n;
+        if (slot != 0 && slot + n >= 4u)
+            buf = nxt;
+        fresh = (draw & 3u) == 0 && (slot != 0 || n == 0);
     }
 
     __device__ __forceinline__ uint32_t gen(uint32_t ub) { return map_gen(word(), ub); }

@@ -22,6 +22,7 @@
 
 #include "knightking_gb300.h"
 #include "knightking_gb300/apps.cuh"
+#include "knightking_gb300/node2vec_walk.cuh"
 
 namespace kk
 {
@@ -372,8 +373,7 @@ struct kk_engine
     /* node2vec adjacency test: 0 edge set (built once per graph), 1 binary
      * search of the sorted adjacency (option node2vec_adjacency) */
     int n2v_adjacency = 0;
-    kk::DevBuf edge_set;
-    uint64_t edge_set_nb = 0;
+    kk::DevBuf edge_set, edge_set_w; /* the rows' ids and their weights */
     bool edge_set_valid = false;
     kk::DevBuf schemes;    /* metapath schemes of the running job */
     kk::BatchSlot bslot;   /* where the synchronous batch calls run */
@@ -549,6 +549,8 @@ bool graph_no_dead_ends(kk_engine *e);
  * empty view when the engine's node2vec_adjacency option asks for binary
  * search. */
 EdgeSetView node2vec_edge_set(kk_engine *e);
+/* The same for an engine that has built it (batch_prepare). */
+EdgeSetView node2vec_edge_set_built(const kk_engine *e);
 
 /* Per-vertex OR of 1 << edge type (metapath.hpp:77-88), cached per graph. */
 const uint8_t *metapath_vertex_masks(kk_engine *e);
@@ -841,6 +843,24 @@ void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &t
     }
 }
 
+/* Node2vec walks: over the edge set, or with the hooks where the engine asks
+ * the sorted adjacency (node2vec_adjacency 1). */
+template <typename S, typename WC, typename TC, typename Bucket>
+void launch_node2vec(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
+                     const float *ra, const WalkLaunch &L)
+{
+    const uint32_t n = L.walker_num;
+    const unsigned bs = (unsigned)e->walk_block;
+    if (tc.respond_query.set.keys == nullptr)
+    {
+        walk_static_kernel<S, WC, TC, Bucket><<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, L);
+        return;
+    }
+    const N2vTables<Bucket> t{alias, (const float *)e->sum.p, ra, tc.respond_query.set};
+    n2v_walk_kernel<TC::has_static, TC::has_outlier, Bucket>
+        <<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, t, n2v_params(tc), L);
+}
+
 /* One walk over walkers [rs.walker_begin, + rs.walker_num): alias tables,
  * regular area, path capacity, the walk kernel.  Events: ev0 before the alias
  * build, ev1 before the walk, ev2 after. */
@@ -994,8 +1014,8 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
                 Lp.park = q[0];
                 Lp.park_count = cnt;
                 Lp.park_below = (uint32_t)e->walk_park;
-                walk_static_kernel<S, WC, TC, Bucket><<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra,
-                                                                                               Lp);
+                walk_static_kernel<S, WC, TC, Bucket>
+                    <<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, Lp);
                 count_launch(e);
                 const unsigned rgrid = (unsigned)e->sm_count * (1024u / bs);
                 for (int r = 0; r < kParkRounds; r++)
@@ -1020,9 +1040,14 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
         {
             launch_straight<S, WC, TC, Bucket>(e, g, wc, tc, alias, L, (uint32_t *)d_status + 14);
         }
+        else if constexpr (is_node2vec<TC>::value)
+        {
+            launch_node2vec<S, WC, TC, Bucket>(e, g, wc, tc, alias, ra, L);
+        }
         else
         {
-            walk_static_kernel<S, WC, TC, Bucket><<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, L);
+            walk_static_kernel<S, WC, TC, Bucket>
+                <<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, L);
         }
         count_launch(e);
     }

@@ -31,6 +31,8 @@
 namespace kk
 {
 
+constexpr unsigned kFullMask = 0xffffffffu;
+
 /* ---- configuration types -------------------------------------------------- */
 
 /* WalkerConfig (include/walk.hpp:147-193). */
@@ -108,150 +110,176 @@ struct SecondOrderTransitionConfig
 };
 
 /* ---- edge set ---------------------------------------------------------------
- * Exact lookup of directed edges (u, v): open addressing over 64 B buckets,
- * linear probing bucket by bucket from bucket mulhi(mix(key), nbuckets), with
- * 4 * nbuckets >= 4E slots so the load is at most 1/4 and a lookup rarely
- * leaves its first bucket.  A bucket is eight 64-bit words: four keys
- * u << 32 | v (one 32 B sector), then per slot (pos << 32 | weight bits):
- * the smallest index of (u, v) within u's adjacency, which for a sorted
- * adjacency is std::lower_bound's position of v in N(u), and the weight of
- * that edge (0 without weights).  A membership test reads the key sector; the
- * return-edge lookup of node2vec's outlier bound reads the whole bucket and
- * has the edge's position and weight in the same access.  Keys only go from
- * empty to filled and an insert moves past a bucket only when all four of its
- * slots hold other keys, so a lookup that meets an empty slot may stop. */
-constexpr uint64_t kEdgeSetEmpty = ~0ull;
-constexpr uint32_t kEdgeSetWords = 8; /* 64-bit words per bucket */
+ * Exact lookup of directed edges (u, v): an open-addressing table of 32-bit
+ * neighbour ids per row, in 32 B sectors of eight slots.  Row u of degree d at
+ * offset e0 has d / 4 + 1 sectors from sector e0 / 4 + u on (rows do not
+ * overlap: (e0 + d) / 4 >= e0 / 4 + d / 4), so a lookup finds the row's table
+ * from its adjacency position alone, the load is below 1/2, and the whole set
+ * takes 8 B an edge and 32 B a vertex: it stays in L2 eight times longer than
+ * a table of 64-bit (u, v) keys at load 1/4 in 64 B buckets did.  v's probe
+ * starts at sector edge_set_sector(v) of the row and goes on in turn; an
+ * insert moves past a sector only when its eight slots hold other ids, so a
+ * lookup that meets a free slot may stop.  Beside the ids, the weight of
+ * (u, v)'s first edge in u's sorted adjacency, std::lower_bound's (weighted
+ * graphs; the same slot of a parallel array). */
+constexpr uint32_t kEdgeSetSlots = 8; /* a sector's slots; kNone: free */
 
 struct EdgeSetView
 {
-    const uint64_t *keys; /* nbuckets buckets of kEdgeSetWords words; nullptr: no set */
-    uint64_t nbuckets;
+    const uint32_t *keys; /* nullptr: no set */
+    const float *w;       /* nullptr: unweighted */
+    const int64_t *off;
 };
 
-/* splitmix64 finalizer (Steele, Lea, Flood, OOPSLA 2014) */
-__host__ __device__ __forceinline__ uint64_t mix64(uint64_t x)
+__host__ __device__ __forceinline__ uint64_t edge_set_row(int64_t e0, vertex_id_t u)
 {
-    x ^= x >> 30;
-    x *= 0xbf58476d1ce4e5b9ull;
-    x ^= x >> 27;
-    x *= 0x94d049bb133111ebull;
-    x ^= x >> 31;
-    return x;
+    return ((uint64_t)e0 >> 2) + u;
+}
+__host__ __device__ __forceinline__ uint32_t edge_set_sectors(uint32_t deg)
+{
+    return (deg >> 2) + 1;
+}
+/* all rows' sectors */
+__host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t V)
+{
+    return (E >> 2) + V + 1;
+}
+/* where v's probe starts among a row's n sectors */
+__host__ __device__ __forceinline__ uint32_t edge_set_sector(vertex_id_t v, uint32_t n)
+{
+    uint32_t a = v * 0x9E3779B1u;
+    a ^= a >> 16;
+    return mulhi32(a * 0x85EBCA6Bu, n);
 }
 
-/* The slot (bucket * 4 + j) of edge (u, v), or ~0 when (u, v) is not an edge. */
-__device__ __forceinline__ uint64_t edge_set_slot(const EdgeSetView &s, vertex_id_t u, vertex_id_t v)
+/* Sector {a, b} against id v: the slot that holds it, 8 for a free slot (v is
+ * not in the row), 9 for neither (the next sector decides). */
+__device__ __forceinline__ uint32_t edge_set_match(const uint4 &a, const uint4 &b, vertex_id_t v)
 {
-    const uint64_t key = ((uint64_t)u << 32) | v;
-    uint64_t b = __umul64hi(mix64(key), s.nbuckets);
-    for (uint64_t probe = 0; probe < s.nbuckets; probe++)
-    {
-        const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + b * kEdgeSetWords);
-        uint4 q[2];
+    const uint32_t k[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t r = k[7] == kNone ? 8u : 9u; /* slots fill from the first on */
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-            q[j] = __ldg(p + j);
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-        {
-            const uint64_t k0 = ((uint64_t)q[j].y << 32) | q[j].x, k1 = ((uint64_t)q[j].w << 32) | q[j].z;
-            if (k0 == key)
-                return b * 4 + 2 * j;
-            if (k1 == key)
-                return b * 4 + 2 * j + 1;
-            if (k0 == kEdgeSetEmpty || k1 == kEdgeSetEmpty)
-                return ~0ull;
-        }
-        b = b + 1 == s.nbuckets ? 0 : b + 1;
-    }
-    return ~0ull;
+    for (uint32_t j = 0; j < 8; j++)
+        r = k[j] == v ? j : r;
+    return r;
 }
 
-/* Edge (u, v)'s first position in N(u) and its weight, read with the keys in
- * one access per bucket probed; false when (u, v) is not an edge. */
-__device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t u, vertex_id_t v, uint32_t &pos,
-                                              float &weight)
+/* Whether (u, v) is an edge, u's adjacency being deg edges from e0, and its
+ * weight where weight is given (weighted sets). */
+__device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t u, int64_t e0, uint32_t deg,
+                                              vertex_id_t v, float *weight)
 {
-    const uint64_t key = ((uint64_t)u << 32) | v;
-    uint64_t b = __umul64hi(mix64(key), s.nbuckets);
-    for (uint64_t probe = 0; probe < s.nbuckets; probe++)
+    const uint64_t row = edge_set_row(e0, u);
+    const uint32_t n = edge_set_sectors(deg);
+    uint32_t b = edge_set_sector(v, n);
+    for (uint32_t probe = 0; probe < n; probe++)
     {
-        const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + b * kEdgeSetWords);
-        uint4 q[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            q[j] = __ldg(p + j);
-        const uint64_t k[4] = {((uint64_t)q[0].y << 32) | q[0].x, ((uint64_t)q[0].w << 32) | q[0].z,
-                               ((uint64_t)q[1].y << 32) | q[1].x, ((uint64_t)q[1].w << 32) | q[1].z};
-        const uint32_t pw[8] = {q[2].x, q[2].y, q[2].z, q[2].w, q[3].x, q[3].y, q[3].z, q[3].w};
-#pragma unroll
-        for (int j = 0; j < 4; j++)
+        const uint64_t at = (row + b) * kEdgeSetSlots;
+        const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + at);
+        const uint32_t m = edge_set_match(__ldg(p), __ldg(p + 1), v);
+        if (m < 8)
         {
-            if (k[j] == key)
-            {
-                weight = __uint_as_float(pw[2 * j]);
-                pos = pw[2 * j + 1];
-                return true;
-            }
-            if (k[j] == kEdgeSetEmpty)
-                return false;
+            if (weight != nullptr)
+                *weight = gather(s.w + at + m);
+            return true;
         }
-        b = b + 1 == s.nbuckets ? 0 : b + 1;
+        if (m == 8)
+            return false;
+        b = b + 1 == n ? 0 : b + 1;
     }
     return false;
 }
 
-/* Adds edge (u, v) at local index `local` of N(u), weight wt: the smallest
- * index of the key wins, with its weight (one 64-bit atomicMin on
- * local << 32 | weight bits). */
-__device__ __forceinline__ void edge_set_insert(uint64_t *buckets, uint64_t nbuckets, vertex_id_t u, vertex_id_t v,
-                                                uint32_t local, float wt)
+/* Puts v (not yet in the row) into the row of n sectors at keys, in shared or
+ * global memory; its slot. */
+__device__ __forceinline__ uint32_t edge_set_insert(uint32_t *keys, uint32_t n, vertex_id_t v)
 {
-    const uint64_t key = ((uint64_t)u << 32) | v;
-    uint64_t b = __umul64hi(mix64(key), nbuckets);
-    for (uint64_t probe = 0; probe < nbuckets; probe++)
+    uint32_t b = edge_set_sector(v, n);
+    for (;;) /* ends: the row has more slots than ids */
     {
-        for (int j = 0; j < 4; j++)
+        for (uint32_t j = 0; j < kEdgeSetSlots; j++)
         {
-            unsigned long long *k = reinterpret_cast<unsigned long long *>(buckets + b * kEdgeSetWords + j);
-            const unsigned long long old = atomicCAS(k, (unsigned long long)kEdgeSetEmpty, (unsigned long long)key);
-            if (old == kEdgeSetEmpty || old == key)
-            {
-                atomicMin(reinterpret_cast<unsigned long long *>(buckets + b * kEdgeSetWords + 4 + j),
-                          ((unsigned long long)local << 32) | __float_as_uint(wt));
-                return;
-            }
+            uint32_t *k = keys + b * kEdgeSetSlots + j;
+            if (*(volatile uint32_t *)k == kNone && atomicCAS(k, kNone, v) == kNone)
+                return b * kEdgeSetSlots + j;
         }
-        b = b + 1 == nbuckets ? 0 : b + 1;
+        b = b + 1 == n ? 0 : b + 1;
     }
 }
 
-/* Inserts the out-edges of the vertices order[lo, hi): a block per vertex
- * (hubs) or a warp per vertex. */
-static __global__ void edge_set_block_kernel(GraphView g, uint64_t *buckets, uint64_t nbuckets,
-                                             const uint32_t *order, uint32_t lo, uint32_t hi)
+/* The rows order[lo, hi), a block each (hubs): the row's table in global
+ * memory.  The adjacency is sorted, so an id's first edge is the one that
+ * differs from the edge before it. */
+static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g, uint32_t *keys, float *w,
+                                                                     const uint32_t *order, uint32_t lo, uint32_t hi)
 {
     for (uint32_t k = lo + blockIdx.x; k < hi; k += gridDim.x)
     {
-        const uint32_t v = order[k];
-        const int64_t e0 = g.off[v];
-        for (int64_t e = e0 + threadIdx.x; e < g.off[v + 1]; e += blockDim.x)
-            edge_set_insert(buckets, nbuckets, v, g.nbr[e], (uint32_t)(e - e0), g.w ? g.w[e] : 0.0f);
+        const uint32_t u = order[k];
+        const int64_t e0 = g.off[u];
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg);
+        const uint64_t at = edge_set_row(e0, u) * kEdgeSetSlots;
+        for (uint32_t i = threadIdx.x; i < n * kEdgeSetSlots; i += blockDim.x)
+            keys[at + i] = kNone;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < deg; i += blockDim.x)
+        {
+            const uint32_t v = g.nbr[e0 + i];
+            if (i > 0 && g.nbr[e0 + i - 1] == v)
+                continue;
+            const uint32_t slot = edge_set_insert(keys + at, n, v);
+            if (w != nullptr)
+                w[at + slot] = g.w[e0 + i];
+        }
+        __syncthreads();
     }
 }
 
-static __global__ void edge_set_warp_kernel(GraphView g, uint64_t *buckets, uint64_t nbuckets,
-                                            const uint32_t *order, uint32_t lo, uint32_t hi)
+/* The rows order[lo, hi) of at most DMAX edges, G lanes each: the row's table
+ * in shared memory (its inserts are chains of atomics, ten times shorter there
+ * than in L2), then out in one coalesced pass. */
+template <uint32_t DMAX>
+constexpr uint32_t edge_set_group_words()
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < hi; k += nwarps)
+    return (DMAX / 4 + 1) * kEdgeSetSlots;
+}
+
+template <uint32_t G, uint32_t DMAX>
+static __global__ void __launch_bounds__(128) edge_set_group_kernel(GraphView g, uint32_t *keys, float *w,
+                                                                    const uint32_t *order, uint32_t lo, uint32_t hi)
+{
+    extern __shared__ uint32_t s_rows[];
+    constexpr uint32_t W = edge_set_group_words<DMAX>();
+    const uint32_t gl = threadIdx.x % G, grp = threadIdx.x / G, groups = blockDim.x / G;
+    const unsigned mask = G == 32 ? kFullMask : ((1u << (G % 32)) - 1u) << (threadIdx.x % 32 / G * G);
+    uint32_t *tk = s_rows + grp * W * (w != nullptr ? 2 : 1);
+    float *tw = reinterpret_cast<float *>(tk + W);
+    for (uint32_t k = lo + blockIdx.x * groups + grp; k < hi; k += gridDim.x * groups)
     {
-        const uint32_t v = order[k];
-        const int64_t e0 = g.off[v];
-        for (int64_t e = e0 + lane; e < g.off[v + 1]; e += 32)
-            edge_set_insert(buckets, nbuckets, v, g.nbr[e], (uint32_t)(e - e0), g.w ? g.w[e] : 0.0f);
+        const uint32_t u = order[k];
+        const int64_t e0 = g.off[u];
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg);
+        for (uint32_t i = gl; i < n * kEdgeSetSlots; i += G)
+            tk[i] = kNone;
+        __syncwarp(mask);
+        for (uint32_t i = gl; i < deg; i += G)
+        {
+            const uint32_t v = g.nbr[e0 + i];
+            if (i > 0 && g.nbr[e0 + i - 1] == v)
+                continue;
+            const uint32_t slot = edge_set_insert(tk, n, v);
+            if (w != nullptr)
+                tw[slot] = g.w[e0 + i];
+        }
+        __syncwarp(mask);
+        const uint64_t at = edge_set_row(e0, u) * kEdgeSetSlots;
+        for (uint32_t i = gl; i < n * kEdgeSetSlots; i += G)
+        {
+            keys[at + i] = tk[i];
+            if (w != nullptr)
+                w[at + i] = tw[i];
+        }
+        __syncwarp(mask);
     }
 }
 
@@ -545,7 +573,6 @@ constexpr uint32_t kAliasHubMin = 16385; /* degree from which a vertex is a hub 
  * degree in (kAliasClassMax[c], kAliasClassMax[c - 1]] */
 constexpr uint32_t kAliasClasses = 8;
 constexpr uint32_t kAliasClassMax[kAliasClasses] = {16384, 4096, 2048, 1024, 512, 128, 32, 16};
-constexpr unsigned kFullMask = 0xffffffffu;
 
 /* A vertex of the degree-descending order with its adjacency range, so an
  * alias kernel reaches a row with one 16-byte load instead of order[] then
@@ -1914,6 +1941,20 @@ struct has_query_matters<F, S,
 {
 };
 
+/* Whether an extension_comp hook may be asked at a vertex without out-edges
+ * (`static constexpr bool any_vertex = true`): its reads then go out beside
+ * the offsets', instead of after the degree is known. */
+template <typename F, typename = void>
+struct ext_any_vertex
+{
+    static constexpr bool value = false;
+};
+template <typename F>
+struct ext_any_vertex<F, std::void_t<decltype(F::any_vertex)>>
+{
+    static constexpr bool value = F::any_vertex;
+};
+
 /* A picked candidate: index local to the adjacency (kNone when the bucket
  * does not carry it), neighbour, and the neighbour's cursor when the bucket
  * carries one (has_cur). */
@@ -1926,42 +1967,38 @@ struct Cand
     uint32_t tag; /* AdjUnit::type_tag of the candidate edge */
 };
 
-/* Candidate pick: uniform (include/walk.hpp:1016-1018) or alias
- * (:1020-1028; the coin is drawn only when the bucket has an alias).  A
- * bucket is read as the two 16 B halves of its 32 B sector. */
+/* A pick by word wp at most: uniform (include/walk.hpp:1016-1018) or alias
+ * (:1020-1028).  The coin is drawn, from word wc, only when the bucket has an
+ * alias; coin says whether it was.  A bucket is read as the two 16 B halves of
+ * its 32 B sector, or as one 16 B read. */
 template <typename TC, typename Bucket>
-__device__ __forceinline__ Cand pick_candidate(const GraphView &g, const Bucket *alias, const Pos &pos, Sampler &rng)
+__device__ __forceinline__ Cand pick_words(const GraphView &g, const Bucket *alias, const Pos &pos, uint32_t wp,
+                                           uint32_t wc, bool &coin)
 {
-    if constexpr (TC::has_static && Bucket::compact)
+    const uint32_t c = map_gen(wp, pos.deg);
+    if constexpr (TC::has_static)
     {
-        /* b = {p, p_nbr, q_nbr, p_type tag | q_type tag << 16} */
-        const uint4 b = gather(reinterpret_cast<const uint4 *>(alias + pos.e0 + rng.gen(pos.deg)));
-        if (b.z == kNone || rng.gen_float(1.0f) < __uint_as_float(b.x))
-            return Cand{kNone, b.y, 0, false, b.w & 0xffffu};
-        return Cand{kNone, b.z, 0, false, b.w >> 16};
-    }
-    else if constexpr (TC::has_static)
-    {
-        const uint4 *b4 = reinterpret_cast<const uint4 *>(alias + pos.e0 + rng.gen(pos.deg));
-        const uint4 lo = gather(b4), hi = gather(b4 + 1);
-        if constexpr (Bucket::cursor)
-        {
-            /* lo = {p, p_nbr, q_nbr, -}, hi = {p_cur, q_cur} */
-            if (lo.z == kNone || rng.gen_float(1.0f) < __uint_as_float(lo.x))
-                return Cand{kNone, lo.y, ((uint64_t)hi.y << 32) | hi.x, true, 0};
-            return Cand{kNone, lo.z, ((uint64_t)hi.w << 32) | hi.z, true, 0};
-        }
+        const uint4 *b = reinterpret_cast<const uint4 *>(alias + pos.e0 + c);
+        const uint4 lo = gather(b);
+        uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (!Bucket::compact)
+            hi = gather(b + 1);
+        /* compact lo = {p, p_nbr, q_nbr, p_type tag | q_type tag << 16};
+         * cursor lo = {p, p_nbr, q_nbr, -}, hi = {p_cur, q_cur};
+         * index lo = {p, p_idx, q_idx, -}, hi = {p_nbr, q_nbr, p_type tag, q_type tag} */
+        coin = lo.z != kNone;
+        const bool first = !coin || map_gen_float(wc, 1.0f) < __uint_as_float(lo.x);
+        if constexpr (Bucket::compact)
+            return Cand{kNone, first ? lo.y : lo.z, 0, false, first ? lo.w & 0xffffu : lo.w >> 16};
+        else if constexpr (Bucket::cursor)
+            return Cand{kNone, first ? lo.y : lo.z,
+                        first ? ((uint64_t)hi.y << 32) | hi.x : ((uint64_t)hi.w << 32) | hi.z, true, 0};
         else
-        {
-            /* lo = {p, p_idx, q_idx, -}, hi = {p_nbr, q_nbr, p_type tag, q_type tag} */
-            if (lo.z == kNone || rng.gen_float(1.0f) < __uint_as_float(lo.x))
-                return Cand{lo.y, hi.x, 0, false, hi.z};
-            return Cand{lo.z, hi.y, 0, false, hi.w};
-        }
+            return Cand{first ? lo.y : lo.z, first ? hi.x : hi.y, 0, false, first ? hi.z : hi.w};
     }
     else
     {
-        const uint32_t c = rng.gen(pos.deg);
+        coin = false;
         if (g.adjc != nullptr)
         {
             const uint4 a = gather(g.adjc + pos.e0 + c);
@@ -2067,6 +2104,54 @@ __device__ __forceinline__ void walk_begin(const GraphView &g, const WC &wc, con
     r.trials = r.queries = r.probes = 0;
 }
 
+/* Walks whose every trial is accepted: first order without a dynamic
+ * component, hence without outliers (DeepWalk, PPR). */
+template <typename TC>
+constexpr bool straight()
+{
+    return TC::order == 1 && !TC::has_dynamic;
+}
+
+/* One step of a straight walk, a trial without the trial state. */
+template <typename S, typename WC, typename TC, typename Bucket>
+__device__ __forceinline__ bool straight_trial(const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
+                                               const WalkLaunch &L, WalkerRun<S> &run, Sampler &rng)
+{
+    Walker<S> &w = run.w;
+    const vertex_id_t v = run.v;
+    if (run.pos.e0 < 0)
+        run.pos = pos_from_offsets(g, v);
+    const Pos pos = run.pos;
+    if (pos.deg == 0)
+        return false;
+    rng.enter(w.id, w.step, 0);
+    const real_t ext = tc.extension_comp(w, v);
+    if (ext == 0.0f || (ext < 1.0f && rng.gen_float(1.0f) > ext))
+        return false;
+    run.trials++;
+    const uint32_t wp = rng.word();
+    bool coin;
+    const Cand ac = pick_words<TC, Bucket>(g, alias, pos, wp, rng.word(), coin);
+    w.step++;
+    if constexpr (is_hook<decltype(wc.walker_update_state)>())
+        wc.walker_update_state(w, v, AdjUnit{ac.nbr, (edge_id_t)(pos.e0 + ac.idx)});
+    if (run.out)
+    {
+        if (run.len >= run.cap)
+        {
+            atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
+            return false;
+        }
+        run.out[run.len] = ac.nbr;
+    }
+    run.len++;
+    run.pv = v;
+    run.ppos = pos;
+    run.v = ac.nbr;
+    run.pos = ac.has_cur ? pos_from_cursor(g, ac.nbr, ac.cur) : Pos{-1, 0};
+    return true;
+}
+
 /* One rejection trial of one walker; false when its walk ends.  The kernels
  * loop over trials, not steps: a lane whose trial is accepted starts its next
  * step on the next iteration instead of waiting for the warp's slowest
@@ -2094,51 +2179,18 @@ __device__ __forceinline__ void walk_begin(const GraphView &g, const WC &wc, con
  * from the taken bucket's cursor when it has one, else it is read from the
  * offsets when its step starts. */
 template <typename S, typename WC, typename TC, typename Bucket>
-__device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
-                                           const float *ra, const WalkLaunch &L, WalkerRun<S> &run, Sampler &rng)
+__device__ __forceinline__ bool rejection_trial(const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
+                                                const float *ra, const WalkLaunch &L, WalkerRun<S> &run,
+                                                Sampler &rng)
 {
     Walker<S> &w = run.w;
     const vertex_id_t v = run.v;
-    if constexpr (TC::order == 1 && !TC::has_dynamic)
-    {
-        /* every trial is accepted (no dynamic component, hence no outlier):
-         * a step is one trial, without the trial state */
-        if (run.pos.e0 < 0)
-            run.pos = pos_from_offsets(g, v);
-        const Pos pos = run.pos;
-        if (pos.deg == 0)
-            return false;
-        rng.enter(w.id, w.step, 0);
-        const real_t ext = tc.extension_comp(w, v);
-        if (ext == 0.0f || (ext < 1.0f && rng.gen_float(1.0f) > ext))
-            return false;
-        run.trials++;
-        const Cand ac = pick_candidate<TC>(g, alias, pos, rng);
-        w.step++;
-        if constexpr (is_hook<decltype(wc.walker_update_state)>())
-            wc.walker_update_state(w, v, AdjUnit{ac.nbr, (edge_id_t)(pos.e0 + ac.idx)});
-        if (run.out)
-        {
-            if (run.len >= run.cap)
-            {
-                atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
-                return false;
-            }
-            run.out[run.len] = ac.nbr;
-        }
-        run.len++;
-        run.pv = v;
-        run.ppos = pos;
-        run.v = ac.nbr;
-        run.pos = ac.has_cur ? pos_from_cursor(g, ac.nbr, ac.cur) : Pos{-1, 0};
-        return true;
-    }
+    /* the position in hand was asked for as the previous step was accepted,
+     * and the step's first words are evaluated before it is needed */
     if (!run.in_step)
     {
         if (run.pos.e0 < 0)
             run.pos = pos_from_offsets(g, v);
-        if (run.pos.deg == 0)
-            return false;
         rng.enter(w.id, w.step, 0);
         run.in_step = true;
         run.need_ext = true;
@@ -2148,18 +2200,28 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
     const Pos pos = run.pos;
     const int64_t e0 = pos.e0;
     const AdjList adj{(edge_id_t)e0, (edge_id_t)(e0 + pos.deg)};
-    Cand ac{kNone, 0, 0, false};
-    bool taken = false;
+    bool ends = false;
     if (run.need_ext)
     {
         /* first order: once per step; second order: at every superstep */
-        const real_t ext = tc.extension_comp(w, v);
-        if (ext == 0.0f || (ext < 1.0f && rng.gen_float(1.0f) > ext))
+        if constexpr (!ext_any_vertex<decltype(tc.extension_comp)>::value)
+            ends = pos.deg == 0;
+        if (!ends)
         {
-            run.trials += run.step_trials;
-            return false;
+            const real_t ext = tc.extension_comp(w, v);
+            ends = ext == 0.0f || (ext < 1.0f && rng.gen_float(1.0f) > ext);
         }
         run.need_ext = false;
+    }
+    /* the trial's words, at most four: the appendix's, the pick's, the coin's,
+     * the dart's */
+    uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
+    uint4 wd = rng.quad(nxt);
+    uint32_t drawn = 0;
+    if (ends || pos.deg == 0)
+    {
+        run.trials += run.step_trials;
+        return false;
     }
     if (++run.step_trials > L.trial_limit)
     {
@@ -2169,7 +2231,8 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
     }
     /* outlier appendix; the bound is a pure function of (walker, vertex,
      * adjacency), all fixed within a step, so one call serves every trial */
-    bool in_app = false, found = false;
+    Cand ac{kNone, 0, 0, false};
+    bool taken = false, in_app = false, found = false;
     Cand cd{kNone, 0, 0, false};
     float randval = 0.0f;
     if constexpr (TC::has_outlier)
@@ -2184,7 +2247,9 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
         if (ob > 0.0f && on > 0)
         {
             const float rav = regular_area<TC>(tc, ra, L, v, adj);
-            const float r = fsub(rng.gen_float(fadd(fmul(ob, u2f(on)), rav)), rav);
+            const float r = fsub(map_gen_float(wd.x, fadd(fmul(ob, u2f(on)), rav)), rav);
+            wd = make_uint4(wd.y, wd.z, wd.w, 0u);
+            drawn = 1;
             if (r > 0.0f)
             {
                 in_app = true;
@@ -2204,42 +2269,29 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
             }
         }
     }
+    if (!in_app)
+    {
+        /* the candidate and its dart */
+        bool coin;
+        cd = pick_words<TC, Bucket>(g, alias, pos, wd.x, wd.y, coin);
+        randval = map_gen_float(coin ? wd.z : wd.y, tc.dcomp_upperbound(v, adj));
+        drawn += coin ? 3u : 2u;
+    }
+    const AdjUnit cu{cd.nbr, (edge_id_t)(e0 + cd.idx), cd.tag};
     if constexpr (TC::order == 1)
     {
-        bool outlier_trial = false;
-        if constexpr (TC::has_outlier)
+        /* an outlier trial is accepted against the dynamic component, and in
+         * any case the next trial follows (no extension test) */
+        if (in_app)
         {
-            /* an outlier trial: accepted against the dynamic component, and
-             * in any case the next trial follows (no extension test) */
-            outlier_trial = in_app;
-            if (in_app && found && randval <= tc.dynamic_comp(w, v, AdjUnit{cd.nbr, (edge_id_t)(e0 + cd.idx)}))
-            {
-                ac = cd;
-                taken = true;
-            }
+            taken = found && randval <= tc.dynamic_comp(w, v, cu);
         }
-        if (!outlier_trial)
+        else
         {
-            const Cand pc = pick_candidate<TC>(g, alias, pos, rng);
-            if constexpr (TC::has_dynamic)
-            {
-                const float dart = rng.gen_float(tc.dcomp_upperbound(v, adj));
-                bool acc = false;
-                if constexpr (TC::has_lowerbound)
-                    acc = dart <= tc.dcomp_lowerbound(v, adj);
-                if (!acc)
-                    acc = dart <= tc.dynamic_comp(w, v, AdjUnit{pc.nbr, (edge_id_t)(e0 + pc.idx), pc.tag});
-                if (acc)
-                {
-                    ac = pc;
-                    taken = true;
-                }
-            }
-            else
-            {
-                ac = pc;
-                taken = true;
-            }
+            if constexpr (TC::has_lowerbound)
+                taken = randval <= tc.dcomp_lowerbound(v, adj);
+            if (!taken)
+                taken = randval <= tc.dynamic_comp(w, v, cu);
         }
     }
     else
@@ -2247,17 +2299,13 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
         typedef typename TC::query_type Q;
         typedef typename TC::response_type R;
         if (in_app && !found)
-            return true; /* the reference's retry within the superstep: no extension test */
-        bool accepted = false;
-        if (!in_app)
         {
-            cd = pick_candidate<TC>(g, alias, pos, rng);
-            randval = rng.gen_float(tc.dcomp_upperbound(v, adj));
-            if constexpr (TC::has_lowerbound)
-                accepted = randval <= tc.dcomp_lowerbound(v, adj);
+            rng.take(drawn, nxt);
+            return true; /* the reference's retry within the superstep: no extension test */
         }
-        const AdjUnit cu{cd.nbr, (edge_id_t)(e0 + cd.idx), cd.tag};
-        if (!accepted)
+        if constexpr (TC::has_lowerbound)
+            taken = !in_app && randval <= tc.dcomp_lowerbound(v, adj);
+        if (!taken)
         {
             R resp{};
             Q query{};
@@ -2290,18 +2338,17 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
                     }
                 }
             }
-            accepted = randval <= tc.dynamic_comp(w, resp, v, cu);
+            taken = randval <= tc.dynamic_comp(w, resp, v, cu);
         }
-        if (!accepted)
-        {
+        if (!taken)
             run.need_ext = true; /* the next superstep re-tests the extension */
-            return true;
-        }
-        ac = cd;
-        taken = true;
     }
+    ac = cd;
     if (!taken)
+    {
+        rng.take(drawn, nxt);
         return true;
+    }
     run.trials += run.step_trials;
     run.in_step = false;
     w.step++;
@@ -2320,19 +2367,18 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
     run.pv = v;
     run.ppos = pos;
     run.v = ac.nbr;
-    if (ac.has_cur)
-        run.pos = pos_from_cursor(g, ac.nbr, ac.cur);
-    else
-        run.pos = Pos{-1, 0};
+    run.pos = ac.has_cur ? pos_from_cursor(g, ac.nbr, ac.cur) : pos_from_offsets(g, ac.nbr);
     return true;
 }
 
-/* Walks whose every trial is accepted: first order without a dynamic
- * component, hence without outliers (DeepWalk, PPR). */
-template <typename TC>
-constexpr bool straight()
+template <typename S, typename WC, typename TC, typename Bucket>
+__device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
+                                           const float *ra, const WalkLaunch &L, WalkerRun<S> &run, Sampler &rng)
 {
-    return TC::order == 1 && !TC::has_dynamic;
+    if constexpr (straight<TC>())
+        return straight_trial<S>(g, wc, tc, alias, L, run, rng);
+    else
+        return rejection_trial<S>(g, wc, tc, alias, ra, L, run, rng);
 }
 
 /* A walker stopped at a step boundary between launches (first-order walks):

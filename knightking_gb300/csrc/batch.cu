@@ -159,9 +159,22 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
             bp.count = cnt;
             bp.below = (uint32_t)e->walk_park;
         }
-        walk_batch_kernel<typename App::S, App, Bucket><<<grid, bs, 0, slot.stream>>>(
-            gv, app, d_jobs, nj, plan.total, alias, (const float *)e->sum.p, *path, length, steps, status,
-            e->trial_limit, st, hdr, bp, slot.notify);
+        bool launched = false;
+        if constexpr (is_node2vec<TC>::value)
+        {
+            if (app.set.keys != nullptr)
+            {
+                const N2vTables<Bucket> t{alias, (const float *)e->sum.p, nullptr, app.set};
+                n2v_batch_kernel<TC::has_static, Bucket><<<grid, bs, 0, slot.stream>>>(
+                    gv, app, t, d_jobs, nj, plan.total, *path, length, steps, status, e->trial_limit, st, hdr,
+                    slot.notify);
+                launched = true;
+            }
+        }
+        if (!launched)
+            walk_batch_kernel<typename App::S, App, Bucket><<<grid, bs, 0, slot.stream>>>(
+                gv, app, d_jobs, nj, plan.total, alias, (const float *)e->sum.p, *path, length, steps, status,
+                e->trial_limit, st, hdr, bp, slot.notify);
         count_launch(e);
         if (park)
         {
@@ -260,10 +273,7 @@ void launch_app_batch(kk_engine *e, const BatchPlan &plan, BatchSlot &slot, cons
     }
     else if (plan.app == KK_APP_NODE2VEC)
     {
-        const EdgeSetView set = p ? e->n2v_adjacency == 0
-                                        ? EdgeSetView{(const uint64_t *)e->edge_set.p, e->edge_set_nb}
-                                        : EdgeSetView{nullptr, 0}
-                                  : node2vec_edge_set(e);
+        const EdgeSetView set = p ? node2vec_edge_set_built(e) : node2vec_edge_set(e);
         if (plan.weighted)
             launch_batch(e, Node2vecBatch<true>{g.nbr, e->d_w, set}, plan, slot, d_jobs, length, path, d_steps,
                          d_status, want_paths, p, hdr);

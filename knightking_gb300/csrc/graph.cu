@@ -280,36 +280,47 @@ const uint4 *cursor_adjacency_of(kk_engine *e)
     return (const uint4 *)e->adjc.p;
 }
 
-EdgeSetView node2vec_edge_set(kk_engine *e)
+EdgeSetView node2vec_edge_set_built(const kk_engine *e)
 {
     if (e->n2v_adjacency != 0)
-        return EdgeSetView{nullptr, 0};
-    if (!e->edge_set_valid)
+        return EdgeSetView{nullptr, nullptr, nullptr};
+    return EdgeSetView{(const uint32_t *)e->edge_set.p, e->d_w ? (const float *)e->edge_set_w.p : nullptr, e->d_off};
+}
+
+EdgeSetView node2vec_edge_set(kk_engine *e)
+{
+    if (e->n2v_adjacency != 0 || e->edge_set_valid)
+        return node2vec_edge_set_built(e);
+    const uint64_t words = edge_set_total(e->E, e->V) * kEdgeSetSlots;
+    uint32_t *keys = e->edge_set.as<uint32_t>(words);
+    float *w = e->d_w ? e->edge_set_w.as<float>(words) : nullptr;
+    const uint32_t *order = vertex_order(e);
+    const GraphView g = e->view();
+    const uint32_t *t = e->tier;
+    /* rows of more than 1024 edges a block each, the others in groups with
+     * their tables in shared memory: the classes of the vertex order */
+    if (t[3])
     {
-        const uint64_t nb = e->E > 0 ? e->E : 1; /* four slots per bucket: load <= 1/4 */
-        uint64_t *buckets = e->edge_set.as<uint64_t>(nb * kEdgeSetWords);
-        /* empty keys and (pos, weight) words at their maximum for atomicMin */
-        KK_CUDA_CHECK(cudaMemsetAsync(buckets, 0xff, nb * kEdgeSetWords * sizeof(uint64_t), e->stream));
-        const uint32_t *order = vertex_order(e);
-        const GraphView g = e->view();
-        if (e->n_hub)
-        {
-            const unsigned grid = e->n_hub < 4u * e->sm_count ? e->n_hub : 4u * e->sm_count;
-            edge_set_block_kernel<<<grid, 1024, 0, e->stream>>>(g, buckets, nb, order, 0, e->n_hub);
-            count_launch(e);
-            KK_CUDA_CHECK(cudaGetLastError());
-        }
-        if (e->n_nz > e->n_hub)
-        {
-            edge_set_warp_kernel<<<grid_for(e, (uint64_t)(e->n_nz - e->n_hub) * 32, 256), 256, 0, e->stream>>>(
-                g, buckets, nb, order, e->n_hub, e->n_nz);
-            count_launch(e);
-            KK_CUDA_CHECK(cudaGetLastError());
-        }
-        e->edge_set_nb = nb;
-        e->edge_set_valid = true;
+        edge_set_block_kernel<<<t[3] < 2u * e->sm_count ? t[3] : 2u * e->sm_count, 1024, 0, e->stream>>>(g, keys, w,
+                                                                                                        order, 0, t[3]);
+        count_launch(e);
+        KK_CUDA_CHECK(cudaGetLastError());
     }
-    return EdgeSetView{(const uint64_t *)e->edge_set.p, e->edge_set_nb};
+    auto group = [&](auto kern, uint32_t G, uint32_t row_words, uint32_t lo, uint32_t hi) {
+        if (hi <= lo)
+            return;
+        const size_t smem = (size_t)(128 / G) * row_words * (w ? 8 : 4);
+        KK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<grid_for(e, hi - lo, 128 / G), 128, smem, e->stream>>>(g, keys, w, order, lo, hi);
+        count_launch(e);
+        KK_CUDA_CHECK(cudaGetLastError());
+    };
+    group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(), t[3], t[4]);
+    group(edge_set_group_kernel<32, 512>, 32, edge_set_group_words<512>(), t[4], t[5]);
+    group(edge_set_group_kernel<16, 128>, 16, edge_set_group_words<128>(), t[5], t[6]);
+    group(edge_set_group_kernel<8, 32>, 8, edge_set_group_words<32>(), t[6], e->n_nz);
+    e->edge_set_valid = true;
+    return node2vec_edge_set_built(e);
 }
 
 const uint8_t *metapath_vertex_masks(kk_engine *e)
