@@ -433,6 +433,9 @@ struct kk_engine
      * stream from the start (a hub row's pairing is a long chain of rounds
      * that the small classes need not wait for) */
     int alias_streams = 3;
+    /* alias_one_launch (option): small graphs' tables in one launch
+     * (build_alias_small); 0: the classes' launches whatever the size */
+    int alias_one_launch = 1;
     /* alias_small_lanes (option): 0 lane groups of 4 (degree 17..32) and 2
      * (1..16) per row; 1 groups of 2 and 1 */
     int alias_small_lanes = 0;
@@ -656,6 +659,70 @@ void launch_alias_class(kk_engine *e, K kern, unsigned nt, size_t smem, uint32_t
     KK_CUDA_CHECK(cudaGetLastError());
 }
 
+/* The build in one launch beside the hubs', for graphs of up to
+ * kAliasSmallEdges edges whose rows of 1025 to 16384 edges are at most four a
+ * resident block (a block of 256 threads takes each; more of them, and the
+ * classes' own launches fill the SMs better); false: left to those.  Classes
+ * against one launch, us: R-MAT 8 48 / 19, 10 71 / 28, 14 151 / 45, 16 219 /
+ * 95, 18 366 / 188, 19 384 / 296, 20 690 / 743 (3,000 such rows: classes); a
+ * graph of 1 M vertices and 32 M edges with 200 such rows 691 / 559. */
+constexpr uint64_t kAliasSmallEdges = 40000000;
+
+template <typename TC, typename Bucket>
+bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *alias, const uint64_t *vcur, float *sum,
+                       uint2 *scratch, const RowDesc *rows, uint32_t *next)
+{
+    if (e->E > kAliasSmallEdges || !e->alias_one_launch)
+        return false;
+    int resident = 0;
+    KK_CUDA_CHECK(cudaFuncSetAttribute(alias_small_kernel<TC, Bucket>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kAliasSmallSmem));
+    KK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, alias_small_kernel<TC, Bucket>, 256,
+                                                                kAliasSmallSmem));
+    const uint32_t *t = e->tier;
+    const uint32_t hold = (uint32_t)e->sm_count * (uint32_t)(resident > 0 ? resident : 1);
+    if (t[3] - t[0] > 4 * hold)
+        return false;
+    AliasSmall a;
+    a.first = t[0]; /* the hubs keep 1024 threads a row, on the side stream */
+    a.big = t[3];
+    a.big_blocks = a.big - a.first < hold ? a.big - a.first : hold;
+    const uint32_t per[kAliasSmallClasses] = {1, 2, 4, 8, 16};
+    uint32_t sum_tasks = 0;
+    for (uint32_t c = 0; c < kAliasSmallClasses; c++)
+    {
+        a.lo[c] = t[3 + c];
+        a.lo[c + 1] = t[4 + c];
+        sum_tasks += (t[4 + c] - t[3 + c] + per[c] - 1) / per[c];
+        a.task[c] = sum_tasks;
+    }
+    const uint32_t want = a.big_blocks + (sum_tasks + 7) / 8;
+    const uint32_t grid = want < hold ? want : hold;
+    if (a.first)
+    {
+        KK_CUDA_CHECK(cudaEventRecord(e->ev_fork, e->stream));
+        KK_CUDA_CHECK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
+        const uint32_t cap = (uint32_t)(e->sm_count > 1 ? e->sm_count / 2 : 1);
+        alias_build_hub_kernel<TC, Bucket><<<a.first < cap ? a.first : cap, 1024, 0, e->side>>>(
+            g, tc, alias, vcur, sum, scratch, (const uint32_t *)e->order.p, 0, a.first, next + 2);
+        count_launch(e);
+        KK_CUDA_CHECK(cudaGetLastError());
+    }
+    if (grid)
+    {
+        alias_small_kernel<TC, Bucket><<<grid, 256, kAliasSmallSmem, e->stream>>>(g, tc, alias, vcur, sum, scratch,
+                                                                                 rows, a, next);
+        count_launch(e);
+        KK_CUDA_CHECK(cudaGetLastError());
+    }
+    if (a.first)
+    {
+        KK_CUDA_CHECK(cudaEventRecord(e->ev_join, e->side));
+        KK_CUDA_CHECK(cudaStreamWaitEvent(e->stream, e->ev_join, 0));
+    }
+    return true;
+}
+
 /* Builds alias tables in the Bucket layout into e->alias/e->sum for a
  * static functor: hubs on the side stream, the other classes in turn on the
  * main stream or (alias_streams) the small-row classes after the hubs on the
@@ -681,6 +748,15 @@ void build_alias(kk_engine *e, const TC &tc)
     uint32_t *next = e->alias_next.as<uint32_t>(16);
     KK_CUDA_CHECK(cudaMemsetAsync(next, 0, 16 * sizeof(uint32_t), e->stream));
     const uint32_t *t = e->tier;
+    if (build_alias_small(e, g, tc, alias, vcur, sum, scratch, rows, next))
+    {
+        if constexpr (weight_tables)
+        {
+            if (tc.static_comp.w == e->d_w)
+                e->alias_cached = layout;
+        }
+        return;
+    }
     cudaStream_t st = e->stream;
     const bool hub_alone = e->alias_streams == 4 && e->n_hub;
     cudaStream_t hub_st = hub_alone ? e->hub : e->side;
@@ -882,7 +958,18 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
     const float *ra = nullptr;
     if constexpr (TC::has_static)
     {
-        build_alias<TC, Bucket>(e, tc);
+        if constexpr (std::is_same<typename TC::static_type, apps::WeightStatic>::value)
+        {
+            /* the tables depend on the static component only: one
+             * instantiation of the build serves every weighted app */
+            TransitionConfig<EmptyData, apps::FixedLengthExt<EmptyData>, apps::WeightStatic> stc;
+            stc.static_comp = tc.static_comp;
+            build_alias<decltype(stc), Bucket>(e, stc);
+        }
+        else
+        {
+            build_alias<TC, Bucket>(e, tc);
+        }
         alias = (const Bucket *)e->alias.p;
     }
     if constexpr (TC::has_outlier)

@@ -1309,28 +1309,163 @@ constexpr size_t alias_group_smem_per_warp()
  * memory before the limit of 32 blocks per SM), so a block is one warp. */
 constexpr uint32_t kAliasGroupWarps = 1;
 
+/* The alias tables of a warp's 32 / G rows d (a row per group of G lanes; deg
+ * 0: none), staged in smem: 8 B per edge of DMAX edges a row.  Every loop runs
+ * to the warp's maximum with per-group predicates, so the groups stay
+ * converged and share each instruction. */
+template <uint32_t G, uint32_t DMAX, typename TC, typename Bucket, typename Mid>
+__device__ __forceinline__ void alias_group_rows(const GraphView &g, const TC &tc, Bucket *out, const uint64_t *vcur,
+                                                 float *sum_out, const RowDesc &d, uint32_t *smem, Mid mid)
+{
+    static_assert(G == 1 || G == 2 || G == 4 || G == 8 || G == 16 || G == 32, "group of 1 to 32 lanes");
+    static_assert(DMAX % 4 == 0 && DMAX <= 65535, "16-bit queue entries");
+    constexpr uint32_t RPW = 32 / G;
+    constexpr uint32_t gbits = G == 32 ? kFullMask : (1u << G) - 1u;
+    const uint32_t lane = threadIdx.x & 31, grp = lane / G, gl = lane % G, gsh = grp * G;
+    const uint32_t glt = (1u << gl) - 1u;
+    float *F = reinterpret_cast<float *>(smem) + (size_t)grp * DMAX;
+    uint16_t *Pq = reinterpret_cast<uint16_t *>(smem + (size_t)RPW * DMAX) + (size_t)grp * 2 * DMAX;
+    uint16_t *Qq = Pq + DMAX;
+    const uint32_t v = d.v, deg = d.deg;
+    const int64_t e0 = d.e0;
+    const uint32_t wdeg = __reduce_max_sync(kFullMask, deg);
+    /* stage the rows' probabilities, G consecutive edges per load */
+#pragma unroll 4
+    for (uint32_t i = gl; i < wdeg; i += G)
+        if (i < deg)
+            F[i] = static_at(g, tc, v, e0 + i);
+    __syncwarp();
+    mid(); /* the rows are on their way: the caller fetches what comes next */
+    /* the sum in edge order (:579-584), one lane per group */
+    float sum = 0.0f;
+    if constexpr (RPW == 1)
+    {
+        /* rows of 513..2048 edges: the exact warp scan */
+        sum = warp_exact_sum<8>(F, deg);
+        if (lane == 0 && deg != 0 && sum_out != nullptr)
+            sum_out[v] = sum;
+    }
+    else if (gl == 0)
+    {
+        /* a group past its row's end adds +0.0f, which leaves a sum of
+         * non-negative terms unchanged, so the FADD chain has no select */
+        uint32_t i = 0;
+        for (; i + 4 <= wdeg; i += 4)
+        {
+            const float a0 = i < deg ? F[i] : 0.0f, a1 = i + 1 < deg ? F[i + 1] : 0.0f;
+            const float a2 = i + 2 < deg ? F[i + 2] : 0.0f, a3 = i + 3 < deg ? F[i + 3] : 0.0f;
+            sum = fadd(fadd(fadd(fadd(sum, a0), a1), a2), a3);
+        }
+        for (; i < wdeg; i++)
+            sum = fadd(sum, i < deg ? F[i] : 0.0f);
+        if (deg != 0 && sum_out != nullptr)
+            sum_out[v] = sum;
+    }
+    sum = __shfl_sync(kFullMask, sum, gsh);
+    const float ave = fdiv(sum, u2f(deg));
+    /* split in edge order (:593-602) into two linear queues of 16-bit
+     * edge indices, P from the front of its array, Q from the front of
+     * its own (each queue gets at most deg entries over the whole
+     * pairing: the q tail is B + I - C <= deg) */
+    uint32_t pt = 0, qt = 0;
+    for (uint32_t base = 0; base < wdeg; base += G)
+    {
+        const uint32_t i = base + gl;
+        const bool valid = i < deg;
+        const float x = valid ? F[i] : 0.0f;
+        const bool sm = valid && x < ave, bg = valid && !(x < ave);
+        const uint32_t mp = (__ballot_sync(kFullMask, sm) >> gsh) & gbits;
+        const uint32_t mq = (__ballot_sync(kFullMask, bg) >> gsh) & gbits;
+        if (sm)
+            Pq[pt + __popc(mp & glt)] = (uint16_t)i;
+        if (bg)
+            Qq[qt + __popc(mq & glt)] = (uint16_t)i;
+        pt += __popc(mp);
+        qt += __popc(mq);
+    }
+    __syncwarp();
+    /* pairing (:603-630) in batches of at most G iterations, queue
+     * mechanics and residuals only: iteration k pops P[k] and Q[k], so
+     * the queues themselves record every pairing, and the buckets are
+     * written afterwards in one converged pass.  A p entry's value is
+     * final when it is popped (only popped q entries change), so the
+     * pass reads the same F[P[k]] the iteration saw.  A batch of b = 0
+     * leaves a finished group's state unchanged.  A group whose q queue
+     * holds a single entry leaves the batches for the chain below. */
+    uint32_t ph = 0, qh = 0;
+    for (;;)
+    {
+        const bool live = ph < pt && qt - qh > 1;
+        if (!__any_sync(kFullMask, live))
+            break;
+        const uint32_t b = live ? min(min(pt - ph, qt - qh), G) : 0;
+        const bool act = gl < b;
+        bool conv = false;
+        uint32_t qi = 0;
+        if (act)
+        {
+            const uint32_t pi = Pq[ph + gl];
+            qi = Qq[qh + gl];
+            const float r = fsub(F[qi], fsub(ave, F[pi]));
+            F[qi] = r;
+            conv = r < ave;
+        }
+        const uint32_t mc = (__ballot_sync(kFullMask, act && conv) >> gsh) & gbits;
+        const uint32_t ms = (__ballot_sync(kFullMask, act && !conv) >> gsh) & gbits;
+        if (act)
+        {
+            if (conv)
+                Pq[pt + __popc(mc & glt)] = (uint16_t)qi;
+            else
+                Qq[qt + __popc(ms & glt)] = (uint16_t)qi;
+        }
+        __syncwarp();
+        ph += b;
+        qh += b;
+        pt += __popc(mc);
+        qt += __popc(ms);
+    }
+    alias_q1_chain<G>(F, Pq, Qq, ph, pt, qh, qt, ave, gl, gsh);
+    /* the buckets in pop order: pairs (P[k], Q[k]) for k < ph (= qh),
+     * then the leftovers of whichever queue is non-empty with p = 1
+     * (:623-638) */
+    Bucket *ob = out + e0;
+    const uint8_t *ty = g.type != nullptr ? g.type + e0 : nullptr;
+    const uint32_t *N = g.nbr + e0; /* the row's neighbours, read from the L1-cached row */
+#pragma unroll 2
+    for (uint32_t base = 0; base < wdeg; base += G)
+    {
+        const uint32_t k = base + gl;
+        if (k < deg)
+        {
+            if (k < ph)
+            {
+                const uint32_t pi = Pq[k], qi = Qq[k];
+                ob[k] = Bucket::make_n(fdiv(F[pi], ave), pi, qi, N[pi], N[qi], vcur, ty);
+            }
+            else
+            {
+                const uint32_t x = k - ph < pt - ph ? Pq[k] : Qq[qh + (k - pt)];
+                ob[k] = Bucket::make_n(1.0f, x, kNone, N[x], 0, vcur, ty);
+            }
+        }
+    }
+    __syncwarp();
+}
+
 template <typename TC, typename Bucket, uint32_t G, uint32_t DMAX>
 __global__ void __launch_bounds__(32 * kAliasGroupWarps) alias_group_kernel(GraphView g, TC tc, Bucket *out,
                                                                           const uint64_t *vcur, float *sum_out,
                                                                           const RowDesc *rows, uint32_t lo,
                                                                           uint32_t hi, uint32_t *next)
 {
-    static_assert(G == 1 || G == 2 || G == 4 || G == 8 || G == 16 || G == 32, "group of 1 to 32 lanes");
-    static_assert(DMAX % 4 == 0 && DMAX <= 65535, "16-bit queue entries");
     constexpr uint32_t RPW = 32 / G;
-    constexpr uint32_t gbits = G == 32 ? kFullMask : (1u << G) - 1u;
     extern __shared__ uint32_t smem_all[];
     /* this warp's slice: 8 B per edge of its RPW rows */
     uint32_t *smem = smem_all + (size_t)(threadIdx.x >> 5) * RPW * DMAX * 2;
-    const uint32_t lane = threadIdx.x & 31, grp = lane / G, gl = lane % G, gsh = grp * G;
-    const uint32_t glt = (1u << gl) - 1u;
-    float *F = reinterpret_cast<float *>(smem) + (size_t)grp * DMAX;
-    uint16_t *Pq = reinterpret_cast<uint16_t *>(smem + (size_t)RPW * DMAX) + (size_t)grp * 2 * DMAX;
-    uint16_t *Qq = Pq + DMAX;
-    /* every loop below runs to the warp's maximum with per-group predicates,
-     * so the groups stay converged and share each instruction.  The next
-     * vertices' counter value and row descriptors are fetched while the
-     * current ones are processed. */
+    const uint32_t lane = threadIdx.x & 31, grp = lane / G;
+    /* the next vertices' counter value and row descriptors are fetched while
+     * the current ones are processed */
     const uint32_t n = hi - lo;
     uint32_t t = 0;
     if (lane == 0)
@@ -1344,134 +1479,12 @@ __global__ void __launch_bounds__(32 * kAliasGroupWarps) alias_group_kernel(Grap
         uint32_t tn = 0;
         if (lane == 0)
             tn = atomicAdd(next, RPW);
-        const uint32_t v = d.v, deg = d.deg;
-        const int64_t e0 = d.e0;
-        const uint32_t wdeg = __reduce_max_sync(kFullMask, deg);
-        /* stage the rows' probabilities, G consecutive edges per load */
-#pragma unroll 4
-        for (uint32_t i = gl; i < wdeg; i += G)
-            if (i < deg)
-                F[i] = static_at(g, tc, v, e0 + i);
-        __syncwarp();
-        tn = __shfl_sync(kFullMask, tn, 0);
         RowDesc dn{0, 0, 0};
-        if (tn + grp < n)
-            dn = rows[lo + tn + grp];
-        /* the sum in edge order (:579-584), one lane per group */
-        float sum = 0.0f;
-        if constexpr (RPW == 1)
-        {
-            /* rows of 513..2048 edges: the exact warp scan */
-            sum = warp_exact_sum<8>(F, deg);
-            if (lane == 0 && deg != 0 && sum_out != nullptr)
-                sum_out[v] = sum;
-        }
-        else if (gl == 0)
-        {
-            /* a group past its row's end adds +0.0f, which leaves a sum of
-             * non-negative terms unchanged, so the FADD chain has no select */
-            uint32_t i = 0;
-            for (; i + 4 <= wdeg; i += 4)
-            {
-                const float a0 = i < deg ? F[i] : 0.0f, a1 = i + 1 < deg ? F[i + 1] : 0.0f;
-                const float a2 = i + 2 < deg ? F[i + 2] : 0.0f, a3 = i + 3 < deg ? F[i + 3] : 0.0f;
-                sum = fadd(fadd(fadd(fadd(sum, a0), a1), a2), a3);
-            }
-            for (; i < wdeg; i++)
-                sum = fadd(sum, i < deg ? F[i] : 0.0f);
-            if (deg != 0 && sum_out != nullptr)
-                sum_out[v] = sum;
-        }
-        sum = __shfl_sync(kFullMask, sum, gsh);
-        const float ave = fdiv(sum, u2f(deg));
-        /* split in edge order (:593-602) into two linear queues of 16-bit
-         * edge indices, P from the front of its array, Q from the front of
-         * its own (each queue gets at most deg entries over the whole
-         * pairing: the q tail is B + I - C <= deg) */
-        uint32_t pt = 0, qt = 0;
-        for (uint32_t base = 0; base < wdeg; base += G)
-        {
-            const uint32_t i = base + gl;
-            const bool valid = i < deg;
-            const float x = valid ? F[i] : 0.0f;
-            const bool sm = valid && x < ave, bg = valid && !(x < ave);
-            const uint32_t mp = (__ballot_sync(kFullMask, sm) >> gsh) & gbits;
-            const uint32_t mq = (__ballot_sync(kFullMask, bg) >> gsh) & gbits;
-            if (sm)
-                Pq[pt + __popc(mp & glt)] = (uint16_t)i;
-            if (bg)
-                Qq[qt + __popc(mq & glt)] = (uint16_t)i;
-            pt += __popc(mp);
-            qt += __popc(mq);
-        }
-        __syncwarp();
-        /* pairing (:603-630) in batches of at most G iterations, queue
-         * mechanics and residuals only: iteration k pops P[k] and Q[k], so
-         * the queues themselves record every pairing, and the buckets are
-         * written afterwards in one converged pass.  A p entry's value is
-         * final when it is popped (only popped q entries change), so the
-         * pass reads the same F[P[k]] the iteration saw.  A batch of b = 0
-         * leaves a finished group's state unchanged.  A group whose q queue
-         * holds a single entry leaves the batches for the chain below. */
-        uint32_t ph = 0, qh = 0;
-        for (;;)
-        {
-            const bool live = ph < pt && qt - qh > 1;
-            if (!__any_sync(kFullMask, live))
-                break;
-            const uint32_t b = live ? min(min(pt - ph, qt - qh), G) : 0;
-            const bool act = gl < b;
-            bool conv = false;
-            uint32_t qi = 0;
-            if (act)
-            {
-                const uint32_t pi = Pq[ph + gl];
-                qi = Qq[qh + gl];
-                const float r = fsub(F[qi], fsub(ave, F[pi]));
-                F[qi] = r;
-                conv = r < ave;
-            }
-            const uint32_t mc = (__ballot_sync(kFullMask, act && conv) >> gsh) & gbits;
-            const uint32_t ms = (__ballot_sync(kFullMask, act && !conv) >> gsh) & gbits;
-            if (act)
-            {
-                if (conv)
-                    Pq[pt + __popc(mc & glt)] = (uint16_t)qi;
-                else
-                    Qq[qt + __popc(ms & glt)] = (uint16_t)qi;
-            }
-            __syncwarp();
-            ph += b;
-            qh += b;
-            pt += __popc(mc);
-            qt += __popc(ms);
-        }
-        alias_q1_chain<G>(F, Pq, Qq, ph, pt, qh, qt, ave, gl, gsh);
-        /* the buckets in pop order: pairs (P[k], Q[k]) for k < ph (= qh),
-         * then the leftovers of whichever queue is non-empty with p = 1
-         * (:623-638) */
-        Bucket *ob = out + e0;
-        const uint8_t *ty = g.type != nullptr ? g.type + e0 : nullptr;
-        const uint32_t *N = g.nbr + e0; /* the row's neighbours, read from the L1-cached row */
-#pragma unroll 2
-        for (uint32_t base = 0; base < wdeg; base += G)
-        {
-            const uint32_t k = base + gl;
-            if (k < deg)
-            {
-                if (k < ph)
-                {
-                    const uint32_t pi = Pq[k], qi = Qq[k];
-                    ob[k] = Bucket::make_n(fdiv(F[pi], ave), pi, qi, N[pi], N[qi], vcur, ty);
-                }
-                else
-                {
-                    const uint32_t x = k - ph < pt - ph ? Pq[k] : Qq[qh + (k - pt)];
-                    ob[k] = Bucket::make_n(1.0f, x, kNone, N[x], 0, vcur, ty);
-                }
-            }
-        }
-        __syncwarp();
+        alias_group_rows<G, DMAX>(g, tc, out, vcur, sum_out, d, smem, [&]() {
+            tn = __shfl_sync(kFullMask, tn, 0);
+            if (tn + grp < n)
+                dn = rows[lo + tn + grp];
+        });
         t = tn;
         d = dn;
     }
@@ -1493,198 +1506,211 @@ constexpr size_t alias_block_row_smem()
     return (size_t)DMAX * 8;
 }
 
+/* What a block's rows share beside the row itself. */
+struct AliasShared
+{
+    SumMap maps[33];
+    uint32_t w[33], row[4];
+    float f;
+    uint32_t u;
+};
+
+template <uint32_t NT, uint32_t DMAX, typename TC, typename Bucket>
+__device__ __forceinline__ void alias_block_row(const GraphView &g, const TC &tc, Bucket *out, const uint64_t *vcur,
+                                                float *sum_out, uint32_t v, int64_t e0, uint32_t deg, uint32_t *smem,
+                                                AliasShared &sh)
+{
+    static_assert(NT % 32 == 0 && NT <= 1024 && DMAX % 8 == 0 && DMAX <= 65535, "block-row tier shape");
+    constexpr uint32_t K = 4; /* terms or iterations per thread per pass */
+    float *F = reinterpret_cast<float *>(smem);
+    uint16_t *P = reinterpret_cast<uint16_t *>(smem + DMAX);
+    uint16_t *Q = P + DMAX;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+#pragma unroll 4
+    for (uint32_t i = tid; i < deg; i += NT)
+        F[i] = static_at(g, tc, v, e0 + i);
+    __syncthreads();
+    /* the sum in edge order (:579-584), exact block scan */
+    const float sum = block_exact_sum<4>([&](uint32_t i) { return F[i]; }, deg, sh.maps, &sh.f, &sh.u, nullptr);
+    if (tid == 0 && sum_out != nullptr)
+        sum_out[v] = sum;
+    const float ave = fdiv(sum, u2f(deg));
+    /* stable split in edge order (:593-602), K consecutive terms per
+     * thread per pass */
+    uint32_t pt = 0, qt = 0;
+    for (uint32_t base = 0; base < deg; base += NT * K)
+    {
+        const uint32_t i0 = base + tid * K;
+        uint32_t cs = 0, cb = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < K; j++)
+        {
+            const bool valid = i0 + j < deg;
+            const bool sm = valid && F[i0 + j] < ave;
+            cs += sm;
+            cb += valid && !sm;
+        }
+        uint32_t tot;
+        const uint32_t ex = block_scan_packed(cs | (cb << 16), tot, sh.w);
+        uint32_t ps = pt + (ex & 0xFFFFu), qs = qt + (ex >> 16);
+#pragma unroll
+        for (uint32_t j = 0; j < K; j++)
+        {
+            if (i0 + j < deg)
+            {
+                if (F[i0 + j] < ave)
+                    P[ps++] = (uint16_t)(i0 + j);
+                else
+                    Q[qs++] = (uint16_t)(i0 + j);
+            }
+        }
+        pt += tot & 0xFFFFu;
+        qt += tot >> 16;
+    }
+    __syncthreads();
+    /* pairing (:603-630); bucket k is the k-th p pop */
+    Bucket *ob = out + e0;
+    const uint8_t *ty = g.type != nullptr ? g.type + e0 : nullptr;
+    uint32_t ph = 0, qh = 0;
+    while (ph < pt && qh < qt)
+    {
+        const uint32_t b = min(min(pt - ph, qt - qh), NT * K);
+        if (b <= 64)
+        {
+            /* warp 0 alone until the pairing ends or both queues are long again */
+            if (tid < 32)
+            {
+                uint32_t wph = ph, wpt = pt, wqh = qh, wqt = qt;
+                const uint32_t lt = (1u << lane) - 1u;
+                while (wph < wpt && wqh < wqt)
+                {
+                    const uint32_t wb = min(min(wpt - wph, wqt - wqh), 32u);
+                    if (wb == 32u && min(wpt - wph, wqt - wqh) > 128u)
+                        break;
+                    const bool act = lane < wb;
+                    bool conv = false;
+                    uint32_t qi = 0;
+                    if (act)
+                    {
+                        const uint32_t pi = P[wph + lane];
+                        qi = Q[wqh + lane];
+                        const float r = fsub(F[qi], fsub(ave, F[pi]));
+                        F[qi] = r;
+                        conv = r < ave;
+                    }
+                    const uint32_t mc = __ballot_sync(kFullMask, act && conv);
+                    const uint32_t ms = __ballot_sync(kFullMask, act && !conv);
+                    if (act)
+                    {
+                        if (conv)
+                            P[wpt + __popc(mc & lt)] = (uint16_t)qi;
+                        else
+                            Q[wqt + __popc(ms & lt)] = (uint16_t)qi;
+                    }
+                    __syncwarp();
+                    wph += wb;
+                    wqh += wb;
+                    wpt += __popc(mc);
+                    wqt += __popc(ms);
+                }
+                if (tid == 0)
+                {
+                    sh.row[0] = wph;
+                    sh.row[1] = wpt;
+                    sh.row[2] = wqh;
+                    sh.row[3] = wqt;
+                }
+            }
+            __syncthreads();
+            ph = sh.row[0];
+            pt = sh.row[1];
+            qh = sh.row[2];
+            qt = sh.row[3];
+            __syncthreads();
+            continue;
+        }
+        /* iterations tid*K .. tid*K + K - 1 of the batch */
+        const uint32_t i0 = tid * K;
+        uint32_t qk[K], convm = 0, nc = 0, ns = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < K; j++)
+        {
+            qk[j] = 0;
+            if (i0 + j < b)
+            {
+                const uint32_t pi = P[ph + i0 + j];
+                qk[j] = Q[qh + i0 + j];
+                const float r = fsub(F[qk[j]], fsub(ave, F[pi]));
+                F[qk[j]] = r;
+                if (r < ave)
+                {
+                    convm |= 1u << j;
+                    nc++;
+                }
+                else
+                {
+                    ns++;
+                }
+            }
+        }
+        uint32_t tot;
+        const uint32_t ex = block_scan_packed(nc | (ns << 16), tot, sh.w);
+        uint32_t pc = pt + (ex & 0xFFFFu), qs = qt + (ex >> 16);
+#pragma unroll
+        for (uint32_t j = 0; j < K; j++)
+        {
+            if (i0 + j < b)
+            {
+                if (convm & (1u << j))
+                    P[pc++] = (uint16_t)qk[j];
+                else
+                    Q[qs++] = (uint16_t)qk[j];
+            }
+        }
+        __syncthreads();
+        ph += b;
+        qh += b;
+        pt += tot & 0xFFFFu;
+        qt += tot >> 16;
+    }
+    /* the buckets in pop order (iteration k popped P[k] and Q[k]; a p
+     * entry's value is final once popped), then the leftovers of
+     * whichever queue is non-empty with p = 1 (:623-638) */
+    const uint32_t *N = g.nbr + e0; /* the row's neighbours, from global memory */
+    for (uint32_t k2 = tid; k2 < deg; k2 += NT)
+    {
+        if (k2 < ph)
+        {
+            const uint32_t pi = P[k2], qi2 = Q[k2];
+            ob[k2] = Bucket::make_n(fdiv(F[pi], ave), pi, qi2, N[pi], N[qi2], vcur, ty);
+        }
+        else
+        {
+            const uint32_t x = k2 < pt ? P[k2] : Q[qh + (k2 - pt)];
+            ob[k2] = Bucket::make_n(1.0f, x, kNone, N[x], 0, vcur, ty);
+        }
+    }
+    __syncthreads();
+}
+
 template <typename TC, typename Bucket, uint32_t NT, uint32_t DMAX>
 __global__ void __launch_bounds__(NT) alias_block_row_kernel(GraphView g, TC tc, Bucket *out, const uint64_t *vcur,
                                                              float *sum_out, const uint32_t *order, uint32_t lo,
                                                              uint32_t hi, uint32_t *next)
 {
-    static_assert(NT % 32 == 0 && NT <= 1024 && DMAX % 8 == 0 && DMAX <= 65535, "block-row tier shape");
     extern __shared__ uint32_t smem[];
-    constexpr uint32_t K = 4; /* terms or iterations per thread per pass */
-    __shared__ uint32_t s_w[33], s_row[4];
-    __shared__ SumMap s_maps[33];
-    __shared__ float s_f;
-    __shared__ uint32_t s_u;
-    float *F = reinterpret_cast<float *>(smem);
-    uint16_t *P = reinterpret_cast<uint16_t *>(smem + DMAX);
-    uint16_t *Q = P + DMAX;
-    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    __shared__ AliasShared sh;
     for (;;)
     {
-        if (tid == 0)
-            s_row[0] = atomicAdd(next, 1u);
+        if (threadIdx.x == 0)
+            sh.row[0] = atomicAdd(next, 1u);
         __syncthreads();
-        const uint32_t t = s_row[0];
+        const uint32_t t = sh.row[0];
         if (t >= hi - lo)
             break;
         const uint32_t v = order[lo + t];
         const int64_t e0 = g.off[v];
-        const uint32_t deg = (uint32_t)(g.off[v + 1] - e0);
-#pragma unroll 4
-        for (uint32_t i = tid; i < deg; i += NT)
-            F[i] = static_at(g, tc, v, e0 + i);
-        __syncthreads();
-        /* the sum in edge order (:579-584), exact block scan */
-        const float sum = block_exact_sum<4>([&](uint32_t i) { return F[i]; }, deg, s_maps, &s_f, &s_u, nullptr);
-        if (tid == 0 && sum_out != nullptr)
-            sum_out[v] = sum;
-        const float ave = fdiv(sum, u2f(deg));
-        /* stable split in edge order (:593-602), K consecutive terms per
-         * thread per pass */
-        uint32_t pt = 0, qt = 0;
-        for (uint32_t base = 0; base < deg; base += NT * K)
-        {
-            const uint32_t i0 = base + tid * K;
-            uint32_t cs = 0, cb = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < K; j++)
-            {
-                const bool valid = i0 + j < deg;
-                const bool sm = valid && F[i0 + j] < ave;
-                cs += sm;
-                cb += valid && !sm;
-            }
-            uint32_t tot;
-            const uint32_t ex = block_scan_packed(cs | (cb << 16), tot, s_w);
-            uint32_t ps = pt + (ex & 0xFFFFu), qs = qt + (ex >> 16);
-#pragma unroll
-            for (uint32_t j = 0; j < K; j++)
-            {
-                if (i0 + j < deg)
-                {
-                    if (F[i0 + j] < ave)
-                        P[ps++] = (uint16_t)(i0 + j);
-                    else
-                        Q[qs++] = (uint16_t)(i0 + j);
-                }
-            }
-            pt += tot & 0xFFFFu;
-            qt += tot >> 16;
-        }
-        __syncthreads();
-        /* pairing (:603-630); bucket k is the k-th p pop */
-        Bucket *ob = out + e0;
-        const uint8_t *ty = g.type != nullptr ? g.type + e0 : nullptr;
-        uint32_t ph = 0, qh = 0;
-        while (ph < pt && qh < qt)
-        {
-            const uint32_t b = min(min(pt - ph, qt - qh), NT * K);
-            if (b <= 64)
-            {
-                /* warp 0 alone until the pairing ends or both queues are long again */
-                if (tid < 32)
-                {
-                    uint32_t wph = ph, wpt = pt, wqh = qh, wqt = qt;
-                    const uint32_t lt = (1u << lane) - 1u;
-                    while (wph < wpt && wqh < wqt)
-                    {
-                        const uint32_t wb = min(min(wpt - wph, wqt - wqh), 32u);
-                        if (wb == 32u && min(wpt - wph, wqt - wqh) > 128u)
-                            break;
-                        const bool act = lane < wb;
-                        bool conv = false;
-                        uint32_t qi = 0;
-                        if (act)
-                        {
-                            const uint32_t pi = P[wph + lane];
-                            qi = Q[wqh + lane];
-                            const float r = fsub(F[qi], fsub(ave, F[pi]));
-                            F[qi] = r;
-                            conv = r < ave;
-                        }
-                        const uint32_t mc = __ballot_sync(kFullMask, act && conv);
-                        const uint32_t ms = __ballot_sync(kFullMask, act && !conv);
-                        if (act)
-                        {
-                            if (conv)
-                                P[wpt + __popc(mc & lt)] = (uint16_t)qi;
-                            else
-                                Q[wqt + __popc(ms & lt)] = (uint16_t)qi;
-                        }
-                        __syncwarp();
-                        wph += wb;
-                        wqh += wb;
-                        wpt += __popc(mc);
-                        wqt += __popc(ms);
-                    }
-                    if (tid == 0)
-                    {
-                        s_row[0] = wph;
-                        s_row[1] = wpt;
-                        s_row[2] = wqh;
-                        s_row[3] = wqt;
-                    }
-                }
-                __syncthreads();
-                ph = s_row[0];
-                pt = s_row[1];
-                qh = s_row[2];
-                qt = s_row[3];
-                __syncthreads();
-                continue;
-            }
-            /* iterations tid*K .. tid*K + K - 1 of the batch */
-            const uint32_t i0 = tid * K;
-            uint32_t qk[K], convm = 0, nc = 0, ns = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < K; j++)
-            {
-                qk[j] = 0;
-                if (i0 + j < b)
-                {
-                    const uint32_t pi = P[ph + i0 + j];
-                    qk[j] = Q[qh + i0 + j];
-                    const float r = fsub(F[qk[j]], fsub(ave, F[pi]));
-                    F[qk[j]] = r;
-                    if (r < ave)
-                    {
-                        convm |= 1u << j;
-                        nc++;
-                    }
-                    else
-                    {
-                        ns++;
-                    }
-                }
-            }
-            uint32_t tot;
-            const uint32_t ex = block_scan_packed(nc | (ns << 16), tot, s_w);
-            uint32_t pc = pt + (ex & 0xFFFFu), qs = qt + (ex >> 16);
-#pragma unroll
-            for (uint32_t j = 0; j < K; j++)
-            {
-                if (i0 + j < b)
-                {
-                    if (convm & (1u << j))
-                        P[pc++] = (uint16_t)qk[j];
-                    else
-                        Q[qs++] = (uint16_t)qk[j];
-                }
-            }
-            __syncthreads();
-            ph += b;
-            qh += b;
-            pt += tot & 0xFFFFu;
-            qt += tot >> 16;
-        }
-        /* the buckets in pop order (iteration k popped P[k] and Q[k]; a p
-         * entry's value is final once popped), then the leftovers of
-         * whichever queue is non-empty with p = 1 (:623-638) */
-        const uint32_t *N = g.nbr + e0; /* the row's neighbours, from global memory */
-        for (uint32_t k2 = tid; k2 < deg; k2 += NT)
-        {
-            if (k2 < ph)
-            {
-                const uint32_t pi = P[k2], qi2 = Q[k2];
-                ob[k2] = Bucket::make_n(fdiv(F[pi], ave), pi, qi2, N[pi], N[qi2], vcur, ty);
-            }
-            else
-            {
-                const uint32_t x = k2 < pt ? P[k2] : Q[qh + (k2 - pt)];
-                ob[k2] = Bucket::make_n(1.0f, x, kNone, N[x], 0, vcur, ty);
-            }
-        }
-        __syncthreads();
+        alias_block_row<NT, DMAX>(g, tc, out, vcur, sum_out, v, e0, (uint32_t)(g.off[v + 1] - e0), smem, sh);
     }
 }
 
@@ -1694,21 +1720,36 @@ __global__ void __launch_bounds__(NT) alias_block_row_kernel(GraphView g, TC tc,
  * iterations per thread per pass, so a 163,585-edge row takes ~40 passes of
  * each instead of one thread's FADD chain and ~160 barrier rounds. */
 template <typename TC, typename Bucket>
+__device__ __forceinline__ void alias_hub_row(const GraphView &g, const TC &tc, Bucket *out, const uint64_t *vcur,
+                                              float *sum_out, uint2 *scratch, uint32_t v, int64_t e0, uint32_t deg,
+                                              AliasShared &sh, uint2 *ring, float *head)
+{
+    auto load = [&](uint32_t i) { return static_at(g, tc, v, e0 + i); };
+    const float sum = block_exact_sum<4>(load, deg, sh.maps, &sh.f, &sh.u, head);
+    const float ave = fdiv(sum, u2f(deg));
+    if (threadIdx.x == 0 && sum_out != nullptr)
+        sum_out[v] = sum;
+    uint2 *P = scratch + 2 * e0;
+    uint2 *Q = P + deg;
+    uint32_t pt, qt;
+    block_split_wide<4>(load, deg, ave, P, Q, pt, qt, sh.w);
+    block_pairing_wide<4>(P, Q, pt, qt, ave, out + e0, g.nbr + e0, vcur, g.type != nullptr ? g.type + e0 : nullptr,
+                          sh.w, sh.row, ring);
+}
+
+template <typename TC, typename Bucket>
 __global__ void __launch_bounds__(1024) alias_build_hub_kernel(GraphView g, TC tc, Bucket *out, const uint64_t *vcur,
                                                                float *sum_out, uint2 *scratch, const uint32_t *order,
                                                                uint32_t lo, uint32_t hi, uint32_t *next)
 {
-    __shared__ SumMap s_maps[33];
-    __shared__ uint32_t s_w[33], s_state[4];
-    __shared__ float s_f;
-    __shared__ uint32_t s_u, s_k;
+    __shared__ AliasShared sh;
+    __shared__ uint32_t s_k;
     __shared__ uint2 s_ring[2 * kRingSize]; /* the short queue's ring, the long queue's staged head */
     __shared__ float s_head[2048];
-    const uint32_t tid = threadIdx.x;
     for (;;)
     {
         /* vertices from *next, largest first */
-        if (tid == 0)
+        if (threadIdx.x == 0)
             s_k = lo + atomicAdd(next, 1u);
         __syncthreads();
         const uint32_t k = s_k;
@@ -1717,18 +1758,89 @@ __global__ void __launch_bounds__(1024) alias_build_hub_kernel(GraphView g, TC t
             break;
         const uint32_t v = order[k];
         const int64_t e0 = g.off[v];
-        const uint32_t deg = (uint32_t)(g.off[v + 1] - e0);
-        auto load = [&](uint32_t i) { return static_at(g, tc, v, e0 + i); };
-        const float sum = block_exact_sum<4>(load, deg, s_maps, &s_f, &s_u, s_head);
-        const float ave = fdiv(sum, u2f(deg));
-        if (tid == 0 && sum_out != nullptr)
-            sum_out[v] = sum;
-        uint2 *P = scratch + 2 * e0;
-        uint2 *Q = P + deg;
-        uint32_t pt, qt;
-        block_split_wide<4>(load, deg, ave, P, Q, pt, qt, s_w);
-        block_pairing_wide<4>(P, Q, pt, qt, ave, out + e0, g.nbr + e0, vcur, g.type != nullptr ? g.type + e0 : nullptr,
-                              s_w, s_state, s_ring);
+        alias_hub_row(g, tc, out, vcur, sum_out, scratch, v, e0, (uint32_t)(g.off[v + 1] - e0), sh, s_ring, s_head);
+    }
+}
+
+/* The whole build in one launch (small graphs): the classes' rows are too few
+ * to fill the SMs one class after another, and each class then waits for its
+ * own longest row.  Blocks of 256 threads: the first take the rows of more
+ * than 1024 edges, largest first, a block each (alias_hub_row above 4096,
+ * else alias_block_row); every block then takes warp tasks (the lane groups of
+ * classes 4 to 8, 32 / G rows a task, largest first) until none is left. */
+constexpr uint32_t kAliasSmallClasses = 5;
+constexpr uint32_t kAliasSmallSmem = 8 * 1024 * 8; /* 8 warps' class-4 rows, 8 B an edge */
+struct AliasSmall
+{
+    uint32_t first, big, big_blocks;     /* rows [first, big) of more than 1024 edges, the blocks that take them */
+    uint32_t lo[kAliasSmallClasses + 1]; /* the classes' bounds in the vertex order */
+    uint32_t task[kAliasSmallClasses];   /* tasks of the classes up to and with this one */
+};
+
+template <typename TC, typename Bucket>
+__global__ void __launch_bounds__(256, 3) alias_small_kernel(GraphView g, TC tc, Bucket *out, const uint64_t *vcur,
+                                                             float *sum_out, uint2 *scratch, const RowDesc *rows,
+                                                             AliasSmall a, uint32_t *next)
+{
+    extern __shared__ uint32_t smem_all[];
+    __shared__ AliasShared sh;
+    __shared__ uint32_t s_k;
+    if (blockIdx.x < a.big_blocks)
+    {
+        for (uint32_t k = a.first + blockIdx.x; k < a.big;)
+        {
+            const RowDesc d = rows[k];
+            if (d.deg > 4096u)
+                alias_hub_row(g, tc, out, vcur, sum_out, scratch, d.v, d.e0, d.deg, sh,
+                              reinterpret_cast<uint2 *>(smem_all),
+                              reinterpret_cast<float *>(smem_all + 4 * kRingSize));
+            else
+                alias_block_row<256, 4096>(g, tc, out, vcur, sum_out, d.v, d.e0, d.deg, smem_all, sh);
+            if (threadIdx.x == 0)
+                s_k = a.first + a.big_blocks + atomicAdd(next, 1u);
+            __syncthreads();
+            k = s_k;
+            __syncthreads();
+        }
+    }
+    uint32_t *smem = smem_all + (threadIdx.x >> 5) * (kAliasSmallSmem / 32);
+    const uint32_t lane = threadIdx.x & 31, tasks = a.task[kAliasSmallClasses - 1];
+    uint32_t t = 0;
+    if (lane == 0)
+        t = atomicAdd(next + 1, 1u);
+    t = __shfl_sync(kFullMask, t, 0);
+    while (t < tasks)
+    {
+        uint32_t tn = 0;
+        if (lane == 0)
+            tn = atomicAdd(next + 1, 1u);
+        auto run = [&](auto Gc, auto Dc, uint32_t c) {
+            constexpr uint32_t G = decltype(Gc)::value, DMAX = decltype(Dc)::value;
+            const uint32_t at = a.lo[c] + (t - (c ? a.task[c - 1] : 0u)) * (32 / G) + lane / G;
+            RowDesc d{0, 0, 0};
+            if (at < a.lo[c + 1])
+                d = rows[at];
+            alias_group_rows<G, DMAX>(g, tc, out, vcur, sum_out, d, smem, []() {});
+        };
+        typedef std::integral_constant<uint32_t, 2> I2;
+        typedef std::integral_constant<uint32_t, 4> I4;
+        typedef std::integral_constant<uint32_t, 8> I8;
+        typedef std::integral_constant<uint32_t, 16> I16;
+        typedef std::integral_constant<uint32_t, 32> I32;
+        typedef std::integral_constant<uint32_t, 128> I128;
+        typedef std::integral_constant<uint32_t, 512> I512;
+        typedef std::integral_constant<uint32_t, 1024> I1024;
+        if (t < a.task[0])
+            run(I32{}, I1024{}, 0);
+        else if (t < a.task[1])
+            run(I16{}, I512{}, 1);
+        else if (t < a.task[2])
+            run(I8{}, I128{}, 2);
+        else if (t < a.task[3])
+            run(I4{}, I32{}, 3);
+        else
+            run(I2{}, I16{}, 4);
+        t = __shfl_sync(kFullMask, tn, 0);
     }
 }
 
