@@ -111,7 +111,7 @@ struct BatchSlot
     bool graph_mode = false;
     uint32_t max_walkers = 0;
     uint64_t max_cap = 0;
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec[2] = {nullptr, nullptr}; /* [1]: small node2vec batches */
     char *h_stage = nullptr; /* pinned: jobs | schemes | header | status */
     /* per-request completion (serving): counters and status words on the
      * device, flags in mapped host memory (notify.count == nullptr: off); the
@@ -144,9 +144,12 @@ struct BatchSlot
             if (ev[i])
                 cudaEventDestroy(ev[i]);
         ev[0] = ev[1] = ev[2] = nullptr;
-        if (exec)
-            cudaGraphExecDestroy(exec);
-        exec = nullptr;
+        for (cudaGraphExec_t &x : exec)
+        {
+            if (x)
+                cudaGraphExecDestroy(x);
+            x = nullptr;
+        }
         if (h_stage)
             cudaFreeHost(h_stage);
         h_stage = nullptr;
@@ -373,7 +376,7 @@ struct kk_engine
     /* node2vec adjacency test: 0 edge set (built once per graph), 1 binary
      * search of the sorted adjacency (option node2vec_adjacency) */
     int n2v_adjacency = 0;
-    kk::DevBuf edge_set, edge_set_w; /* the rows' ids and their weights */
+    kk::DevBuf edge_set;
     bool edge_set_valid = false;
     kk::DevBuf schemes;    /* metapath schemes of the running job */
     kk::BatchSlot bslot;   /* where the synchronous batch calls run */
@@ -899,16 +902,21 @@ void walk_regrouped(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc
  * R-MAT 22 weighted, 2.4 M walkers: 4.95 ms against 4.72 in tiles. */
 template <typename S, typename WC, typename TC, typename Bucket>
 void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
-                     const WalkLaunch &L, uint32_t *next)
+                     const WalkLaunch &L, bool uneven, uint32_t *next)
 {
     const uint32_t n = L.walker_num;
     const unsigned bs = (unsigned)e->walk_block;
+    /* paths that stream out as their segments end: a segment of uneven walks
+     * ends with its longest, whose steps take four times as long while every
+     * lane walks, and nothing would be left to copy beside (R-MAT 20, 1.8 M
+     * PPR walkers into pinned buffers: 7.2 ms in turn, 5.7 a thread each) */
+    const bool segments = uneven && L.seg_count != nullptr;
     const size_t smem = (size_t)(bs / 32) * kTileWords * sizeof(uint32_t);
     int resident = 0;
     KK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, walk_stream_kernel<S, WC, TC, Bucket>,
                                                                 (int)bs, smem));
     const unsigned hold = (unsigned)e->sm_count * (resident > 0 ? resident : 1), all = grid_for(e, n, bs);
-    if (all > hold)
+    if (all > hold && !segments)
     {
         walk_stream_kernel<S, WC, TC, Bucket><<<hold, bs, smem, e->stream>>>(g, wc, tc, alias, L, next);
     }
@@ -920,14 +928,14 @@ void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &t
 }
 
 /* Node2vec walks: over the edge set, or with the hooks where the engine asks
- * the sorted adjacency (node2vec_adjacency 1). */
+ * the sorted adjacency (node2vec_adjacency 1) or has no 32-bit offsets. */
 template <typename S, typename WC, typename TC, typename Bucket>
 void launch_node2vec(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
                      const float *ra, const WalkLaunch &L)
 {
     const uint32_t n = L.walker_num;
     const unsigned bs = (unsigned)e->walk_block;
-    if (tc.respond_query.set.keys == nullptr)
+    if (tc.respond_query.set.keys == nullptr || g.off32 == nullptr)
     {
         walk_static_kernel<S, WC, TC, Bucket><<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, L);
         return;
@@ -1125,7 +1133,7 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
         }
         if constexpr (straight<TC>())
         {
-            launch_straight<S, WC, TC, Bucket>(e, g, wc, tc, alias, L, (uint32_t *)d_status + 14);
+            launch_straight<S, WC, TC, Bucket>(e, g, wc, tc, alias, L, !rs.fixed_cap, (uint32_t *)d_status + 14);
         }
         else if constexpr (is_node2vec<TC>::value)
         {

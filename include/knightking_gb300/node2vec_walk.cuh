@@ -17,9 +17,9 @@
  * its pick beside it, at the draw the pick has when the bound is positive.
  * The previous vertex's row of the edge set is kept with it, so a question is
  * one read.  Against walk_trial()'s loop over a table of (u, v) keys in 64 B
- * buckets (same box): R-MAT 16, 65,536 walkers, p 2, q 0.5 353 -> 250 us;
- * R-MAT 19, 300,007 walkers, p 0.25, q 3 1558 -> 1330 us; R-MAT 22, 2.4 M
- * walkers, p 2, q 0.5 8.42 -> 7.45 ms; 20 jobs on 32 M edges 2.73 -> 2.30 ms.
+ * buckets (same box): R-MAT 16, 65,536 walkers, p 2, q 0.5 355 -> 263 us;
+ * R-MAT 19, 300,007 walkers, p 0.25, q 3 1550 -> 1170 us; R-MAT 22, 2.4 M
+ * walkers, p 2, q 0.5 8.36 -> 7.85 ms; 20 jobs on 32 M edges 2.73 -> 1.55 ms.
  */
 #pragma once
 
@@ -36,6 +36,42 @@ struct N2vParams
     step_t walk_length;
 };
 
+/* The same constants as the walk asks for them: in registers (or a launch's
+ * constant bank), or read from the job's row, which L1 holds, at each use: a
+ * batch's lanes have each their own, and eight registers more than the 64 of
+ * four blocks an SM spill into the loop. */
+struct N2vInRegs
+{
+    N2vParams p;
+    __device__ __forceinline__ float upperbound() const { return p.upperbound; }
+    __device__ __forceinline__ float lowerbound() const { return p.lowerbound; }
+    __device__ __forceinline__ float overflow() const { return p.overflow; }
+    __device__ __forceinline__ float inv_p() const { return p.inv_p; }
+    __device__ __forceinline__ float inv_q() const { return p.inv_q; }
+    __device__ __forceinline__ float sure_below() const { return p.sure_below; }
+    __device__ __forceinline__ uint32_t walk_length() const { return p.walk_length; }
+};
+
+struct N2vInJob
+{
+    const BatchJob *job;
+    /* volatile: read here, not kept */
+    __device__ __forceinline__ static uint32_t word(const void *at)
+    {
+        uint32_t x;
+        asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(x) : "l"(at));
+        return x;
+    }
+    __device__ __forceinline__ float c(int k) const { return __uint_as_float(word(job->c + k)); }
+    __device__ __forceinline__ float upperbound() const { return c(0); }
+    __device__ __forceinline__ float lowerbound() const { return c(1); }
+    __device__ __forceinline__ float overflow() const { return c(2); }
+    __device__ __forceinline__ float inv_p() const { return c(3); }
+    __device__ __forceinline__ float inv_q() const { return c(4); }
+    __device__ __forceinline__ float sure_below() const { return fminf(c(4), 1.0f); }
+    __device__ __forceinline__ uint32_t walk_length() const { return word(&job->walk_length); }
+};
+
 /* What every walk of the launch reads. */
 template <typename Bucket>
 struct N2vTables
@@ -46,15 +82,20 @@ struct N2vTables
     EdgeSetView set;
 };
 
-/* Walks run (just begun: start vertex, path slot) to its end. */
-template <bool Weighted, bool Outlier, typename Bucket>
-__device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const N2vParams &P,
-                                         const WalkLaunch &L, unsigned team,
-                                         WalkerRun<apps::Node2vecState> &run, Sampler &rng)
+/* Walks walker id from v to its end (the 32-bit offsets at hand), its path to
+ * out (vertex 0 on; or nullptr); the path's length in len.  team: the warp's
+ * lanes that call this together.  False when a step passed the trial limit. */
+template <bool Weighted, bool Outlier, typename Bucket, typename Params>
+__device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const Params &P,
+                                         walker_id_t id, vertex_id_t v, uint32_t *out, uint32_t trial_limit,
+                                         unsigned long long *stats, unsigned team, Sampler &rng, uint32_t &len)
 {
-    const uint32_t id = run.w.id;
-    uint32_t step = 0, prev = 0, v = run.v, trials = 0;
-    Pos pos = pos_from_offsets(g, v);
+    uint32_t step = 0, prev = 0, trials = 0;
+    bool within = true;
+    /* v's adjacency as read, its first edge and the one past its last: what
+     * follows from them is computed where it is used, or the walk would wait
+     * for them here */
+    uint32_t pb = gather(g.off32 + v), pe = gather(g.off32 + v + 1);
     float rav = 0.0f; /* regular_area of v */
     /* the step's outlier area, once its return edge is known (find: not yet),
      * and that edge: its weight, and its index unless it leads to prev */
@@ -63,22 +104,22 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
     uint32_t back_i = kNone;
     /* prev's row of the edge set, and the sector to read next, in it (query)
      * or in v's (find) */
-    uint64_t prow = 0;
-    uint32_t pn = 1, sec = 0;
+    uint32_t prow = 0, pn = 1, sec = 0;
     /* the pending question: is cand a neighbour of prev, and its dart */
     bool query = false;
-    Cand cand{kNone, 0, 0, false};
+    vertex_id_t cand = 0;
+    uint64_t cand_cur = 0;
     float dart = 0.0f;
     /* q > 1: most candidates are no neighbours, and a no rejects */
-    const bool ahead = P.inv_q < 1.0f;
+    const bool ahead = P.inv_q() < 1.0f;
     auto begin_step = [&]() {
         rng.enter(id, step, 0);
         trials = 0;
         if constexpr (Outlier)
         {
-            const bool on = P.overflow > 0.0f;
+            const bool on = P.overflow() > 0.0f;
             find = Weighted && on;
-            ob = Weighted ? 0.0f : P.overflow;
+            ob = Weighted ? 0.0f : P.overflow();
             back_i = kNone;
             sec = kNone; /* find's first sector follows from the position */
             if (on)
@@ -93,7 +134,7 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
     begin_step();
     /* one way through the loop, and the warp's lanes (team) meet at its top:
      * they share the instructions of every pass */
-    bool alive = P.walk_length > 0;
+    bool alive = P.walk_length() > 0;
     while (__any_sync(team, alive))
     {
         if (alive)
@@ -104,36 +145,38 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
              * at or below every neighbour: position 0, no lookup. */
             const bool asked = query;
             const bool look = asked || (Outlier && find && prev != 0);
-            uint4 k0, k1, w0, w1;
+            uint4 k0, k1; /* a sector: ids, and more ids or weights */
             if (asked)
             {
-                const uint4 *b = reinterpret_cast<const uint4 *>(t.set.keys + (prow + sec) * kEdgeSetSlots);
+                const uint4 *b =
+                    reinterpret_cast<const uint4 *>(t.set.keys + (uint64_t)(prow + sec) * kEdgeSectorWords);
                 k0 = __ldg(b);
-                k1 = __ldg(b + 1);
+                if (!Weighted)
+                    k1 = __ldg(b + 1);
             }
             uint4 nxt = make_uint4(0u, 0u, 0u, 0u), wd = nxt, lo = nxt, hi = nxt;
             bool app = false, trial = !asked || ahead;
             auto load = [&](uint32_t at) {
                 if constexpr (Weighted)
                 {
-                    const uint4 *b = reinterpret_cast<const uint4 *>(t.alias + pos.e0 + at);
+                    const uint4 *b = reinterpret_cast<const uint4 *>(t.alias + pb + at);
                     lo = gather(b);
                     if constexpr (!Bucket::compact)
                         hi = gather(b + 1);
                 }
                 else if (g.adjc != nullptr)
                 {
-                    lo = gather(g.adjc + pos.e0 + at);
+                    lo = gather(g.adjc + pb + at);
                 }
                 else
                 {
-                    lo.x = gather(g.nbr + pos.e0 + at);
+                    lo.x = gather(g.nbr + pb + at);
                 }
             };
             if (trial)
             {
                 wd = rng.quad(nxt);
-                alive = pos.deg != 0; /* a vertex without edges ends the walk as its step begins */
+                alive = pe != pb; /* a vertex without edges ends the walk as its step begins */
                 trial = alive;
                 app = Outlier && (find || ob > 0.0f);
                 if (alive)
@@ -141,59 +184,53 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
                     if (Outlier && Weighted && look && !asked)
                     {
                         if (sec == kNone)
-                            sec = edge_set_sector(prev, edge_set_sectors(pos.deg));
-                        const uint64_t at = (edge_set_row(pos.e0, v) + sec) * kEdgeSetSlots;
-                        const uint4 *b = reinterpret_cast<const uint4 *>(t.set.keys + at);
-                        const uint4 *bw = reinterpret_cast<const uint4 *>(t.set.w + at);
+                            sec = edge_set_sector(prev, edge_set_sectors(pe - pb, Weighted));
+                        const uint4 *b = reinterpret_cast<const uint4 *>(
+                            t.set.keys + (edge_set_row(pb, v, Weighted) + sec) * kEdgeSectorWords);
                         k0 = __ldg(b);
                         k1 = __ldg(b + 1);
-                        w0 = __ldg(bw);
-                        w1 = __ldg(bw + 1);
                     }
-                    load(map_gen(app ? wd.y : wd.x, pos.deg));
+                    load(map_gen(app ? wd.y : wd.x, pe - pb));
                 }
             }
             bool taken = false;
             if (look && alive)
             {
-                const uint32_t m = edge_set_match(k0, k1, asked ? cand.nbr : prev);
+                const vertex_id_t x = asked ? cand : prev;
+                const uint32_t m = Weighted ? edge_set_match(k0, x) : edge_set_match(k0, k1, x);
                 if (m == 9)
                 {
                     /* undecided: the next sector, next time */
-                    sec = sec + 1 == (asked ? pn : edge_set_sectors(pos.deg)) ? 0 : sec + 1;
+                    sec = sec + 1 == (asked ? pn : edge_set_sectors(pe - pb, Weighted)) ? 0 : sec + 1;
                     trial = false;
                 }
                 else if (asked)
                 {
                     query = false;
-                    taken = dart <= (m < 8 ? 1.0f : P.inv_q);
+                    taken = dart <= (m < 8 ? 1.0f : P.inv_q());
                     trial = trial && !taken;
                 }
                 else if constexpr (Outlier && Weighted)
                 {
-                    const float wl = m & 1 ? (m & 2 ? __uint_as_float(w0.w) : __uint_as_float(w0.y))
-                                           : (m & 2 ? __uint_as_float(w0.z) : __uint_as_float(w0.x));
-                    const float wh = m & 1 ? (m & 2 ? __uint_as_float(w1.w) : __uint_as_float(w1.y))
-                                           : (m & 2 ? __uint_as_float(w1.z) : __uint_as_float(w1.x));
-                    back_w = m & 4 ? wh : wl;
+                    back_w = __uint_as_float(word_of(k1, m));
                     bool edge = m < 8;
                     if (!edge)
                     {
                         /* directed graphs: std::lower_bound's edge, if any */
-                        back_i = apps::lower_bound_adj(g.nbr, (edge_id_t)pos.e0, pos.deg, prev);
-                        edge = back_i < pos.deg;
+                        back_i = apps::lower_bound_adj(g.nbr, pb, pe - pb, prev);
+                        edge = back_i < pe - pb;
                         if (edge)
-                            back_w = gather(g.w + pos.e0 + back_i);
+                            back_w = gather(g.w + pb + back_i);
                     }
-                    ob = edge ? fmul(back_w, P.overflow) : 0.0f;
+                    ob = edge ? fmul(back_w, P.overflow()) : 0.0f;
                     find = false;
                 }
             }
             else if (Outlier && find && alive)
             {
                 back_i = 0;
-                back_w = gather(g.w + pos.e0);
-                ob = fmul(back_w, P.overflow);
+                back_w = gather(g.w + pb);
+                ob = fmul(back_w, P.overflow());
                 find = false;
             }
             if (trial)
@@ -206,7 +243,7 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
                     {
                         float area = rav;
                         if (t.ra == nullptr)
-                            area = fmul(Weighted ? rav : u2f(pos.deg), P.upperbound);
+                            area = fmul(Weighted ? rav : u2f(pe - pb), P.upperbound());
                         const float r = fsub(map_gen_float(wd.x, fadd(fmul(ob, u2f(1u)), area)), area);
                         wd = make_uint4(wd.y, wd.z, wd.w, 0u);
                         drawn = 1;
@@ -225,89 +262,101 @@ __device__ __forceinline__ void n2v_walk(const GraphView &g, const N2vTables<Buc
                             }
                             else
                             {
-                                at = prev == 0 ? 0 : apps::lower_bound_adj(g.nbr, (edge_id_t)pos.e0, pos.deg, prev);
-                                some = at < pos.deg; /* none: the retry within the superstep */
+                                at = prev == 0 ? 0 : apps::lower_bound_adj(g.nbr, pb, pe - pb, prev);
+                                some = at < pe - pb; /* none: the retry within the superstep */
                             }
-                            cand = Cand{kNone, Weighted && at == kNone ? prev : some ? gather(g.nbr + pos.e0 + at) : 0, 0,
-                                        false, 0};
-                            dart = fadd(fdiv(fsub(r, fmul(u2f(oi), ob)), sc), P.upperbound);
+                            cand = Weighted && at == kNone ? prev : some ? gather(g.nbr + pb + at) : 0;
+                            cand_cur = ~0ull;
+                            dart = fadd(fdiv(fsub(r, fmul(u2f(oi), ob)), sc), P.upperbound());
                         }
                     }
                 }
                 if (!in_app)
                 {
                     if (Outlier && app != (drawn != 0))
-                        load(map_gen(wd.x, pos.deg)); /* the bound came out the other way */
+                        load(map_gen(wd.x, pe - pb)); /* the bound came out the other way */
                     if constexpr (Weighted)
                     {
                         const bool coin = lo.z != kNone;
                         const bool first = !coin || map_gen_float(wd.y, 1.0f) < __uint_as_float(lo.x);
-                        if constexpr (Bucket::compact)
-                            cand = Cand{kNone, first ? lo.y : lo.z, 0, false, 0};
-                        else if constexpr (Bucket::cursor)
-                            cand = Cand{kNone, first ? lo.y : lo.z,
-                                        first ? ((uint64_t)hi.y << 32) | hi.x : ((uint64_t)hi.w << 32) | hi.z, true, 0};
+                        if constexpr (Bucket::compact || Bucket::cursor)
+                            cand = first ? lo.y : lo.z;
                         else
-                            cand = Cand{kNone, first ? hi.x : hi.y, 0, false, 0};
-                        dart = map_gen_float(coin ? wd.z : wd.y, P.upperbound);
+                            cand = first ? hi.x : hi.y;
+                        if constexpr (Bucket::cursor)
+                            cand_cur = first ? ((uint64_t)hi.y << 32) | hi.x : ((uint64_t)hi.w << 32) | hi.z;
+                        dart = map_gen_float(coin ? wd.z : wd.y, P.upperbound());
                         drawn += coin ? 3u : 2u;
                     }
                     else
                     {
-                        cand = Cand{kNone, lo.x, g.adjc != nullptr ? ((uint64_t)lo.w << 32) | lo.z : 0, g.adjc != nullptr,
-                                    0};
-                        dart = map_gen_float(wd.y, P.upperbound);
+                        cand = lo.x;
+                        if (g.adjc != nullptr)
+                            cand_cur = ((uint64_t)lo.w << 32) | lo.z;
+                        dart = map_gen_float(wd.y, P.upperbound());
                         drawn += 2u;
                     }
-                    taken = dart <= P.lowerbound;
+                    taken = dart <= P.lowerbound();
                 }
                 rng.take(drawn, nxt);
-                const bool back = prev == cand.nbr;
-                if (!taken && some && step != 0 && !back && !(dart <= P.sure_below))
+                const bool back = prev == cand;
+                if (!taken && some && step != 0 && !back && !(dart <= P.sure_below()))
                 {
                     query = true;
-                    run.queries++;
-                    sec = edge_set_sector(cand.nbr, pn);
+                    if (stats != nullptr)
+                        atomicAdd(stats + 1, 1ull);
+                    sec = edge_set_sector(cand, pn);
                 }
                 else if (!taken && some)
                 {
-                    taken = dart <= (step == 0 ? P.upperbound : back ? P.inv_p : P.inv_q);
+                    taken = dart <= (step == 0 ? P.upperbound() : back ? P.inv_p() : P.inv_q());
                 }
-                if (++trials > L.trial_limit)
-                {
-                    /* this trial was one too many */
-                    atomicOr(L.status, KK_STATUS_TRIAL_LIMIT);
-                    run.trials += trials;
-                    alive = taken = false;
-                }
+                if (stats != nullptr)
+                    atomicAdd(stats, 1ull);
+                if (++trials > trial_limit)
+                    alive = taken = within = false; /* this trial was one too many */
             }
             if (taken)
             {
-                run.trials += trials;
                 step++;
-                prow = edge_set_row(pos.e0, v);
-                pn = edge_set_sectors(pos.deg);
+                prow = (uint32_t)edge_set_row(pb, v, Weighted);
+                pn = edge_set_sectors(pe - pb, Weighted);
                 prev = v;
-                v = cand.nbr;
-                if (run.out != nullptr)
-                    run.out[step] = v;
-                pos = cand.has_cur ? pos_from_cursor(g, v, cand.cur) : pos_from_offsets(g, v);
+                v = cand;
+                if (out != nullptr)
+                    out[step] = v;
+                bool cursor = false;
+                if constexpr (Weighted)
+                    cursor = Bucket::cursor && cand_cur != ~0ull;
+                else
+                    cursor = g.adjc != nullptr && cand_cur != ~0ull;
+                if (cursor)
+                {
+                    const Pos np = pos_from_cursor(g, v, cand_cur);
+                    pb = (uint32_t)np.e0;
+                    pe = pb + np.deg;
+                }
+                else
+                {
+                    pb = gather(g.off32 + v);
+                    pe = gather(g.off32 + v + 1);
+                }
                 begin_step();
-                alive = step < P.walk_length;
+                alive = step < P.walk_length();
             }
         }
     }
-    run.len = step + 1;
+    len = step + 1;
+    return within;
 }
 
 /* One thread per walker for its whole walk. */
 template <bool Weighted, bool Outlier, typename Bucket>
 __global__ void __launch_bounds__(256, 4) n2v_walk_kernel(GraphView g, N2vTables<Bucket> t, N2vParams P, WalkLaunch L)
 {
-    unsigned long long my_steps = 0;
-    WalkCounts counts;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned team = __ballot_sync(kFullMask, i < L.walker_num);
+    unsigned long long my_steps = 0;
     if (i < L.walker_num)
     {
         Sampler rng;
@@ -315,11 +364,15 @@ __global__ void __launch_bounds__(256, 4) n2v_walk_kernel(GraphView g, N2vTables
         WalkerRun<apps::Node2vecState> run;
         WalkerConfig<apps::Node2vecState> wc;
         walk_begin<apps::Node2vecState>(g, wc, L, i, run, rng);
-        n2v_walk<Weighted, Outlier, Bucket>(g, t, P, L, team, run, rng);
-        walk_finish<apps::Node2vecState>(L, i, run, my_steps, counts);
+        uint32_t len;
+        if (!n2v_walk<Weighted, Outlier, Bucket>(g, t, N2vInRegs{P}, run.w.id, run.v, run.out, L.trial_limit, L.stats, team, rng,
+                                                 len))
+            atomicOr(L.status, KK_STATUS_TRIAL_LIMIT);
+        L.length[i] = len;
+        segment_done(L, i);
+        my_steps = len - 1;
     }
     flush_steps(L.total_steps, my_steps);
-    counts.flush(L.stats);
 }
 
 /* Whether a transition is node2vec's, with its outlier or without. */
@@ -351,14 +404,13 @@ N2vParams n2v_params(const TC &tc)
 }
 
 /* The batch kernel (walk_batch_kernel) of node2vec jobs over the edge set.  A
- * warp may hold walkers of several jobs: the lanes of its last pass over the
- * walkers are its team. */
-template <bool Weighted, typename Bucket>
-__global__ void __launch_bounds__(256, KK_BATCH_MINB)
-    n2v_batch_kernel(GraphView g, apps::Node2vecBatch<Weighted> app, N2vTables<Bucket> t, const BatchJob *jobs,
-                     uint32_t njobs, uint32_t total, uint32_t *path, uint32_t *length,
-                     unsigned long long *total_steps, int *status, uint32_t trial_limit, unsigned long long *stats,
-                     const uint32_t *hdr, BatchNotify nt)
+ * warp may hold walkers of several jobs: the lanes that take a walker in a pass
+ * over the batch are its team. */
+template <bool Weighted, typename Bucket, int MinBlocks>
+__global__ void __launch_bounds__(256, MinBlocks)
+    n2v_batch_kernel(GraphView g, N2vTables<Bucket> t, const BatchJob *jobs, uint32_t njobs, uint32_t total,
+                     uint32_t *path, uint32_t *length, unsigned long long *total_steps, int *status,
+                     uint32_t trial_limit, unsigned long long *stats, const uint32_t *hdr, BatchNotify nt)
 {
     __shared__ uint32_t s_first[2 * kMaxBatchJobs];
     if (hdr != nullptr)
@@ -374,35 +426,61 @@ __global__ void __launch_bounds__(256, KK_BATCH_MINB)
     }
     __syncthreads();
     unsigned long long my_steps = 0;
-    WalkCounts counts;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; at < total; at += stride)
     {
         const unsigned team = __activemask();
-        typename apps::Node2vecBatch<Weighted>::WC wc;
-        typename apps::Node2vecBatch<Weighted>::TC tc;
-        WalkLaunch L;
-        WalkerRun<apps::Node2vecState> run;
+        /* the walker's job, by its position in the launch order */
+        uint32_t k = 0, hi = njobs;
+        while (hi - k > 1)
+        {
+            const uint32_t mid = (k + hi) >> 1;
+            if (s_first[mid] <= (uint32_t)at)
+                k = mid;
+            else
+                hi = mid;
+        }
+        const BatchJob *job = jobs + s_first[kMaxBatchJobs + k];
+        const uint32_t i = (uint32_t)at - s_first[k], cap = job->cap;
         Sampler rng;
-        const uint32_t i = batch_walker_begin<apps::Node2vecState>(g, app, jobs, s_first, njobs, (uint32_t)at, t.sum,
-                                                                  path, length, total_steps, status, trial_limit, wc,
-                                                                  tc, L, run, rng, nt);
-        N2vParams P;
-        P.upperbound = tc.dcomp_upperbound.value;
-        P.lowerbound = tc.dcomp_lowerbound.value;
-        P.overflow = tc.outlier_upperbound.overflow;
-        P.inv_p = tc.dynamic_comp.inv_p;
-        P.inv_q = tc.dynamic_comp.inv_q;
-        P.sure_below = tc.post_query.sure_below;
-        P.walk_length = tc.extension_comp.walk_length;
-        n2v_walk<Weighted, true, Bucket>(g, t, P, L, team, run, rng);
-        L.length[i] = run.len;
+        rng.init(job->seed);
+        const walker_id_t id = job->walker_begin + i;
+        const vertex_id_t v = id % g.V;
+        uint32_t *out = path != nullptr ? path + job->path_base + (uint64_t)i * cap : nullptr;
+        if (out != nullptr)
+            out[0] = v;
+        uint32_t len;
+        bool within;
+        if constexpr (MinBlocks >= 4)
+        {
+            within = n2v_walk<Weighted, true, Bucket>(g, t, N2vInJob{job}, id, v, out, trial_limit, stats, team, rng,
+                                                      len);
+        }
+        else
+        {
+            const N2vParams P{job->c[0], job->c[1], job->c[2], job->c[3], job->c[4], fminf(job->c[4], 1.0f),
+                              job->walk_length};
+            within = n2v_walk<Weighted, true, Bucket>(g, t, N2vInRegs{P}, id, v, out, trial_limit, stats, team, rng,
+                                                      len);
+        }
+        const uint32_t j = (uint32_t)(job - jobs);
+        if (!within)
+            atomicOr(nt.count != nullptr ? nt.status + j : status, KK_STATUS_TRIAL_LIMIT);
+        length[job->first_task + i] = len;
+        my_steps += len - 1;
+        WalkLaunch L;
+        if (nt.count != nullptr)
+        {
+            /* the job is one segment of its own */
+            L.walker_num = job->walker_num;
+            L.seg_count = nt.count + j;
+            L.seg_flag = nt.flag + j;
+            L.seg_shift = 31;
+            L.seg_status = nt.status + j;
+        }
         segment_done(L, i);
-        my_steps += run.len - 1;
-        counts.add(run);
     }
     flush_steps(total_steps, my_steps);
-    counts.flush(stats);
 }
 
 } // namespace kk

@@ -111,38 +111,39 @@ struct SecondOrderTransitionConfig
 
 /* ---- edge set ---------------------------------------------------------------
  * Exact lookup of directed edges (u, v): an open-addressing table of 32-bit
- * neighbour ids per row, in 32 B sectors of eight slots.  Row u of degree d at
- * offset e0 has d / 4 + 1 sectors from sector e0 / 4 + u on (rows do not
- * overlap: (e0 + d) / 4 >= e0 / 4 + d / 4), so a lookup finds the row's table
- * from its adjacency position alone, the load is below 1/2, and the whole set
- * takes 8 B an edge and 32 B a vertex: it stays in L2 eight times longer than
- * a table of 64-bit (u, v) keys at load 1/4 in 64 B buckets did.  v's probe
- * starts at sector edge_set_sector(v) of the row and goes on in turn; an
- * insert moves past a sector only when its eight slots hold other ids, so a
- * lookup that meets a free slot may stop.  Beside the ids, the weight of
- * (u, v)'s first edge in u's sorted adjacency, std::lower_bound's (weighted
- * graphs; the same slot of a parallel array). */
-constexpr uint32_t kEdgeSetSlots = 8; /* a sector's slots; kNone: free */
+ * neighbour ids per row, in sectors of 32 B: eight ids, or in a weighted graph
+ * four ids and their edges' weights (the weight of (u, v)'s first edge in u's
+ * sorted adjacency, std::lower_bound's), so that either lookup is one read.
+ * Row u of degree d at offset e0 has d / 4 + 1 sectors from sector e0 / 4 + u
+ * on, weighted d / 2 + 1 from e0 / 2 + u (rows do not overlap: (e0 + d) / 4 >=
+ * e0 / 4 + d / 4), so a lookup finds the row's table from its adjacency
+ * position alone, the load is below 1/2, and the set takes 8 or 16 B an edge
+ * and 32 B a vertex: it stays in L2 where a table of 64-bit (u, v) keys at
+ * load 1/4 in 64 B buckets did not.  v's probe starts at sector
+ * edge_set_sector(v) of the row and goes on in turn; an insert moves past a
+ * sector only when its slots hold other ids, so a lookup that meets a free
+ * slot may stop. */
+constexpr uint32_t kEdgeSectorWords = 8;
 
 struct EdgeSetView
 {
     const uint32_t *keys; /* nullptr: no set */
-    const float *w;       /* nullptr: unweighted */
+    bool weighted;
     const int64_t *off;
 };
 
-__host__ __device__ __forceinline__ uint64_t edge_set_row(int64_t e0, vertex_id_t u)
+__host__ __device__ __forceinline__ uint64_t edge_set_row(int64_t e0, vertex_id_t u, bool weighted)
 {
-    return ((uint64_t)e0 >> 2) + u;
+    return ((uint64_t)e0 >> (weighted ? 1 : 2)) + u;
 }
-__host__ __device__ __forceinline__ uint32_t edge_set_sectors(uint32_t deg)
+__host__ __device__ __forceinline__ uint32_t edge_set_sectors(uint32_t deg, bool weighted)
 {
-    return (deg >> 2) + 1;
+    return (deg >> (weighted ? 1 : 2)) + 1;
 }
 /* all rows' sectors */
-__host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t V)
+__host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t V, bool weighted)
 {
-    return (E >> 2) + V + 1;
+    return (E >> (weighted ? 1 : 2)) + V + 1;
 }
 /* where v's probe starts among a row's n sectors */
 __host__ __device__ __forceinline__ uint32_t edge_set_sector(vertex_id_t v, uint32_t n)
@@ -152,16 +153,26 @@ __host__ __device__ __forceinline__ uint32_t edge_set_sector(vertex_id_t v, uint
     return mulhi32(a * 0x85EBCA6Bu, n);
 }
 
-/* Sector {a, b} against id v: the slot that holds it, 8 for a free slot (v is
- * not in the row), 9 for neither (the next sector decides). */
+/* A sector's ids against id v: the slot that holds it, 8 for a free slot (v is
+ * not in the row), 9 for neither (the next sector decides).  Slots fill from
+ * the first on. */
+__device__ __forceinline__ uint32_t edge_set_match(const uint4 &a, vertex_id_t v)
+{
+    uint32_t r = a.w == kNone ? 8u : 9u;
+    r = a.x == v ? 0u : r;
+    r = a.y == v ? 1u : r;
+    r = a.z == v ? 2u : r;
+    return a.w == v ? 3u : r;
+}
 __device__ __forceinline__ uint32_t edge_set_match(const uint4 &a, const uint4 &b, vertex_id_t v)
 {
-    const uint32_t k[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t r = k[7] == kNone ? 8u : 9u; /* slots fill from the first on */
-#pragma unroll
-    for (uint32_t j = 0; j < 8; j++)
-        r = k[j] == v ? j : r;
-    return r;
+    const uint32_t m = edge_set_match(b, v), l = edge_set_match(a, v);
+    return l < 4 ? l : m < 4 ? m + 4 : m;
+}
+__device__ __forceinline__ uint32_t word_of(const uint4 &a, uint32_t j)
+{
+    const uint32_t lo = j & 1 ? a.y : a.x, hi = j & 1 ? a.w : a.z;
+    return j & 2 ? hi : lo;
 }
 
 /* Whether (u, v) is an edge, u's adjacency being deg edges from e0, and its
@@ -169,18 +180,18 @@ __device__ __forceinline__ uint32_t edge_set_match(const uint4 &a, const uint4 &
 __device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t u, int64_t e0, uint32_t deg,
                                               vertex_id_t v, float *weight)
 {
-    const uint64_t row = edge_set_row(e0, u);
-    const uint32_t n = edge_set_sectors(deg);
+    const uint64_t row = edge_set_row(e0, u, s.weighted);
+    const uint32_t n = edge_set_sectors(deg, s.weighted);
     uint32_t b = edge_set_sector(v, n);
     for (uint32_t probe = 0; probe < n; probe++)
     {
-        const uint64_t at = (row + b) * kEdgeSetSlots;
-        const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + at);
-        const uint32_t m = edge_set_match(__ldg(p), __ldg(p + 1), v);
+        const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + (row + b) * kEdgeSectorWords);
+        const uint4 x = __ldg(p), y = __ldg(p + 1);
+        const uint32_t m = s.weighted ? edge_set_match(x, v) : edge_set_match(x, y, v);
         if (m < 8)
         {
             if (weight != nullptr)
-                *weight = gather(s.w + at + m);
+                *weight = __uint_as_float(word_of(y, m));
             return true;
         }
         if (m == 8)
@@ -191,46 +202,55 @@ __device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t 
 }
 
 /* Puts v (not yet in the row) into the row of n sectors at keys, in shared or
- * global memory; its slot. */
-__device__ __forceinline__ uint32_t edge_set_insert(uint32_t *keys, uint32_t n, vertex_id_t v)
+ * global memory; the word it takes. */
+__device__ __forceinline__ uint32_t edge_set_insert(uint32_t *keys, uint32_t n, vertex_id_t v, bool weighted)
 {
     uint32_t b = edge_set_sector(v, n);
     for (;;) /* ends: the row has more slots than ids */
     {
-        for (uint32_t j = 0; j < kEdgeSetSlots; j++)
+        for (uint32_t j = 0; j < (weighted ? 4u : 8u); j++)
         {
-            uint32_t *k = keys + b * kEdgeSetSlots + j;
+            uint32_t *k = keys + (uint64_t)b * kEdgeSectorWords + j;
             if (*(volatile uint32_t *)k == kNone && atomicCAS(k, kNone, v) == kNone)
-                return b * kEdgeSetSlots + j;
+                return b * kEdgeSectorWords + j;
         }
         b = b + 1 == n ? 0 : b + 1;
     }
 }
 
+/* Edges threadIdx-wise i, i + step, ... of a row into its table.  The
+ * adjacency is sorted, so an id's first edge is the one that differs from the
+ * edge before it. */
+__device__ __forceinline__ void edge_set_fill(const GraphView &g, int64_t e0, uint32_t deg, uint32_t *row, uint32_t n,
+                                              uint32_t i, uint32_t step)
+{
+    const bool weighted = g.w != nullptr;
+    for (; i < deg; i += step)
+    {
+        const uint32_t v = g.nbr[e0 + i];
+        if (i > 0 && g.nbr[e0 + i - 1] == v)
+            continue;
+        const uint32_t at = edge_set_insert(row, n, v, weighted);
+        if (weighted)
+            row[at + 4] = __float_as_uint(g.w[e0 + i]);
+    }
+}
+
 /* The rows order[lo, hi), a block each (hubs): the row's table in global
- * memory.  The adjacency is sorted, so an id's first edge is the one that
- * differs from the edge before it. */
-static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g, uint32_t *keys, float *w,
+ * memory. */
+static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g, uint32_t *keys,
                                                                      const uint32_t *order, uint32_t lo, uint32_t hi)
 {
     for (uint32_t k = lo + blockIdx.x; k < hi; k += gridDim.x)
     {
         const uint32_t u = order[k];
         const int64_t e0 = g.off[u];
-        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg);
-        const uint64_t at = edge_set_row(e0, u) * kEdgeSetSlots;
-        for (uint32_t i = threadIdx.x; i < n * kEdgeSetSlots; i += blockDim.x)
-            keys[at + i] = kNone;
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, g.w != nullptr);
+        uint32_t *row = keys + edge_set_row(e0, u, g.w != nullptr) * kEdgeSectorWords;
+        for (uint32_t i = threadIdx.x; i < n * kEdgeSectorWords; i += blockDim.x)
+            row[i] = kNone;
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < deg; i += blockDim.x)
-        {
-            const uint32_t v = g.nbr[e0 + i];
-            if (i > 0 && g.nbr[e0 + i - 1] == v)
-                continue;
-            const uint32_t slot = edge_set_insert(keys + at, n, v);
-            if (w != nullptr)
-                w[at + slot] = g.w[e0 + i];
-        }
+        edge_set_fill(g, e0, deg, row, n, threadIdx.x, blockDim.x);
         __syncthreads();
     }
 }
@@ -239,46 +259,32 @@ static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g
  * in shared memory (its inserts are chains of atomics, ten times shorter there
  * than in L2), then out in one coalesced pass. */
 template <uint32_t DMAX>
-constexpr uint32_t edge_set_group_words()
+constexpr uint32_t edge_set_group_words(bool weighted)
 {
-    return (DMAX / 4 + 1) * kEdgeSetSlots;
+    return (DMAX / (weighted ? 2 : 4) + 1) * kEdgeSectorWords;
 }
 
 template <uint32_t G, uint32_t DMAX>
-static __global__ void __launch_bounds__(128) edge_set_group_kernel(GraphView g, uint32_t *keys, float *w,
+static __global__ void __launch_bounds__(128) edge_set_group_kernel(GraphView g, uint32_t *keys,
                                                                     const uint32_t *order, uint32_t lo, uint32_t hi)
 {
     extern __shared__ uint32_t s_rows[];
-    constexpr uint32_t W = edge_set_group_words<DMAX>();
     const uint32_t gl = threadIdx.x % G, grp = threadIdx.x / G, groups = blockDim.x / G;
     const unsigned mask = G == 32 ? kFullMask : ((1u << (G % 32)) - 1u) << (threadIdx.x % 32 / G * G);
-    uint32_t *tk = s_rows + grp * W * (w != nullptr ? 2 : 1);
-    float *tw = reinterpret_cast<float *>(tk + W);
+    uint32_t *row = s_rows + grp * edge_set_group_words<DMAX>(g.w != nullptr);
     for (uint32_t k = lo + blockIdx.x * groups + grp; k < hi; k += gridDim.x * groups)
     {
         const uint32_t u = order[k];
         const int64_t e0 = g.off[u];
-        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg);
-        for (uint32_t i = gl; i < n * kEdgeSetSlots; i += G)
-            tk[i] = kNone;
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, g.w != nullptr);
+        for (uint32_t i = gl; i < n * kEdgeSectorWords; i += G)
+            row[i] = kNone;
         __syncwarp(mask);
-        for (uint32_t i = gl; i < deg; i += G)
-        {
-            const uint32_t v = g.nbr[e0 + i];
-            if (i > 0 && g.nbr[e0 + i - 1] == v)
-                continue;
-            const uint32_t slot = edge_set_insert(tk, n, v);
-            if (w != nullptr)
-                tw[slot] = g.w[e0 + i];
-        }
+        edge_set_fill(g, e0, deg, row, n, gl, G);
         __syncwarp(mask);
-        const uint64_t at = edge_set_row(e0, u) * kEdgeSetSlots;
-        for (uint32_t i = gl; i < n * kEdgeSetSlots; i += G)
-        {
-            keys[at + i] = tk[i];
-            if (w != nullptr)
-                w[at + i] = tw[i];
-        }
+        const uint64_t at = edge_set_row(e0, u, g.w != nullptr) * kEdgeSectorWords;
+        for (uint32_t i = gl; i < n * kEdgeSectorWords; i += G)
+            keys[at + i] = row[i];
         __syncwarp(mask);
     }
 }

@@ -101,6 +101,20 @@ BatchPlan plan_batch(kk_engine *e, const kk_walk_opts *jobs, int n, bool longest
 namespace
 {
 
+/* node2vec batches of no more walkers than four blocks of 256 an SM wait on
+ * latency: their kernel keeps a walk's state in registers at two blocks an SM
+ * (20 jobs, 148,000 walkers, 32 M edges: walk 2.17 -> 1.55 ms); a larger batch
+ * is bound by the reads of all SMs (512 jobs on R-MAT 22: 15.5 ms at four
+ * blocks, 18.3 at two). */
+uint32_t batch_wide_limit(const kk_engine *e)
+{
+    return 1024u * (uint32_t)e->sm_count;
+}
+bool batch_wide(const kk_engine *e, const BatchPlan &plan)
+{
+    return plan.app == KK_APP_NODE2VEC && plan.total <= batch_wide_limit(e);
+}
+
 /* Launches the batch on the slot, reading alias tables in the Bucket layout
  * (built on the engine's stream first unless prepared). */
 template <typename App, typename Bucket>
@@ -138,7 +152,7 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
     unsigned long long *st = e->walk_stats ? steps + 1 : nullptr;
     if (e->walk_schedule == 0)
     {
-        unsigned grid = grid_for(e, walkers, bs);
+        unsigned grid = grid_for(e, hdr && batch_wide(e, plan) ? std::min(walkers, batch_wide_limit(e)) : walkers, bs);
         if (hdr && grid > 64u * (unsigned)e->sm_count)
             grid = 64u * (unsigned)e->sm_count; /* grid-stride over whatever the header holds */
         /* parking (first-order rejection walks) on the engine's own batch
@@ -162,12 +176,17 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
         bool launched = false;
         if constexpr (is_node2vec<TC>::value)
         {
-            if (app.set.keys != nullptr)
+            if (app.set.keys != nullptr && gv.off32 != nullptr)
             {
                 const N2vTables<Bucket> t{alias, (const float *)e->sum.p, nullptr, app.set};
-                n2v_batch_kernel<TC::has_static, Bucket><<<grid, bs, 0, slot.stream>>>(
-                    gv, app, t, d_jobs, nj, plan.total, *path, length, steps, status, e->trial_limit, st, hdr,
-                    slot.notify);
+                auto launch = [&](auto kern) {
+                    kern<<<grid, bs, 0, slot.stream>>>(gv, t, d_jobs, nj, plan.total, *path, length, steps, status,
+                                                       e->trial_limit, st, hdr, slot.notify);
+                };
+                if (batch_wide(e, plan))
+                    launch(n2v_batch_kernel<TC::has_static, Bucket, 2>);
+                else
+                    launch(n2v_batch_kernel<TC::has_static, Bucket, 4>);
                 launched = true;
             }
         }
@@ -415,7 +434,9 @@ static void launch_batch_graph(kk_engine *e, BatchPlan &plan, BatchSlot &slot)
         memcpy(h.schemes, plan.schemes.data(), plan.schemes.size() * sizeof(MetaSchemes));
     h.hdr[0] = nj;
     h.hdr[1] = plan.total;
-    if (slot.exec == nullptr)
+    /* one graph per kernel a batch's size may ask for */
+    cudaGraphExec_t &exec = slot.exec[batch_wide(e, plan) ? 1 : 0];
+    if (exec == nullptr)
     {
         cudaGraph_t graph = nullptr;
         KK_CUDA_CHECK(cudaStreamBeginCapture(slot.stream, cudaStreamCaptureModeThreadLocal));
@@ -446,12 +467,12 @@ static void launch_batch_graph(kk_engine *e, BatchPlan &plan, BatchSlot &slot)
             throw;
         }
         KK_CUDA_CHECK(cudaStreamEndCapture(slot.stream, &graph));
-        const cudaError_t ie = cudaGraphInstantiate(&slot.exec, graph, 0);
+        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         KK_CUDA_CHECK(ie);
     }
     KK_CUDA_CHECK(cudaEventRecord(slot.ev[1], slot.stream));
-    KK_CUDA_CHECK(cudaGraphLaunch(slot.exec, slot.stream));
+    KK_CUDA_CHECK(cudaGraphLaunch(exec, slot.stream));
     KK_CUDA_CHECK(cudaEventRecord(slot.ev[2], slot.stream));
 }
 

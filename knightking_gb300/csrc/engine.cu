@@ -798,7 +798,6 @@ void kk_engine_destroy(kk_engine *e)
         e->host_pool->release();
     e->vcur.release();
     e->edge_set.release();
-    e->edge_set_w.release();
     e->bslot.release();
     if (e->hub)
     {

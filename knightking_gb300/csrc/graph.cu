@@ -283,17 +283,16 @@ const uint4 *cursor_adjacency_of(kk_engine *e)
 EdgeSetView node2vec_edge_set_built(const kk_engine *e)
 {
     if (e->n2v_adjacency != 0)
-        return EdgeSetView{nullptr, nullptr, nullptr};
-    return EdgeSetView{(const uint32_t *)e->edge_set.p, e->d_w ? (const float *)e->edge_set_w.p : nullptr, e->d_off};
+        return EdgeSetView{nullptr, false, nullptr};
+    return EdgeSetView{(const uint32_t *)e->edge_set.p, e->d_w != nullptr, e->d_off};
 }
 
 EdgeSetView node2vec_edge_set(kk_engine *e)
 {
     if (e->n2v_adjacency != 0 || e->edge_set_valid)
         return node2vec_edge_set_built(e);
-    const uint64_t words = edge_set_total(e->E, e->V) * kEdgeSetSlots;
-    uint32_t *keys = e->edge_set.as<uint32_t>(words);
-    float *w = e->d_w ? e->edge_set_w.as<float>(words) : nullptr;
+    const bool weighted = e->d_w != nullptr;
+    uint32_t *keys = e->edge_set.as<uint32_t>(edge_set_total(e->E, e->V, weighted) * kEdgeSectorWords);
     const uint32_t *order = vertex_order(e);
     const GraphView g = e->view();
     const uint32_t *t = e->tier;
@@ -301,24 +300,32 @@ EdgeSetView node2vec_edge_set(kk_engine *e)
      * their tables in shared memory: the classes of the vertex order */
     if (t[3])
     {
-        edge_set_block_kernel<<<t[3] < 2u * e->sm_count ? t[3] : 2u * e->sm_count, 1024, 0, e->stream>>>(g, keys, w,
-                                                                                                        order, 0, t[3]);
+        const uint32_t cap = 2u * (uint32_t)e->sm_count;
+        edge_set_block_kernel<<<t[3] < cap ? t[3] : cap, 1024, 0, e->stream>>>(g, keys, order, 0, t[3]);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
     auto group = [&](auto kern, uint32_t G, uint32_t row_words, uint32_t lo, uint32_t hi) {
         if (hi <= lo)
             return;
-        const size_t smem = (size_t)(128 / G) * row_words * (w ? 8 : 4);
+        const size_t smem = (size_t)(128 / G) * row_words * sizeof(uint32_t);
         KK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid_for(e, hi - lo, 128 / G), 128, smem, e->stream>>>(g, keys, w, order, lo, hi);
+        kern<<<grid_for(e, hi - lo, 128 / G), 128, smem, e->stream>>>(g, keys, order, lo, hi);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     };
-    group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(), t[3], t[4]);
-    group(edge_set_group_kernel<32, 512>, 32, edge_set_group_words<512>(), t[4], t[5]);
-    group(edge_set_group_kernel<16, 128>, 16, edge_set_group_words<128>(), t[5], t[6]);
-    group(edge_set_group_kernel<8, 32>, 8, edge_set_group_words<32>(), t[6], e->n_nz);
+    if (e->E < 1u << 20)
+    {
+        /* a launch a class costs more than their lanes save */
+        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(weighted), t[3], e->n_nz);
+    }
+    else
+    {
+        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(weighted), t[3], t[4]);
+        group(edge_set_group_kernel<32, 512>, 32, edge_set_group_words<512>(weighted), t[4], t[5]);
+        group(edge_set_group_kernel<16, 128>, 16, edge_set_group_words<128>(weighted), t[5], t[6]);
+        group(edge_set_group_kernel<8, 32>, 8, edge_set_group_words<32>(weighted), t[6], e->n_nz);
+    }
     e->edge_set_valid = true;
     return node2vec_edge_set_built(e);
 }
