@@ -83,6 +83,20 @@ struct DevBuf
     }
 };
 
+/* A graph's arrays in HBM. */
+struct GraphBufs
+{
+    DevBuf off, nbr, w, type;
+    size_t bytes() const { return off.bytes + nbr.bytes + w.bytes + type.bytes; }
+    void release()
+    {
+        off.release();
+        nbr.release();
+        w.release();
+        type.release();
+    }
+};
+
 /* Where one walk call's results are (device). */
 struct WalkResult
 {
@@ -312,6 +326,11 @@ struct kk_engine
     uint32_t *d_nbr = nullptr;
     float *d_w = nullptr;
     uint8_t *d_type = nullptr;
+    /* the arrays' memory, kept from graph to graph (an allocation and a free
+     * take 40 to 80 us each), and the set the next graph is put in, so that a
+     * refused one leaves this one as it is */
+    kk::GraphBufs gb, gnext;
+    kk::DevBuf order_tmp; /* vertex_order's degrees and ids */
     /* the offsets as 32-bit words, made with the graph when E < 2^32
      * (compact_offsets, an option: 0 makes the walks read the 64-bit ones) */
     kk::DevBuf off32;
@@ -1227,6 +1246,9 @@ void run_app_node2vec(kk_engine *e, const kk_walk_opts &o, const RunSpec &rs, Wa
  * the engine's stream. */
 void graph_offsets32(kk_engine *e);
 void graph_check_sorted(kk_engine *e);
+/* The graph in gnext's arrays (V vertices, E edges, with weights, with types)
+ * becomes the engine's; sorted: -1 unknown, 0, 1. */
+void graph_commit(kk_engine *e, uint32_t V, uint64_t E, bool w, bool type, int sorted);
 void graph_sort_adjacency(kk_engine *e);
 
 /* Runs one epoch of a walk: fills the WalkResult for rs's walkers. */

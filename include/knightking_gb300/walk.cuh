@@ -1861,12 +1861,14 @@ static __global__ void row_desc_kernel(GraphView g, const uint32_t *order, RowDe
     }
 }
 
-/* Degree-descending vertex order support: degrees and iota for a radix sort. */
+/* Degree-descending vertex order support: degrees (of at most 65535) and iota
+ * for a radix sort. */
 static __global__ void degree_keys_kernel(GraphView g, uint32_t *deg, uint32_t *ids)
 {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += gridDim.x * blockDim.x)
     {
-        deg[v] = (uint32_t)(g.off[v + 1] - g.off[v]);
+        const int64_t d = g.off[v + 1] - g.off[v];
+        deg[v] = d < 65535 ? (uint32_t)d : 65535u;
         ids[v] = v;
     }
 }

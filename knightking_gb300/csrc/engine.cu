@@ -21,14 +21,6 @@
 
 void kk_engine::free_graph()
 {
-    if (d_off)
-        cudaFree(d_off);
-    if (d_nbr)
-        cudaFree(d_nbr);
-    if (d_w)
-        cudaFree(d_w);
-    if (d_type)
-        cudaFree(d_type);
     d_off = nullptr;
     d_nbr = nullptr;
     d_w = nullptr;
@@ -51,8 +43,6 @@ void kk_engine::free_graph()
 
 namespace kk
 {
-void graph_upload(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const float *w,
-                  const uint8_t *type);
 void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const float *w,
                        const uint8_t *type);
 void graph_load_binary(kk_engine *e, uint32_t V, const char *path, int kind, int undirected);
@@ -736,6 +726,9 @@ void kk_engine_destroy(kk_engine *e)
     e->rows.release();
     e->adjc.release();
     e->off32.release();
+    e->gb.release();
+    e->gnext.release();
+    e->order_tmp.release();
     if (e->h_status)
         cudaFreeHost(e->h_status);
     for (int r = 0; r < kk_engine::kReaders; r++)

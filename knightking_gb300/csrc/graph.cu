@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 #include <memory>
 #include <string>
 #include <thread>
@@ -35,6 +36,9 @@
 
 namespace kk
 {
+
+/* Memory a load leaves for the next one: up to this much is kept. */
+constexpr size_t kKeepBytes = (size_t)1 << 30;
 
 void exclusive_scan_u64(kk_engine *e, const uint64_t *in, uint64_t *out, uint64_t n, cudaStream_t st, DevBuf &tmpb)
 {
@@ -62,18 +66,199 @@ void sort_pairs_u32(kk_engine *e, const uint32_t *keys_in, uint32_t *keys_out, c
 namespace
 {
 
-__global__ void check_sorted_kernel(const int64_t *off, const uint32_t *nbr, uint32_t V, int *unsorted)
+/* What a pass over a graph's arrays tells (one 64-bit word each): bad marks,
+ * the descents between consecutive neighbours, and those of them that lie
+ * between two rows.  The adjacency is sorted when all of them do. */
+enum : int
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+    kScanBad = 0, /* an OR of the marks below */
+    kScanDescents,
+    kScanBetween,
+    kScanWords
+};
+enum : unsigned
+{
+    kBadNeighbour = 1,
+    kBadOffsets = 2,
+    kBadType = 4
+};
+
+__device__ __forceinline__ void scan_out(unsigned long long *out, unsigned bad, uint32_t descents, int word)
+{
+    bad = __reduce_or_sync(kFullMask, bad);
+    descents = __reduce_add_sync(kFullMask, descents);
+    if ((threadIdx.x & 31) == 0)
     {
-        for (int64_t e = off[v] + 1; e < off[v + 1]; e++)
+        if (bad)
+            atomicOr(out + kScanBad, (unsigned long long)bad);
+        if (descents)
+            atomicAdd(out + word, (unsigned long long)descents);
+    }
+}
+
+/* Every thread of a full block takes part (the grid is rounded up). */
+__global__ void edge_scan_kernel(const uint32_t *nbr, const uint8_t *type, uint64_t E, uint32_t V,
+                                 unsigned long long *out)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    unsigned bad = 0;
+    uint32_t descents = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += stride)
+    {
+        const uint32_t v = nbr[i];
+        if (v >= V)
+            bad |= kBadNeighbour;
+        if (type != nullptr && type[i] >= 8)
+            bad |= kBadType;
+        descents += i > 0 && nbr[i - 1] > v;
+    }
+    __syncwarp();
+    scan_out(out, bad, descents, kScanDescents);
+}
+
+__global__ void vertex_scan_kernel(const int64_t *off, const uint32_t *nbr, uint64_t E, uint32_t V,
+                                   unsigned long long *out)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    unsigned bad = 0;
+    uint32_t between = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += stride)
+    {
+        const int64_t a = off[v], b = off[v + 1];
+        if (b < a)
+            bad |= kBadOffsets;
+        /* in range whatever the other offsets are */
+        if (b > a && a > 0 && (uint64_t)a < E)
+            between += nbr[a - 1] > nbr[a];
+    }
+    __syncwarp();
+    scan_out(out, bad, between, kScanBetween);
+}
+
+/* Both passes over off, nbr and type on the engine's stream; the words. */
+void scan_graph(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const uint8_t *type,
+                uint64_t words[kScanWords])
+{
+    unsigned long long *d = (unsigned long long *)e->alias_next.as<uint32_t>(16); /* free between builds */
+    KK_CUDA_CHECK(cudaMemsetAsync(d, 0, kScanWords * 8, e->stream));
+    const uint64_t cap = 16ull * (uint64_t)e->sm_count;
+    edge_scan_kernel<<<(unsigned)std::min<uint64_t>(grid_for(e, E, 256), cap), 256, 0, e->stream>>>(nbr, type, E, V,
+                                                                                                   d);
+    count_launch(e);
+    vertex_scan_kernel<<<(unsigned)std::min<uint64_t>(grid_for(e, V, 256), cap), 256, 0, e->stream>>>(off, nbr, E, V,
+                                                                                                     d);
+    count_launch(e);
+    KK_CUDA_CHECK(cudaGetLastError());
+    words_to_host(e, (const uint32_t *)d, 48, 2 * kScanWords);
+    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
+    memcpy(words, (const char *)e->h_status + 48 * 4, kScanWords * 8);
+}
+
+/* Rows of at most 128 edges by rank: lane i of a group of G takes elements i,
+ * i + G, ..., whose place is the number of smaller neighbours in the row and
+ * of equal ones before them (stable).  The ids stand in shared memory, read by
+ * all lanes at once; weights and types go straight to their places. */
+constexpr uint32_t kRankMax = 128;
+
+template <uint32_t G, uint32_t DMAX>
+__global__ void __launch_bounds__(128) rank_rows_kernel(const RowDesc *rows, uint32_t lo, uint32_t hi,
+                                                        const uint32_t *nbr, const float *w, const uint8_t *type,
+                                                        uint32_t *nbr_out, float *w_out, uint8_t *type_out)
+{
+    __shared__ uint32_t s_id[128 / G][DMAX];
+    const uint32_t grp = threadIdx.x / G, gl = threadIdx.x % G;
+    const unsigned mask = G == 32 ? kFullMask : ((1u << (G % 32)) - 1u) << (threadIdx.x % 32 / G * G);
+    for (uint32_t k = lo + blockIdx.x * (128 / G) + grp; k < hi; k += gridDim.x * (128 / G))
+    {
+        const RowDesc d = rows[k];
+        for (uint32_t i = gl; i < d.deg; i += G)
+            s_id[grp][i] = nbr[d.e0 + i];
+        __syncwarp(mask);
+        for (uint32_t i = gl; i < d.deg; i += G)
         {
-            if (nbr[e - 1] > nbr[e])
+            const uint32_t x = s_id[grp][i];
+            uint32_t at = 0;
+            for (uint32_t j = 0; j < d.deg; j++)
             {
-                atomicExch(unsorted, 1);
-                break;
+                const uint32_t y = s_id[grp][j];
+                at += y < x || (y == x && j < i);
             }
+            nbr_out[d.e0 + at] = x;
+            if (w != nullptr)
+                w_out[d.e0 + at] = w[d.e0 + i];
+            if (type != nullptr)
+                type_out[d.e0 + at] = type[d.e0 + i];
         }
+        __syncwarp(mask);
+    }
+}
+
+/* Rows of up to kBitonicMax edges by a bitonic sort in shared memory, a block
+ * each: the key is the id above its place in the row, so equal ids keep their
+ * order. */
+constexpr uint32_t kBitonicMax = 2048;
+
+__global__ void __launch_bounds__(256) bitonic_rows_kernel(const RowDesc *rows, uint32_t lo, uint32_t hi,
+                                                           const uint32_t *nbr, const float *w, const uint8_t *type,
+                                                           uint32_t *nbr_out, float *w_out, uint8_t *type_out)
+{
+    __shared__ uint64_t s_key[kBitonicMax];
+    for (uint32_t r = lo + blockIdx.x; r < hi; r += gridDim.x)
+    {
+        const RowDesc d = rows[r];
+        uint32_t n = 256;
+        while (n < d.deg)
+            n <<= 1;
+        for (uint32_t i = threadIdx.x; i < n; i += 256)
+            s_key[i] = i < d.deg ? ((uint64_t)nbr[d.e0 + i] << 32) | i : ~0ull;
+        __syncthreads();
+        for (uint32_t k = 2; k <= n; k <<= 1)
+            for (uint32_t j = k >> 1; j > 0; j >>= 1)
+            {
+                for (uint32_t t = threadIdx.x; t < n / 2; t += 256)
+                {
+                    const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;
+                    const uint64_t x = s_key[a], y = s_key[b];
+                    if ((x > y) == ((a & k) == 0))
+                    {
+                        s_key[a] = y;
+                        s_key[b] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        for (uint32_t i = threadIdx.x; i < d.deg; i += 256)
+        {
+            const uint64_t x = s_key[i];
+            nbr_out[d.e0 + i] = (uint32_t)(x >> 32);
+            if (w != nullptr)
+                w_out[d.e0 + i] = w[d.e0 + (uint32_t)x];
+            if (type != nullptr)
+                type_out[d.e0 + i] = type[d.e0 + (uint32_t)x];
+        }
+        __syncthreads();
+    }
+}
+
+/* Where the sort of the larger rows finds its segments. */
+struct RowBegin
+{
+    __host__ __device__ int64_t operator()(const RowDesc &d) const { return d.e0; }
+};
+struct RowEnd
+{
+    __host__ __device__ int64_t operator()(const RowDesc &d) const { return d.e0 + (int64_t)d.deg; }
+};
+
+/* The arrays of the row's other columns, permuted as the ids were. */
+template <typename T>
+__global__ void gather_rows_kernel(const RowDesc *rows, uint32_t n, const T *src, const uint32_t *idx, T *dst)
+{
+    for (uint32_t k = blockIdx.x; k < n; k += gridDim.x)
+    {
+        const RowDesc d = rows[k];
+        for (uint32_t i = threadIdx.x; i < d.deg; i += blockDim.x)
+            dst[d.e0 + i] = src[idx[d.e0 + i]];
     }
 }
 
@@ -81,13 +266,6 @@ __global__ void iota_u32_kernel(uint32_t *x, uint64_t n)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         x[i] = (uint32_t)i;
-}
-
-template <typename T>
-__global__ void gather_kernel(const T *src, const uint32_t *idx, T *dst, uint64_t n)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        dst[i] = src[idx[i]];
 }
 
 /* ---- R-MAT -------------------------------------------------------------- */
@@ -192,20 +370,19 @@ const uint32_t *vertex_order(kk_engine *e)
     if (e->order_valid)
         return (const uint32_t *)e->order.p;
     const uint32_t V = e->V;
-    uint32_t *deg = nullptr, *deg_sorted = nullptr, *ids = nullptr, *bounds = nullptr;
-    KK_CUDA_CHECK(cudaMalloc(&deg, (size_t)V * 4 + 4));
-    KK_CUDA_CHECK(cudaMalloc(&deg_sorted, (size_t)V * 4 + 4));
-    KK_CUDA_CHECK(cudaMalloc(&ids, (size_t)V * 4 + 4));
-    KK_CUDA_CHECK(cudaMalloc(&bounds, kTierBounds * sizeof(uint32_t)));
+    /* degrees of 65535 and more are one key: the classes end far below, and
+     * two radix passes fewer */
+    uint32_t *deg = e->order_tmp.as<uint32_t>(3 * (uint64_t)V), *deg_sorted = deg + V, *ids = deg_sorted + V;
+    uint32_t *bounds = e->alias_next.as<uint32_t>(16); /* free between builds */
     uint32_t *order = e->order.as<uint32_t>(V);
     degree_keys_kernel<<<grid_for(e, V, 256), 256, 0, e->stream>>>(e->view(), deg, ids);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
     size_t bytes = 0;
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairsDescending(nullptr, bytes, deg, deg_sorted, ids, order, (int64_t)V, 0,
-                                                            32, e->stream));
+                                                            16, e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairsDescending(e->cub_tmp.ensure(bytes), bytes, deg, deg_sorted, ids,
-                                                            order, (int64_t)V, 0, 32, e->stream));
+                                                            order, (int64_t)V, 0, 16, e->stream));
     KK_CUDA_CHECK(cudaMemsetAsync(bounds, 0, kTierBounds * sizeof(uint32_t), e->stream));
     TierThresholds thr;
     for (uint32_t k = 0; k < kAliasClasses; k++)
@@ -214,12 +391,11 @@ const uint32_t *vertex_order(kk_engine *e)
     tier_bounds_kernel<<<grid_for(e, V, 256), 256, 0, e->stream>>>(deg_sorted, V, thr, bounds);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    KK_CUDA_CHECK(cudaMemcpyAsync(e->tier, bounds, kTierBounds * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
+    words_to_host(e, bounds, 48, kTierBounds);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    cudaFree(deg);
-    cudaFree(deg_sorted);
-    cudaFree(ids);
-    cudaFree(bounds);
+    memcpy(e->tier, (const char *)e->h_status + 48 * 4, kTierBounds * sizeof(uint32_t));
+    if (e->order_tmp.bytes > kKeepBytes)
+        e->order_tmp.release();
     e->n_hub = e->tier[0];
     e->n_nz = e->tier[kAliasClasses];
     RowDesc *rows = e->rows.as<RowDesc>(V > 0 ? V : 1);
@@ -247,6 +423,8 @@ const uint64_t *vertex_cursors(kk_engine *e)
 
 bool graph_no_dead_ends(kk_engine *e)
 {
+    if (!e->dead_ends_valid && e->order_valid && e->n_nz == e->V)
+        e->no_dead_ends = e->dead_ends_valid = true; /* every vertex has out-edges */
     if (!e->dead_ends_valid)
     {
         int *flag = (int *)e->small.ensure(64) + 12; /* a word the walks' status does not use */
@@ -345,20 +523,66 @@ const uint8_t *metapath_vertex_masks(kk_engine *e)
 
 void graph_check_sorted(kk_engine *e)
 {
-    int *flag = (int *)e->small.ensure(64);
-    KK_CUDA_CHECK(cudaMemsetAsync(flag, 0, sizeof(int), e->stream));
-    check_sorted_kernel<<<grid_for(e, e->V, 256), 256, 0, e->stream>>>(e->d_off, e->d_nbr, e->V, flag);
-    count_launch(e);
-    KK_CUDA_CHECK(cudaGetLastError());
-    int h = 0;
-    KK_CUDA_CHECK(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    uint64_t words[kScanWords];
+    scan_graph(e, e->V, e->E, e->d_off, e->d_nbr, nullptr, words);
+    e->sorted = words[kScanDescents] == words[kScanBetween];
+}
+
+/* Room for a graph in gnext's arrays.  When the device is full, the graph the
+ * engine holds goes first (drop: the caller has checked the new one, which
+ * will replace it). */
+static void next_arrays(kk_engine *e, uint32_t V, uint64_t E, bool off, bool w, bool type, bool drop)
+{
+    auto make = [&]() {
+        if (off)
+            e->gnext.off.as<int64_t>((uint64_t)V + 1);
+        e->gnext.nbr.as<uint32_t>(E + 1);
+        if (w)
+            e->gnext.w.as<float>(E + 1);
+        if (type)
+            e->gnext.type.as<uint8_t>(E + 4);
+    };
+    try
+    {
+        make();
+    }
+    catch (const Error &x)
+    {
+        if (x.status != KK_ERR_OOM || !drop)
+            throw;
+        cudaGetLastError();
+        e->gnext.release();
+        e->free_graph();
+        KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
+        e->gb.release();
+        make();
+    }
+}
+
+void graph_commit(kk_engine *e, uint32_t V, uint64_t E, bool w, bool type, int sorted)
+{
+    e->free_graph();
+    std::swap(e->gb, e->gnext);
+    e->d_off = (int64_t *)e->gb.off.p;
+    e->d_nbr = (uint32_t *)e->gb.nbr.p;
+    e->d_w = w ? (float *)e->gb.w.p : nullptr;
+    e->d_type = type ? (uint8_t *)e->gb.type.p : nullptr;
+    e->V = V;
+    e->E = E;
+    graph_offsets32(e);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    e->sorted = h ? 0 : 1;
+    if (e->gnext.bytes() > kKeepBytes)
+        e->gnext.release();
+    e->has_graph = true;
+    e->sorted = sorted;
 }
 
 /* Sorts every adjacency by neighbour, carrying weights and types (what
  * node2vec() does with std::sort, src/apps/node2vec.hpp:122-125).  Stable, so
- * with duplicate neighbours the file order of the duplicates is kept. */
+ * with duplicate neighbours the file order of the duplicates is kept.  The
+ * rows of up to kRankMax edges by rank, of up to kBitonicMax in shared memory,
+ * the others by CUB's segmented sort (all of them by it, 1 M rows of 24 M
+ * edges: 1.14 ms and two passes for the weights against 0.34 ms). */
 void graph_sort_adjacency(kk_engine *e)
 {
     require_graph(e);
@@ -369,81 +593,98 @@ void graph_sort_adjacency(kk_engine *e)
     e->alias_cached = -1;      /* the tables follow the adjacency order */
     e->edge_set_valid = false; /* and so do the edge set's indices */
     e->adjc_valid = false;     /* and the cursor adjacency */
-    uint64_t E = e->E;
-    uint32_t *nbr_out = nullptr, *idx_in = nullptr, *idx_out = nullptr;
-    KK_CUDA_CHECK(cudaMalloc(&nbr_out, E * 4 + 4));
-    KK_CUDA_CHECK(cudaMalloc(&idx_in, E * 4 + 4));
-    KK_CUDA_CHECK(cudaMalloc(&idx_out, E * 4 + 4));
-    iota_u32_kernel<<<grid_for(e, E, 256), 256, 0, e->stream>>>(idx_in, E);
-    count_launch(e);
-    size_t bytes = 0;
-    KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortPairs(nullptr, bytes, e->d_nbr, nbr_out, idx_in, idx_out,
-                                                            (int64_t)E, (int64_t)e->V, e->d_off, e->d_off + 1,
-                                                            e->stream));
-    void *tmp = e->cub_tmp.ensure(bytes);
-    KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortPairs(tmp, bytes, e->d_nbr, nbr_out, idx_in, idx_out, (int64_t)E,
-                                                            (int64_t)e->V, e->d_off, e->d_off + 1, e->stream));
+    const uint64_t E = e->E;
+    vertex_order(e);
+    const RowDesc *rows = (const RowDesc *)e->rows.p;
+    const uint32_t *t = e->tier;
+    next_arrays(e, e->V, E, false, e->d_w != nullptr, e->d_type != nullptr, false);
+    uint32_t *nbr_out = (uint32_t *)e->gnext.nbr.p;
+    float *w_out = (float *)e->gnext.w.p;
+    uint8_t *type_out = (uint8_t *)e->gnext.type.p;
+    if (t[6] > t[5])
+    {
+        rank_rows_kernel<32, kRankMax><<<grid_for(e, (uint64_t)(t[6] - t[5]) * 32, 128), 128, 0, e->stream>>>(
+            rows, t[5], t[6], e->d_nbr, e->d_w, e->d_type, nbr_out, w_out, type_out);
+        count_launch(e);
+    }
+    if (e->n_nz > t[6])
+    {
+        rank_rows_kernel<8, 32><<<grid_for(e, (uint64_t)(e->n_nz - t[6]) * 8, 128), 128, 0, e->stream>>>(
+            rows, t[6], e->n_nz, e->d_nbr, e->d_w, e->d_type, nbr_out, w_out, type_out);
+        count_launch(e);
+    }
+    if (t[5] > t[2])
+    {
+        const unsigned cap = 16u * (unsigned)e->sm_count;
+        bitonic_rows_kernel<<<t[5] - t[2] < cap ? t[5] - t[2] : cap, 256, 0, e->stream>>>(
+            rows, t[2], t[5], e->d_nbr, e->d_w, e->d_type, nbr_out, w_out, type_out);
+        count_launch(e);
+    }
+    KK_CUDA_CHECK(cudaGetLastError());
+    if (t[2] > 0)
+    {
+        const int64_t n = (int64_t)t[2];
+        const auto begin = thrust::make_transform_iterator(rows, RowBegin{});
+        const auto end = thrust::make_transform_iterator(rows, RowEnd{});
+        auto sort = [&](auto in, auto out) {
+            size_t bytes = 0;
+            KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortPairs(nullptr, bytes, e->d_nbr, nbr_out, in, out,
+                                                                    (int64_t)E, n, begin, end, e->stream));
+            KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortPairs(e->cub_tmp.ensure(bytes), bytes, e->d_nbr, nbr_out,
+                                                                    in, out, (int64_t)E, n, begin, end, e->stream));
+        };
+        const unsigned grid = t[2] < 8u * (unsigned)e->sm_count ? t[2] : 8u * (unsigned)e->sm_count;
+        if (e->d_w && !e->d_type)
+        {
+            sort((const float *)e->d_w, w_out);
+        }
+        else if (!e->d_w && e->d_type)
+        {
+            sort((const uint8_t *)e->d_type, type_out);
+        }
+        else if (!e->d_w)
+        {
+            size_t bytes = 0;
+            KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortKeys(nullptr, bytes, e->d_nbr, nbr_out, (int64_t)E, n,
+                                                                   begin, end, e->stream));
+            KK_CUDA_CHECK(cub::DeviceSegmentedSort::StableSortKeys(e->cub_tmp.ensure(bytes), bytes, e->d_nbr, nbr_out,
+                                                                   (int64_t)E, n, begin, end, e->stream));
+        }
+        else
+        {
+            uint32_t *idx = e->scratch.as<uint32_t>(2 * E + 2), *idx_out = idx + E + 1;
+            iota_u32_kernel<<<grid_for(e, E, 256), 256, 0, e->stream>>>(idx, E);
+            count_launch(e);
+            sort((const uint32_t *)idx, idx_out);
+            gather_rows_kernel<float><<<grid, 256, 0, e->stream>>>(rows, t[2], e->d_w, idx_out, w_out);
+            count_launch(e);
+            gather_rows_kernel<uint8_t><<<grid, 256, 0, e->stream>>>(rows, t[2], e->d_type, idx_out, type_out);
+            count_launch(e);
+            KK_CUDA_CHECK(cudaGetLastError());
+        }
+    }
+    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
+    std::swap(e->gb.nbr, e->gnext.nbr);
+    e->d_nbr = (uint32_t *)e->gb.nbr.p;
     if (e->d_w)
     {
-        float *w2 = nullptr;
-        KK_CUDA_CHECK(cudaMalloc(&w2, E * 4 + 4));
-        gather_kernel<float><<<grid_for(e, E, 256), 256, 0, e->stream>>>(e->d_w, idx_out, w2, E);
-        count_launch(e);
-        KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-        cudaFree(e->d_w);
-        e->d_w = w2;
+        std::swap(e->gb.w, e->gnext.w);
+        e->d_w = (float *)e->gb.w.p;
     }
     if (e->d_type)
     {
-        uint8_t *t2 = nullptr;
-        KK_CUDA_CHECK(cudaMalloc(&t2, E + 4));
-        gather_kernel<uint8_t><<<grid_for(e, E, 256), 256, 0, e->stream>>>(e->d_type, idx_out, t2, E);
-        count_launch(e);
-        KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-        cudaFree(e->d_type);
-        e->d_type = t2;
+        std::swap(e->gb.type, e->gnext.type);
+        e->d_type = (uint8_t *)e->gb.type.p;
     }
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    cudaFree(e->d_nbr);
-    e->d_nbr = nbr_out;
-    cudaFree(idx_in);
-    cudaFree(idx_out);
+    if (e->gnext.bytes() > kKeepBytes)
+        e->gnext.release();
     e->sorted = 1;
 }
 
-void graph_upload(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const float *w,
-                  const uint8_t *type)
+/* The checks of a host CSR on the host, one array after another: where the
+ * device has no room for it beside the graph it holds. */
+static void check_arrays(uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const uint8_t *type)
 {
-    e->free_graph();
-    KK_CUDA_CHECK(cudaMalloc(&e->d_off, (V + 1) * sizeof(int64_t)));
-    KK_CUDA_CHECK(cudaMalloc(&e->d_nbr, E * 4 + 4));
-    KK_CUDA_CHECK(cudaMemcpyAsync(e->d_off, off, (V + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, e->stream));
-    KK_CUDA_CHECK(cudaMemcpyAsync(e->d_nbr, nbr, E * 4, cudaMemcpyHostToDevice, e->stream));
-    if (w)
-    {
-        KK_CUDA_CHECK(cudaMalloc(&e->d_w, E * 4 + 4));
-        KK_CUDA_CHECK(cudaMemcpyAsync(e->d_w, w, E * 4, cudaMemcpyHostToDevice, e->stream));
-    }
-    if (type)
-    {
-        KK_CUDA_CHECK(cudaMalloc(&e->d_type, E + 4));
-        KK_CUDA_CHECK(cudaMemcpyAsync(e->d_type, type, E, cudaMemcpyHostToDevice, e->stream));
-    }
-    e->V = V;
-    e->E = E;
-    graph_offsets32(e);
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    e->has_graph = true;
-    e->sorted = -1;
-}
-
-void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const float *w,
-                       const uint8_t *type)
-{
-    if (V == 0 || off == nullptr || (E > 0 && nbr == nullptr))
-        fail(KK_ERR_INVALID_CONFIG, "graph needs V > 0, off and nbr");
-    if (off[0] != 0 || (uint64_t)off[V] != E)
-        fail(KK_ERR_INVALID_CONFIG, "off[0] must be 0 and off[V] must be E");
     for (uint32_t v = 0; v < V; v++)
         if (off[v + 1] < off[v])
             fail(KK_ERR_INVALID_CONFIG, "offsets must be non-decreasing");
@@ -454,18 +695,57 @@ void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off,
         for (uint64_t i = 0; i < E; i++)
             if (type[i] >= 8)
                 fail(KK_ERR_INVALID_CONFIG, "edge types must be < 8 (8-bit type masks)");
-    graph_upload(e, V, E, off, nbr, w, type);
+}
+
+/* A host CSR goes to the device as it is and is checked there, where a pass
+ * over it costs microseconds (24 M edges: 9 ms on one host thread), beside
+ * the graph the engine holds, which a refused one leaves in place. */
+void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off, const uint32_t *nbr, const float *w,
+                       const uint8_t *type)
+{
+    if (V == 0 || off == nullptr || (E > 0 && nbr == nullptr))
+        fail(KK_ERR_INVALID_CONFIG, "graph needs V > 0, off and nbr");
+    if (off[0] != 0 || (uint64_t)off[V] != E)
+        fail(KK_ERR_INVALID_CONFIG, "off[0] must be 0 and off[V] must be E");
+    bool checked = false;
+    try
+    {
+        next_arrays(e, V, E, true, w != nullptr, type != nullptr, false);
+    }
+    catch (const Error &x)
+    {
+        if (x.status != KK_ERR_OOM)
+            throw;
+        cudaGetLastError();
+        check_arrays(V, E, off, nbr, type);
+        checked = true;
+        next_arrays(e, V, E, true, w != nullptr, type != nullptr, true);
+    }
+    GraphBufs &n = e->gnext;
+    KK_CUDA_CHECK(cudaMemcpyAsync(n.off.p, off, ((size_t)V + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, e->stream));
+    KK_CUDA_CHECK(cudaMemcpyAsync(n.nbr.p, nbr, E * 4, cudaMemcpyHostToDevice, e->stream));
+    if (w)
+        KK_CUDA_CHECK(cudaMemcpyAsync(n.w.p, w, E * 4, cudaMemcpyHostToDevice, e->stream));
+    if (type)
+        KK_CUDA_CHECK(cudaMemcpyAsync(n.type.p, type, E, cudaMemcpyHostToDevice, e->stream));
+    uint64_t words[kScanWords];
+    scan_graph(e, V, E, (const int64_t *)n.off.p, (const uint32_t *)n.nbr.p, type ? (const uint8_t *)n.type.p : nullptr,
+               words);
+    if (!checked)
+    {
+        if (words[kScanBad] & kBadOffsets)
+            fail(KK_ERR_INVALID_CONFIG, "offsets must be non-decreasing");
+        if (words[kScanBad] & kBadNeighbour)
+            fail(KK_ERR_INVALID_CONFIG, "neighbour id out of range");
+        if (words[kScanBad] & kBadType)
+            fail(KK_ERR_INVALID_CONFIG, "edge types must be < 8 (8-bit type masks)");
+    }
+    graph_commit(e, V, E, w != nullptr, type != nullptr, words[kScanDescents] == words[kScanBetween]);
 }
 
 /* include/storage.hpp:35-55 + include/graph.hpp:408-530 on one rank. */
 namespace
 {
-
-__global__ void count_sources_kernel(const uint32_t *src, uint64_t m, unsigned long long *cnt)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
-        atomicAdd(cnt + src[i], 1ull);
-}
 
 template <typename T>
 __global__ void permute_kernel(const T *in, const uint32_t *perm, T *out, uint64_t m)
@@ -526,6 +806,16 @@ __global__ void unpack_values_kernel(const uint64_t *val, uint64_t m, uint32_t *
 
 } // namespace
 
+/* After a load: an unweighted graph's walks use neither of the buffers the
+ * load's temporaries stood in; large ones are given back. */
+static void load_temps_done(kk_engine *e, bool weighted)
+{
+    if (weighted || e->alias.bytes + e->scratch.bytes <= kKeepBytes)
+        return;
+    e->alias.release();
+    e->scratch.release();
+}
+
 /* CSR in HBM from the raw records of an untyped binary edge file (8-byte
  * src/dst or 12-byte src/dst/weight, include/storage.hpp:35-55), which
  * fill(d) puts into device memory at d as they are; they are split (and mirrored,
@@ -540,19 +830,13 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
     if (m >= 0xffffffffull)
         fail(KK_ERR_INVALID_CONFIG, "edge lists are limited to 2^32 - 1 edges");
     const bool weighted = rec == 12;
-    struct Temps
-    {
-        DevBuf raw, key, key2, val, val2;
-        ~Temps()
-        {
-            DevBuf *b[] = {&raw, &key, &key2, &val, &val2};
-            for (DevBuf *x : b)
-                x->release();
-        }
-    } tmp;
-    uint32_t *d_raw = tmp.raw.as<uint32_t>(n * (rec / 4) + 1);
-    uint32_t *d_key = tmp.key.as<uint32_t>(m + 1), *d_key2 = tmp.key2.as<uint32_t>(m + 1);
-    uint64_t *d_val = tmp.val.as<uint64_t>(m + 1), *d_val2 = tmp.val2.as<uint64_t>(m + 1);
+    /* the records and the sort's keys and values stand where the walks' alias
+     * tables and queues will: both are rebuilt for the new graph */
+    e->alias_cached = -1;
+    const uint64_t m1 = (m + 64) & ~(uint64_t)63; /* every array aligned */
+    uint64_t *d_val = e->scratch.as<uint64_t>(2 * m1), *d_val2 = d_val + m1;
+    uint32_t *d_key = e->alias.as<uint32_t>(2 * m1 + n * (rec / 4) + 1), *d_key2 = d_key + m1;
+    uint32_t *d_raw = d_key2 + m1;
     uint32_t *bad = (uint32_t *)e->small.ensure(64) + 13; /* a word the walks' status does not use */
     /* the records in HBM, as read (fill returns once they have arrived) */
     fill((unsigned char *)d_raw);
@@ -567,8 +851,7 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     if (((volatile uint32_t *)e->h_status)[41] != 0)
         fail(KK_ERR_INVALID_CONFIG, "edge endpoint >= v_num"); /* the engine keeps its graph */
-    tmp.raw.release();
-    e->free_graph();
+    next_arrays(e, V, m, true, weighted, false, true);
     int bits = 1;
     while (bits < 32 && ((uint64_t)1 << bits) < V)
         bits++;
@@ -577,23 +860,16 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
                                                   e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(e->cub_tmp.ensure(bytes), bytes, d_key, d_key2, d_val, d_val2,
                                                   (int64_t)m, 0, bits, e->stream));
-    KK_CUDA_CHECK(cudaMalloc(&e->d_off, ((uint64_t)V + 1) * sizeof(int64_t)));
-    offsets_from_sorted_kernel<<<grid_for(e, m + 1, 256), 256, 0, e->stream>>>(d_key2, m, V, e->d_off);
+    offsets_from_sorted_kernel<<<grid_for(e, m + 1, 256), 256, 0, e->stream>>>(d_key2, m, V,
+                                                                               (int64_t *)e->gnext.off.p);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    KK_CUDA_CHECK(cudaMalloc(&e->d_nbr, m * 4 + 4));
-    if (weighted)
-        KK_CUDA_CHECK(cudaMalloc(&e->d_w, m * 4 + 4));
-    unpack_values_kernel<<<grid_for(e, m ? m : 1, 256), 256, 0, e->stream>>>(d_val2, m, e->d_nbr,
-                                                                             weighted ? e->d_w : nullptr);
+    unpack_values_kernel<<<grid_for(e, m ? m : 1, 256), 256, 0, e->stream>>>(
+        d_val2, m, (uint32_t *)e->gnext.nbr.p, weighted ? (float *)e->gnext.w.p : nullptr);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    e->V = V;
-    e->E = m;
-    graph_offsets32(e);
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    e->has_graph = true;
-    e->sorted = -1;
+    graph_commit(e, V, m, weighted, false, -1);
+    load_temps_done(e, weighted);
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
@@ -606,19 +882,12 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
     if (m >= 0xffffffffull)
         fail(KK_ERR_INVALID_CONFIG, "edge lists are limited to 2^32 - 1 edges");
     const auto t0 = std::chrono::steady_clock::now();
-    e->free_graph();
-    struct Temps
-    {
-        DevBuf src, src2, idx, perm, cnt, in;
-        ~Temps()
-        {
-            DevBuf *b[] = {&src, &src2, &idx, &perm, &cnt, &in};
-            for (DevBuf *x : b)
-                x->release();
-        }
-    } tmp;
-    uint32_t *d_src = tmp.src.as<uint32_t>(m), *d_src2 = tmp.src2.as<uint32_t>(m);
-    uint32_t *d_idx = tmp.idx.as<uint32_t>(m), *d_perm = tmp.perm.as<uint32_t>(m);
+    e->alias_cached = -1; /* the sort's arrays stand in the tables' memory */
+    const uint64_t m1 = (m + 64) & ~(uint64_t)63; /* every array aligned */
+    uint32_t *d_src = e->alias.as<uint32_t>(4 * m1), *d_src2 = d_src + m1, *d_idx = d_src2 + m1, *d_perm = d_idx + m1;
+    uint32_t *d_in = e->scratch.as<uint32_t>(m1);
+    next_arrays(e, V, m, true, h_w != nullptr, h_t != nullptr, true);
+    GraphBufs &nx = e->gnext;
     KK_CUDA_CHECK(cudaMemcpyAsync(d_src, h_src, m * 4, cudaMemcpyHostToDevice, e->stream));
     iota_u32_kernel<<<grid_for(e, m, 256), 256, 0, e->stream>>>(d_idx, m);
     count_launch(e);
@@ -631,44 +900,32 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
                                                   e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(e->cub_tmp.ensure(bytes), bytes, d_src, d_src2, d_idx, d_perm,
                                                   (int64_t)m, 0, bits, e->stream));
-    /* offsets */
-    unsigned long long *cnt = tmp.cnt.as<unsigned long long>((uint64_t)V + 1);
-    KK_CUDA_CHECK(cudaMemsetAsync(cnt, 0, ((uint64_t)V + 1) * 8, e->stream));
-    count_sources_kernel<<<grid_for(e, m, 256), 256, 0, e->stream>>>(d_src, m, cnt);
+    offsets_from_sorted_kernel<<<grid_for(e, m + 1, 256), 256, 0, e->stream>>>(d_src2, m, V, (int64_t *)nx.off.p);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    KK_CUDA_CHECK(cudaMalloc(&e->d_off, ((uint64_t)V + 1) * sizeof(int64_t)));
-    exclusive_scan_u64(e, (const uint64_t *)cnt, (uint64_t *)e->d_off, (uint64_t)V + 1);
     /* neighbours, weights, types in sorted order */
-    KK_CUDA_CHECK(cudaMalloc(&e->d_nbr, m * 4 + 4));
-    uint32_t *d_in = tmp.in.as<uint32_t>(m);
     KK_CUDA_CHECK(cudaMemcpyAsync(d_in, h_dst, m * 4, cudaMemcpyHostToDevice, e->stream));
-    permute_kernel<uint32_t><<<grid_for(e, m, 256), 256, 0, e->stream>>>(d_in, d_perm, e->d_nbr, m);
+    permute_kernel<uint32_t><<<grid_for(e, m, 256), 256, 0, e->stream>>>(d_in, d_perm, (uint32_t *)nx.nbr.p, m);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
     if (h_w)
     {
-        KK_CUDA_CHECK(cudaMalloc(&e->d_w, m * 4 + 4));
         KK_CUDA_CHECK(cudaMemcpyAsync(d_in, h_w, m * 4, cudaMemcpyHostToDevice, e->stream));
-        permute_kernel<float><<<grid_for(e, m, 256), 256, 0, e->stream>>>((const float *)d_in, d_perm, e->d_w, m);
+        permute_kernel<float><<<grid_for(e, m, 256), 256, 0, e->stream>>>((const float *)d_in, d_perm, (float *)nx.w.p,
+                                                                          m);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
     if (h_t)
     {
-        KK_CUDA_CHECK(cudaMalloc(&e->d_type, m + 4));
         KK_CUDA_CHECK(cudaMemcpyAsync(d_in, h_t, m, cudaMemcpyHostToDevice, e->stream));
-        permute_kernel<uint8_t><<<grid_for(e, m, 256), 256, 0, e->stream>>>((const uint8_t *)d_in, d_perm, e->d_type,
-                                                                            m);
+        permute_kernel<uint8_t><<<grid_for(e, m, 256), 256, 0, e->stream>>>((const uint8_t *)d_in, d_perm,
+                                                                            (uint8_t *)nx.type.p, m);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
-    e->V = V;
-    e->E = m;
-    graph_offsets32(e);
-    KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    e->has_graph = true;
-    e->sorted = -1;
+    graph_commit(e, V, m, h_w != nullptr, h_t != nullptr, -1);
+    load_temps_done(e, h_w != nullptr);
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
@@ -1059,6 +1316,8 @@ void graph_generate_rmat(kk_engine *e, uint32_t scale, uint32_t ef, double a, do
     if (types < 0 || types > 8 || weights < 0 || weights > 2)
         fail(KK_ERR_INVALID_CONFIG, "R-MAT weights in {0,1,2}, types in [0, 8]");
     e->free_graph();
+    if (e->gb.bytes() > kKeepBytes)
+        e->gb.release();
     uint32_t V = 1u << scale;
     uint64_t m = (uint64_t)ef << scale;
     RmatThresholds t;
@@ -1102,34 +1361,27 @@ void graph_generate_rmat(kk_engine *e, uint32_t scale, uint32_t ef, double a, do
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, bytes, mir, mir_sorted, E, 0, 64, e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(e->cub_tmp.ensure(bytes), bytes, mir, mir_sorted, E, 0, 64, e->stream));
     cudaFree(mir);
-    KK_CUDA_CHECK(cudaMalloc(&e->d_nbr, E * 4 + 4));
-    if (weights)
-        KK_CUDA_CHECK(cudaMalloc(&e->d_w, E * 4 + 4));
-    if (types)
-        KK_CUDA_CHECK(cudaMalloc(&e->d_type, E + 4));
+    next_arrays(e, V, E, true, weights != 0, types != 0, true);
+    GraphBufs &nx = e->gnext;
     unsigned int *deg = nullptr;
     uint64_t *deg64 = nullptr;
     KK_CUDA_CHECK(cudaMalloc(&deg, (size_t)V * 4 + 4));
     KK_CUDA_CHECK(cudaMalloc(&deg64, ((size_t)V + 1) * 8));
     KK_CUDA_CHECK(cudaMemsetAsync(deg, 0, (size_t)V * 4, e->stream));
-    rmat_csr_kernel<<<grid_for(e, E, 256), 256, 0, e->stream>>>(mir_sorted, E, e->d_nbr, deg, seed + 1000, e->d_w,
-                                                                weights, e->d_type, (uint32_t)types);
+    rmat_csr_kernel<<<grid_for(e, E, 256), 256, 0, e->stream>>>(
+        mir_sorted, E, (uint32_t *)nx.nbr.p, deg, seed + 1000, weights ? (float *)nx.w.p : nullptr, weights,
+        types ? (uint8_t *)nx.type.p : nullptr, (uint32_t)types);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
     deg_to_u64_kernel<<<grid_for(e, (uint64_t)V + 1, 256), 256, 0, e->stream>>>(deg, deg64, V);
     count_launch(e);
-    KK_CUDA_CHECK(cudaMalloc(&e->d_off, ((size_t)V + 1) * 8));
-    exclusive_scan_u64(e, deg64, (uint64_t *)e->d_off, (uint64_t)V + 1);
-    e->V = V;
-    e->E = E;
-    graph_offsets32(e);
+    exclusive_scan_u64(e, deg64, (uint64_t *)nx.off.p, (uint64_t)V + 1);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     cudaFree(mir_sorted);
     cudaFree(deg);
     cudaFree(deg64);
     cudaFree(d_count);
-    e->has_graph = true;
-    e->sorted = 1;
+    graph_commit(e, V, E, weights != 0, types != 0, 1);
 }
 
 } // namespace kk
