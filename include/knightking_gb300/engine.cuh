@@ -416,14 +416,12 @@ struct kk_engine
     /* walkers per thread of the always-accepting first-order walks (option
      * walk_multi: 1, 2 or 4) */
     int walk_multi = 1;
-    /* walk_park (option): first-order walks with rejection trials park the
-     * walkers of a warp with fewer than this many lanes still walking and
-     * resume them in kParkRounds later launches (0: no parking; default 20:
-     * metapath S22 walk 19.3 -> 13.6 ms) */
+    /* walk_park (option): 0 gives every first-order rejection walk a thread of
+     * its own; else, beyond what the SMs hold, lanes take the walkers in turn
+     * (walk_turns_kernel) */
     int walk_park = 20;
-    kk::DevBuf park[2], park_count;
     /* regroup_interval (option): 0 off; k > 0 runs the walks of walk_static
-     * scheduling that do not park in phases of k steps, each phase's walkers
+     * scheduling that do not take turns in phases of k steps, each phase's walkers
      * sorted by the vertex they stand on (walk_regroup_kernel): records,
      * sort keys in and out, sort values, the sorted order, the counts */
     int regroup = 0;
@@ -486,9 +484,6 @@ inline void count_launch(kk_engine *e) { e->launches.fetch_add(1, std::memory_or
 /* n 32-bit words from src to the engine's mapped host words at word `at`,
  * written by a kernel on the engine's stream (no copy engine involved). */
 void words_to_host(kk_engine *e, const uint32_t *src, int at, int n);
-/* Resume launches after a parking walk; the last one parks nothing. */
-constexpr int kParkRounds = 6;
-
 /* The path offsets of segments 0..nseg (walker k << shift, the last one n)
  * into the mapped status block at kSegBoundAt, on the engine's stream. */
 void segment_bounds_to_host(kk_engine *e, const uint64_t *off, uint32_t n, uint32_t shift, uint32_t nseg);
@@ -1104,7 +1099,7 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
             goto launched;
         }
     }
-    if (e->walk_schedule == 0 && e->regroup > 0 && !(parks<TC>() && e->walk_park > 0) && n > 0)
+    if (e->walk_schedule == 0 && e->regroup > 0 && !(uneven_walks<TC>() && e->walk_park > 0) && n > 0)
     {
         walk_regrouped<S, WC, TC, Bucket>(e, g, wc, tc, alias, ra, L);
         goto launched;
@@ -1112,41 +1107,18 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
     if (e->walk_schedule == 0)
     {
         const unsigned bs = (unsigned)e->walk_block;
-        if constexpr (parks<TC>())
+        if constexpr (uneven_walks<TC>())
         {
-            if (e->walk_park > 0 && n > 0)
+            const unsigned b = bs < 128u ? bs : 128u; /* 8.54 ms against 8.59 at 256 (metapath R-MAT 22) */
+            int resident = 0;
+            KK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &resident, walk_turns_kernel<S, WC, TC, Bucket>, (int)b, 0));
+            const unsigned hold = (unsigned)e->sm_count * (resident > 0 ? resident : 1);
+            if (e->walk_park > 0 && grid_for(e, n, b) > hold)
             {
-                /* the first launch parks the stragglers of thinned-out warps
-                 * into queue 0; each resume round runs one queue 32 walkers
-                 * to a warp and parks into the other, the last round parks
-                 * nothing */
-                typedef ParkedWalker<S> PW;
-                PW *q[2] = {e->park[0].as<PW>(n), e->park[1].as<PW>(n)};
-                uint32_t *cnt = e->park_count.as<uint32_t>(2);
-                KK_CUDA_CHECK(cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), e->stream));
-                WalkLaunch Lp = L;
-                Lp.park = q[0];
-                Lp.park_count = cnt;
-                Lp.park_below = (uint32_t)e->walk_park;
-                walk_static_kernel<S, WC, TC, Bucket>
-                    <<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, Lp);
+                walk_turns_kernel<S, WC, TC, Bucket>
+                    <<<hold, b, 0, e->stream>>>(g, wc, tc, alias, ra, L, (uint32_t *)d_status + 14);
                 count_launch(e);
-                const unsigned rgrid = (unsigned)e->sm_count * (1024u / bs);
-                for (int r = 0; r < kParkRounds; r++)
-                {
-                    const int cur = r & 1, nxt = cur ^ 1;
-                    KK_CUDA_CHECK(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), e->stream));
-                    WalkLaunch Lr = L;
-                    if (r + 1 < kParkRounds)
-                    {
-                        Lr.park = q[nxt];
-                        Lr.park_count = cnt + nxt;
-                        Lr.park_below = (uint32_t)e->walk_park;
-                    }
-                    walk_resume_kernel<S, WC, TC, Bucket><<<rgrid, bs, 0, e->stream>>>(g, wc, tc, alias, ra, Lr,
-                                                                                      q[cur], cnt + cur);
-                    count_launch(e);
-                }
                 goto launched;
             }
         }

@@ -1944,19 +1944,7 @@ struct WalkLaunch
      * segment with its own status), reported in its flag as 1 + status;
      * nullptr: the flag is 1 */
     const int *seg_status = nullptr;
-    /* parking (first-order walks with rejection trials): once fewer than
-     * park_below of a warp's lanes are still walking, each of them stops at
-     * its next step boundary and is appended to park (a ParkedWalker<S>
-     * array, park_count entries), so that the warp ends and a later launch
-     * resumes the stragglers 32 to a warp.  park == nullptr: no parking. */
-    void *park = nullptr;
-    uint32_t *park_count = nullptr;
-    uint32_t park_below = 0;
 };
-
-/* Trials each lane runs on its own between a parking warp's ballots (metapath
- * S22: 1 -> 16.8 ms, 8 -> 13.6 ms, 16 -> 13.7 ms per walk). */
-constexpr uint32_t kParkCheck = 8;
 
 /* Walker i has written its whole path and its length.  The lanes that end a
  * walker of the same segment together are counted by one of them (a counter
@@ -2501,8 +2489,7 @@ __device__ __forceinline__ bool walk_trial(const GraphView &g, const WC &wc, con
         return rejection_trial<S>(g, wc, tc, alias, ra, L, run, rng);
 }
 
-/* A walker stopped at a step boundary between launches (first-order walks):
- * its position i in the launch, the vertex it stands on, its step, its path
+/* A walker stopped at a step boundary between launches: its position i in the launch, the vertex it stands on, its step, its path
  * length so far and its state.  The stream is keyed by (walker, step), so
  * a walk resumed from this record draws and writes what it would have. */
 template <typename S>
@@ -2515,11 +2502,10 @@ struct ParkedWalker
     S data;
 };
 
-/* Walks that park: first order with rejection trials (a step takes a
- * geometric number of trials and a walk may end at any step, so the lanes
- * of a warp finish far apart). */
+/* First order with rejection trials: a step takes a geometric number of trials
+ * and a walk may end at any step, so the lanes of a warp finish far apart. */
 template <typename TC>
-constexpr bool parks()
+constexpr bool uneven_walks()
 {
     return TC::order == 1 && TC::has_dynamic;
 }
@@ -2714,75 +2700,6 @@ __device__ __forceinline__ void resume_run(const WalkLaunch &L, uint32_t i, cons
     run.trials = run.queries = run.probes = 0;
 }
 
-/* Runs the warp's walkers (alive: lane holds walker i) to their ends, or,
- * with parking on, until fewer than L.park_below lanes are walking; then each
- * lane still walking finishes its step and parks (record under park_id),
- * once it has taken a step in this launch (so every launch moves every walker
- * it holds).  Every lane of the warp calls it with the same L.park and
- * L.park_below (the ballots take the full warp). */
-template <typename S, typename WC, typename TC, typename Bucket>
-__device__ __forceinline__ void walk_lanes(const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
-                                           const float *ra, const WalkLaunch &L, bool alive, uint32_t i,
-                                           WalkerRun<S> &run, Sampler &rng, unsigned long long &my_steps,
-                                           WalkCounts &counts, uint32_t park_id)
-{
-    /* between the warp's ballots each lane runs up to kParkCheck trials on
-     * its own, so lanes in different phases of a step overlap their reads (a
-     * ballot per trial forces the warp to reconverge every trial: 16.8 vs
-     * 13.6 ms); a lane that may park stops at its step boundary.  Without
-     * parking one pass runs every walk to its end. */
-    const uint32_t check = L.park != nullptr ? kParkCheck : 0xffffffffu;
-    bool parking = false;
-    const step_t step0 = alive ? run.w.step : 0;
-    for (;;)
-    {
-        const unsigned live = __ballot_sync(kFullMask, alive);
-        if (live == 0)
-            return;
-        if (L.park != nullptr)
-        {
-            if ((unsigned)__popc(live) < L.park_below)
-                parking = true;
-            const bool stop = alive && parking && !run.in_step && run.w.step != step0;
-            const unsigned stops = __ballot_sync(kFullMask, stop);
-            if (stops != 0)
-            {
-                const unsigned lane = threadIdx.x & 31;
-                uint32_t base = 0;
-                if (lane == (unsigned)(__ffs(stops) - 1))
-                    base = atomicAdd(L.park_count, (uint32_t)__popc(stops));
-                base = __shfl_sync(kFullMask, base, __ffs(stops) - 1);
-                if (stop)
-                {
-                    ParkedWalker<S> *q = (ParkedWalker<S> *)L.park;
-                    q[base + __popc(stops & ((1u << lane) - 1u))] = ParkedWalker<S>{park_id, run.v, run.w.step,
-                                                                                   run.len, run.w.data};
-                    counts.add(run);
-                    alive = false;
-                }
-            }
-        }
-        bool ended = false;
-        for (uint32_t k = 0; alive && k < check; k++)
-        {
-            if (parking && !run.in_step && run.w.step != step0)
-                break;
-            if (!walk_trial<S>(g, wc, tc, alias, ra, L, run, rng))
-            {
-                ended = true;
-                break;
-            }
-        }
-        /* outside the divergent loop: walk_finish's segment count synchronises
-         * lanes (inside it the walk took 25 instead of 19 ms) */
-        if (ended)
-        {
-            walk_finish<S>(L, i, run, my_steps, counts);
-            alive = false;
-        }
-    }
-}
-
 /* One thread per walker for its whole walk, walker state in registers. */
 template <typename S, typename WC, typename TC, typename Bucket>
 __global__ void __launch_bounds__(256, 4) walk_static_kernel(GraphView g, WC wc, TC tc, const Bucket *alias,
@@ -2795,20 +2712,7 @@ __global__ void __launch_bounds__(256, 4) walk_static_kernel(GraphView g, WC wc,
     for (uint32_t it = 0; it < n_iter; it++)
     {
         const uint32_t i = (it * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-        if constexpr (parks<TC>())
-        {
-            /* every lane takes part in walk_lanes' ballots */
-            const bool alive = i < L.walker_num;
-            Sampler rng;
-            WalkerRun<S> run;
-            if (alive)
-            {
-                rng.init(L.seed);
-                walk_begin<S>(g, wc, L, i, run, rng);
-            }
-            walk_lanes<S>(g, wc, tc, alias, ra, L, alive, i, run, rng, my_steps, counts, i);
-        }
-        else if (i < L.walker_num)
+        if (i < L.walker_num)
         {
             Sampler rng;
             rng.init(L.seed);
@@ -2898,32 +2802,67 @@ __global__ void __launch_bounds__(256, 4) walk_stream_kernel(GraphView g, WC wc,
     counts.flush(L.stats);
 }
 
-/* Resumes the walkers parked by the previous launch (*in_count of them),
- * 32 to a warp, parking again into L.park (or running them to their ends
- * when L.park is nullptr). */
+/* First-order rejection walks of more walkers than the SMs hold: a walk ends at
+ * any step, so lanes take the walkers in turn (*next + the launch's threads),
+ * kTurnIdle of a warp's lanes or more at a time: a refill reads the start, its
+ * offsets and the state's hooks, and costs the lanes that walk on as much as
+ * those it serves.  Between the warp's ballots a lane runs up to kTurnTrials
+ * trials of its own, so that lanes in different phases of a step overlap their
+ * reads; a ballot a trial makes the warp wait for each of them.  Metapath on
+ * R-MAT 22, 2.4 M walkers: 12.2 ms with the stragglers of thinned-out warps
+ * recorded and resumed 32 to a warp by later launches (20 of 32 warps of an SM
+ * resident, 13 to 16 of 32 lanes walking), 8.6 ms in turn; 4 to 16 trials and
+ * 4 or 8 lanes are within 1%, 16 lanes 3% slower. */
+constexpr uint32_t kTurnTrials = 8, kTurnIdle = 8;
+
 template <typename S, typename WC, typename TC, typename Bucket>
-__global__ void __launch_bounds__(256, 4) walk_resume_kernel(GraphView g, WC wc, TC tc, const Bucket *alias,
-                                                          const float *ra, WalkLaunch L,
-                                                          const ParkedWalker<S> *in, const uint32_t *in_count)
+__global__ void __launch_bounds__(256, 4) walk_turns_kernel(GraphView g, WC wc, TC tc, const Bucket *alias,
+                                                         const float *ra, WalkLaunch L, uint32_t *next)
 {
+    const uint32_t lane = threadIdx.x & 31, threads = gridDim.x * blockDim.x;
     unsigned long long my_steps = 0;
     WalkCounts counts;
-    const uint32_t n = *in_count;
-    for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x)
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    Sampler rng;
+    WalkerRun<S> run;
+    rng.init(L.seed);
+    bool alive = i < L.walker_num, more = threads < L.walker_num;
+    if (alive)
+        walk_begin<S>(g, wc, L, i, run, rng);
+    for (;;)
     {
-        const uint32_t k = b + threadIdx.x;
-        const bool alive = k < n;
-        uint32_t i = 0;
-        Sampler rng;
-        WalkerRun<S> run;
-        if (alive)
+        const unsigned idle = __ballot_sync(kFullMask, !alive);
+        if (more && (uint32_t)__popc(idle) >= kTurnIdle)
         {
-            const ParkedWalker<S> pw = in[k];
-            i = pw.i;
-            rng.init(L.seed);
-            resume_run<S>(L, i, pw, run);
+            uint32_t base = 0;
+            if (lane == (unsigned)(__ffs(idle) - 1))
+                base = atomicAdd(next, (uint32_t)__popc(idle));
+            base = threads + __shfl_sync(kFullMask, base, __ffs(idle) - 1);
+            more = base + (uint32_t)__popc(idle) < L.walker_num;
+            if (!alive)
+            {
+                i = base + __popc(idle & lanemask_lt());
+                alive = i < L.walker_num;
+                if (alive)
+                    walk_begin<S>(g, wc, L, i, run, rng);
+            }
         }
-        walk_lanes<S>(g, wc, tc, alias, ra, L, alive, i, run, rng, my_steps, counts, i);
+        else if (idle == kFullMask)
+        {
+            break;
+        }
+        bool ended = false;
+        for (uint32_t k = 0; alive && k < kTurnTrials; k++)
+            if (!walk_trial<S>(g, wc, tc, alias, ra, L, run, rng))
+            {
+                ended = true;
+                break;
+            }
+        if (ended)
+        {
+            walk_finish<S>(L, i, run, my_steps, counts);
+            alive = false;
+        }
     }
     flush_steps(L.total_steps, my_steps);
     counts.flush(L.stats);
@@ -3344,15 +3283,6 @@ __device__ __forceinline__ uint32_t batch_walker_begin(const GraphView &g, const
     return i;
 }
 
-/* Parking of a batch launch (first-order rejection walks): the queue the
- * stragglers go to and the lane threshold; out == nullptr: none. */
-struct BatchPark
-{
-    void *out = nullptr;
-    uint32_t *count = nullptr;
-    uint32_t below = 0;
-};
-
 /* One thread per walker over the concatenated walkers of all jobs.
  * App::make(job, wc, tc) builds the job's WalkerConfig / TransitionConfig. */
 template <typename S, typename App, typename Bucket>
@@ -3361,7 +3291,7 @@ __global__ void __launch_bounds__(256, KK_BATCH_MINB) walk_batch_kernel(GraphVie
                                                          const float *alias_sum, uint32_t *path, uint32_t *length,
                                                          unsigned long long *total_steps, int *status,
                                                          uint32_t trial_limit, unsigned long long *stats,
-                                                         const uint32_t *hdr, BatchPark bp, BatchNotify nt)
+                                                         const uint32_t *hdr, BatchNotify nt)
 {
     __shared__ uint32_t s_first[2 * kMaxBatchJobs];
     if (hdr != nullptr)
@@ -3383,27 +3313,7 @@ __global__ void __launch_bounds__(256, KK_BATCH_MINB) walk_batch_kernel(GraphVie
     for (uint32_t it = 0; it < n_iter; it++)
     {
         const uint32_t t = (it * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-        if constexpr (parks<typename App::TC>())
-        {
-            /* every lane takes part in walk_lanes' ballots, with the same
-             * parking fields */
-            typename App::WC wc;
-            typename App::TC tc;
-            WalkLaunch L;
-            L.park = bp.out;
-            L.park_count = bp.count;
-            L.park_below = bp.below;
-            WalkerRun<S> run;
-            Sampler rng;
-            const bool alive = t < total;
-            uint32_t i = 0;
-            if (alive)
-                i = batch_walker_begin<S>(g, app, jobs, s_first, njobs, t, alias_sum, path, length, total_steps,
-                                          status, trial_limit, wc, tc, L, run, rng, nt);
-            L.stats = stats;
-            walk_lanes<S>(g, wc, tc, alias, nullptr, L, alive, i, run, rng, my_steps, counts, t);
-        }
-        else if constexpr (straight<typename App::TC>())
+        if constexpr (straight<typename App::TC>())
         {
             __shared__ uint32_t s_tile[8 * kTileWords]; /* of up to 256 threads */
             typename App::WC wc;
@@ -3443,19 +3353,14 @@ __global__ void __launch_bounds__(256, KK_BATCH_MINB) walk_batch_kernel(GraphVie
     counts.flush(stats);
 }
 
-/* Resumes the batch walkers parked by the previous launch (*in_count of
- * them; a record holds the walker's position t in the batch), 32 to a warp,
- * parking again into bp (or running them to their ends when bp.out is
- * nullptr). */
+/* walk_turns_kernel over the concatenated walkers of all jobs. */
 template <typename S, typename App, typename Bucket>
-__global__ void __launch_bounds__(256, 4) walk_batch_resume_kernel(GraphView g, App app, const BatchJob *jobs,
-                                                                uint32_t njobs, const Bucket *alias,
-                                                                const float *alias_sum, uint32_t *path,
-                                                                uint32_t *length, unsigned long long *total_steps,
-                                                                int *status, uint32_t trial_limit,
-                                                                unsigned long long *stats,
-                                                                const ParkedWalker<S> *in, const uint32_t *in_count,
-                                                                BatchPark bp)
+__global__ void __launch_bounds__(256, 4) walk_batch_turns_kernel(GraphView g, App app, const BatchJob *jobs,
+                                                               uint32_t njobs, uint32_t total, const Bucket *alias,
+                                                               const float *alias_sum, uint32_t *path,
+                                                               uint32_t *length, unsigned long long *total_steps,
+                                                               int *status, uint32_t trial_limit,
+                                                               unsigned long long *stats, uint32_t *next)
 {
     __shared__ uint32_t s_first[2 * kMaxBatchJobs];
     for (uint32_t j = threadIdx.x; j < njobs; j += blockDim.x)
@@ -3464,33 +3369,57 @@ __global__ void __launch_bounds__(256, 4) walk_batch_resume_kernel(GraphView g, 
         s_first[kMaxBatchJobs + j] = jobs[j].launch_job;
     }
     __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, threads = gridDim.x * blockDim.x;
     unsigned long long my_steps = 0;
     WalkCounts counts;
-    const uint32_t n = *in_count;
-    for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x)
-    {
-        const uint32_t k = b + threadIdx.x;
-        typename App::WC wc;
-        typename App::TC tc;
-        WalkLaunch L;
-        L.park = bp.out;
-        L.park_count = bp.count;
-        L.park_below = bp.below;
-        WalkerRun<S> run;
-        Sampler rng;
-        const bool alive = k < n;
-        uint32_t i = 0, t = 0;
-        if (alive)
-        {
-            const ParkedWalker<S> pw = in[k];
-            t = pw.i;
-            i = batch_launch(app, jobs, s_first, njobs, t, alias_sum, path, length, total_steps, status, trial_limit,
-                             wc, tc, L, BatchNotify{});
-            rng.init(L.seed);
-            resume_run<S>(L, i, pw, run);
-        }
+    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = 0;
+    typename App::WC wc;
+    typename App::TC tc;
+    WalkLaunch L;
+    WalkerRun<S> run;
+    Sampler rng;
+    bool alive = t < total, more = threads < total;
+    auto begin = [&]() {
+        i = batch_walker_begin<S>(g, app, jobs, s_first, njobs, t, alias_sum, path, length, total_steps, status,
+                                  trial_limit, wc, tc, L, run, rng, BatchNotify{});
         L.stats = stats;
-        walk_lanes<S>(g, wc, tc, alias, nullptr, L, alive, i, run, rng, my_steps, counts, t);
+    };
+    if (alive)
+        begin();
+    for (;;)
+    {
+        const unsigned idle = __ballot_sync(kFullMask, !alive);
+        if (more && (uint32_t)__popc(idle) >= kTurnIdle)
+        {
+            uint32_t base = 0;
+            if (lane == (unsigned)(__ffs(idle) - 1))
+                base = atomicAdd(next, (uint32_t)__popc(idle));
+            base = threads + __shfl_sync(kFullMask, base, __ffs(idle) - 1);
+            more = base + (uint32_t)__popc(idle) < total;
+            if (!alive)
+            {
+                t = base + __popc(idle & lanemask_lt());
+                alive = t < total;
+                if (alive)
+                    begin();
+            }
+        }
+        else if (idle == kFullMask)
+        {
+            break;
+        }
+        bool ended = false;
+        for (uint32_t k = 0; alive && k < kTurnTrials; k++)
+            if (!walk_trial<S>(g, wc, tc, alias, nullptr, L, run, rng))
+            {
+                ended = true;
+                break;
+            }
+        if (ended)
+        {
+            walk_finish<S>(L, i, run, my_steps, counts);
+            alive = false;
+        }
     }
     flush_steps(total_steps, my_steps);
     counts.flush(stats);

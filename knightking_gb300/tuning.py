@@ -2,7 +2,7 @@
 
 The options (kk_engine_set_option) never change a path, only how fast it is
 produced: alias-table layout, the alias build's stream split, node2vec
-adjacency test, walk block size, the parking threshold of rejection walks,
+adjacency test, walk block size, whether rejection walks take turns,
 walkers per thread, the context's L2 fetch-granularity hint, the walk schedule,
 the cursor adjacency of uniform walks and the regroup interval (walkers sorted
 by the vertex they stand on every k steps).  The tuner runs a
@@ -19,7 +19,7 @@ DEFAULT_SPACE = (
     ("node2vec_adjacency", (0, 1)),
     ("walk_block", (256, 128, 64)),
     ("walk_multi", (1, 2, 4)),
-    ("walk_park", (20, 0, 12, 28)),
+    ("walk_park", (20, 0)),
     ("l2_fetch_bytes", (0, 64)),
     ("walk_schedule", (0, 1)),
     ("cursor_adjacency", (0, 1)),
