@@ -129,7 +129,9 @@ kk_status kk_engine_set_stream(kk_engine *e, void *stream);
  *   "into_stream"        1 (default): kk_walk_into walks whose path lengths are known before they
  *                        run (DeepWalk, PPR, node2vec on graphs without reachable dead ends) in one
  *                        launch per epoch and copies each segment of walkers out as soon as its
- *                        last walker finishes; 0: walker chunks for every walk (into_chunks)
+ *                        last walker finishes, and kk_walk does the same for such walks of one
+ *                        epoch and 16 MB of vertices or more; 0: walker chunks for every
+ *                        kk_walk_into (into_chunks), and kk_walk copies after the walk
  *   "into_chunks"        kk_walk_into walks that are not streamed (metapath excepted: one chunk) run in
  *                        up to this many walker chunks (>= 2^18 walkers each), copying each chunk's
  *                        paths out while the next chunk walks (default 6; 1 = whole)

@@ -352,6 +352,127 @@ uint64_t pack_paths_on(kk_engine *e, const WalkResult &r, cudaStream_t st, int s
     return total;
 }
 
+constexpr uint32_t kIntoMinChunk = 1u << 18;
+constexpr uint32_t kIntoMinRun = 4; /* streamed segments per copy while the walk runs */
+
+/* Whether kk_walk's paths leave while the walk runs: below 16 MB of vertices
+ * the segments' bookkeeping takes what the overlap saves (host wall of a call,
+ * after the walk / streamed: DeepWalk R-MAT 12, 1543 to 49382 walkers of 80
+ * steps, 126/138 to 231/235 us; node2vec R-MAT 18 at 16 MB 684/656, at 256 MB
+ * 3956/2653; DeepWalk R-MAT 22 at 16 MB 2573/2567, at 256 MB 5441/4245). */
+bool stream_pays(const kk_walk_opts *o)
+{
+    const double mean = o->app == KK_APP_PPR ? 1.0 / (o->terminate_prob > 0.0f ? (double)o->terminate_prob : 1.0)
+                                             : (double)o->walk_length + 1.0;
+    return (double)o->walker_num * mean * 4.0 >= 16.0e6;
+}
+
+/* The copy stream and its events, made on first use. */
+void make_copy_stream(kk_engine *e)
+{
+    if (e->copy_stream != nullptr)
+        return;
+    /* the highest priority: a chunk's packing kernels start as soon as its
+     * walk ends, not after the next chunk's walk blocks are all issued */
+    int lo = 0, hi = 0;
+    KK_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    KK_CUDA_CHECK(cudaStreamCreateWithPriority(&e->copy_stream, cudaStreamNonBlocking, hi));
+    for (int i = 0; i < 3; i++)
+    {
+        KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_walked[i], cudaEventDisableTiming));
+        KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_copied[i], cudaEventDisableTiming));
+    }
+    KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_seg_copy, cudaEventDisableTiming));
+}
+
+/* Where a streamed walk's paths go: its walkers' lengths and offsets, and the
+ * vertices, whose first is number base of the caller's. */
+struct StreamDest
+{
+    uint32_t *length = nullptr;
+    uint64_t *offset = nullptr;
+    uint32_t *vertices = nullptr;
+    uint64_t base = 0;
+};
+
+/* SegmentSink::before: the offsets are final (the engine's stream has been
+ * synchronised), and so are the lengths, which the walk fills exactly: both
+ * out at once, while the walk's first segments are still walking.  s: the
+ * output set whose buffers they pass through. */
+void stream_before(kk_engine *e, int s, const StreamDest &to, const uint64_t *d_off, uint32_t n)
+{
+    cudaStream_t cs = e->copy_stream;
+    uint64_t *ob = e->into_offb[s].as<uint64_t>((uint64_t)n + 1);
+    uint32_t *lb = e->into_lenb[s].as<uint32_t>((uint64_t)n + 1);
+    offsets_lengths_kernel<<<grid_for(e, n, 256), 256, 0, cs>>>(d_off, to.base, n, ob, lb);
+    count_launch(e);
+    KK_CUDA_CHECK(cudaGetLastError());
+    KK_CUDA_CHECK(cudaMemcpyAsync(to.offset, ob, (size_t)n * 8, cudaMemcpyDeviceToHost, cs));
+    KK_CUDA_CHECK(cudaMemcpyAsync(to.length, lb, (size_t)n * 4, cudaMemcpyDeviceToHost, cs));
+}
+
+/* SegmentSink::during: the segments' copies as they end, and whatever is left
+ * once the walk has. */
+void stream_during(kk_engine *e, const StreamDest &to, const uint32_t *d_path, uint32_t nseg,
+                   const volatile uint32_t *flag, const volatile uint64_t *bound, cudaEvent_t walked)
+{
+    cudaStream_t cs = e->copy_stream;
+    std::vector<char> out(nseg, 0);
+    uint32_t left = nseg;
+    bool all = false, issued_any = false;
+    while (left > 0)
+    {
+        if (!all)
+        {
+            /* once the walk has ended every segment is final,
+             * whether or not its flag has arrived */
+            const cudaError_t q = cudaEventQuery(walked);
+            if (q == cudaSuccess)
+                all = true;
+            else if (q != cudaErrorNotReady)
+                KK_CUDA_CHECK(q);
+        }
+        for (uint32_t a = 0; a < nseg;)
+        {
+            if (out[a] || !(all || flag[a]))
+            {
+                a++;
+                continue;
+            }
+            uint32_t b = a;
+            while (b < nseg && !out[b] && (all || flag[b]))
+                b++;
+            /* while the copy engine has work queued, finished
+             * segments wait to go out in runs of at least
+             * kIntoMinRun (it moves fewer, larger copies
+             * faster); an idle engine takes whatever is ready */
+            if (!all && b - a < kIntoMinRun && b < nseg && issued_any)
+            {
+                const cudaError_t q = cudaEventQuery(e->ev_seg_copy);
+                if (q == cudaErrorNotReady)
+                {
+                    a = b;
+                    continue;
+                }
+                if (q != cudaSuccess)
+                    KK_CUDA_CHECK(q);
+            }
+            for (uint32_t k = a; k < b; k++)
+                out[k] = 1;
+            const uint64_t va = bound[a], vb = bound[b];
+            if (vb > va)
+                KK_CUDA_CHECK(cudaMemcpyAsync(to.vertices + to.base + va, d_path + va,
+                                              (size_t)(vb - va) * 4, cudaMemcpyDeviceToHost, cs));
+            KK_CUDA_CHECK(cudaEventRecord(e->ev_seg_copy, cs));
+            issued_any = true;
+            left -= b - a;
+            a = b;
+        }
+        /* no yield: the thread keeps its core, so a finished
+         * segment waits microseconds, not a time slice */
+    }
+}
+
 /* kk_walk_into for the built-in apps: the walkers of each epoch in chunks
  * (the into_chunks option; about kIntoMinChunk walkers at least).  Chunks
  * rotate over three output sets: chunk c + 1 walks while chunk c's lengths,
@@ -360,28 +481,12 @@ uint64_t pack_paths_on(kk_engine *e, const WalkResult &r, cudaStream_t st, int s
  * alias tables are built once per call, by the first chunk (the same tables
  * every chunk would build), unless the alias_cache option keeps them across
  * calls anyway. */
-constexpr uint32_t kIntoMinChunk = 1u << 18;
-constexpr uint32_t kIntoMinRun = 4; /* streamed segments per copy while the walk runs */
-
 uint64_t walk_into_chunked(kk_engine *e, const kk_walk_opts *o, uint32_t *h_length, uint64_t *h_offset,
                            uint32_t *h_vertices, uint64_t capacity)
 {
     validate_opts(e, o, true);
     const uint32_t *d_start = upload_start(e, o);
-    if (e->copy_stream == nullptr)
-    {
-        /* the highest priority: a chunk's packing kernels start as soon as its
-         * walk ends, not after the next chunk's walk blocks are all issued */
-        int lo = 0, hi = 0;
-        KK_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-        KK_CUDA_CHECK(cudaStreamCreateWithPriority(&e->copy_stream, cudaStreamNonBlocking, hi));
-        for (int i = 0; i < 3; i++)
-        {
-            KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_walked[i], cudaEventDisableTiming));
-            KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_copied[i], cudaEventDisableTiming));
-        }
-        KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_seg_copy, cudaEventDisableTiming));
-    }
+    make_copy_stream(e);
     const int user_cache = e->alias_cache;
     struct Restore
     {
@@ -434,80 +539,18 @@ uint64_t walk_into_chunked(kk_engine *e, const kk_walk_opts *o, uint32_t *h_leng
             e->walk_set = s;
             cudaStream_t cs = e->copy_stream;
             SegmentSink sink;
+            StreamDest to;
             if (streamed)
             {
+                to = StreamDest{h_length + cb, h_offset + cb, h_vertices, base};
                 sink.before = [&](const uint64_t *d_off, uint32_t n, uint64_t total) {
                     if (base + total > capacity)
                         fail(KK_ERR_PATH_CAPACITY, "vertices buffer too small");
-                    /* the offsets are final (the engine's stream has been
-                     * synchronised), and so are the lengths, which the walk
-                     * fills exactly: both out at once, while the walk's first
-                     * segments are still walking */
-                    uint64_t *ob = e->into_offb[s].as<uint64_t>((uint64_t)n + 1);
-                    uint32_t *lb = e->into_lenb[s].as<uint32_t>((uint64_t)n + 1);
-                    offsets_lengths_kernel<<<grid_for(e, n, 256), 256, 0, cs>>>(d_off, base, n, ob, lb);
-                    count_launch(e);
-                    KK_CUDA_CHECK(cudaGetLastError());
-                    KK_CUDA_CHECK(cudaMemcpyAsync(h_offset + cb, ob, (size_t)n * 8, cudaMemcpyDeviceToHost, cs));
-                    KK_CUDA_CHECK(cudaMemcpyAsync(h_length + cb, lb, (size_t)n * 4, cudaMemcpyDeviceToHost, cs));
+                    stream_before(e, s, to, d_off, n);
                 };
-                sink.during = [&](const uint32_t *d_len, const uint32_t *d_path, uint32_t n, uint32_t shift,
-                                  uint32_t nseg, const volatile uint32_t *flag, const volatile uint64_t *bound,
-                                  cudaEvent_t walked) {
-                    std::vector<char> out(nseg, 0);
-                    uint32_t left = nseg;
-                    bool all = false, issued_any = false;
-                    while (left > 0)
-                    {
-                        if (!all)
-                        {
-                            /* once the walk has ended every segment is final,
-                             * whether or not its flag has arrived */
-                            const cudaError_t q = cudaEventQuery(walked);
-                            if (q == cudaSuccess)
-                                all = true;
-                            else if (q != cudaErrorNotReady)
-                                KK_CUDA_CHECK(q);
-                        }
-                        for (uint32_t a = 0; a < nseg;)
-                        {
-                            if (out[a] || !(all || flag[a]))
-                            {
-                                a++;
-                                continue;
-                            }
-                            uint32_t b = a;
-                            while (b < nseg && !out[b] && (all || flag[b]))
-                                b++;
-                            /* while the copy engine has work queued, finished
-                             * segments wait to go out in runs of at least
-                             * kIntoMinRun (it moves fewer, larger copies
-                             * faster); an idle engine takes whatever is ready */
-                            if (!all && b - a < kIntoMinRun && b < nseg && issued_any)
-                            {
-                                const cudaError_t q = cudaEventQuery(e->ev_seg_copy);
-                                if (q == cudaErrorNotReady)
-                                {
-                                    a = b;
-                                    continue;
-                                }
-                                if (q != cudaSuccess)
-                                    KK_CUDA_CHECK(q);
-                            }
-                            for (uint32_t k = a; k < b; k++)
-                                out[k] = 1;
-                            const uint64_t va = bound[a], vb = bound[b];
-                            if (vb > va)
-                                KK_CUDA_CHECK(cudaMemcpyAsync(h_vertices + base + va, d_path + va,
-                                                              (size_t)(vb - va) * 4, cudaMemcpyDeviceToHost, cs));
-                            KK_CUDA_CHECK(cudaEventRecord(e->ev_seg_copy, cs));
-                            issued_any = true;
-                            left -= b - a;
-                            a = b;
-                        }
-                        /* no yield: the thread keeps its core, so a finished
-                         * segment waits microseconds, not a time slice */
-                    }
+                sink.during = [&](const uint32_t *, const uint32_t *d_path, uint32_t, uint32_t, uint32_t nseg,
+                                  const volatile uint32_t *flag, const volatile uint64_t *bound, cudaEvent_t walked) {
+                    stream_during(e, to, d_path, nseg, flag, bound, walked);
                 };
                 e->seg_sink = &sink;
             }
@@ -1102,37 +1145,75 @@ kk_status walk_to_host(kk_engine *e, const kk_walk_opts *opts, kk_paths **out, c
         const bool one_epoch = n > 0 && p->epoch_walkers >= n;
         const bool bounded = n > 0 && (custom != nullptr || opts->app == KK_APP_DEEPWALK ||
                                        opts->app == KK_APP_NODE2VEC);
+        /* the result block, for up to `verts` vertices */
+        auto make_block = [&](uint64_t verts) {
+            const size_t len_bytes = ((size_t)n * 4 + 15) & ~(size_t)15;
+            const size_t off_bytes = ((size_t)n * 8 + 15) & ~(size_t)15;
+            if (e->host_pool == nullptr)
+            {
+                e->host_pool = new HostPool();
+                e->host_pool->limit = kBatchPoolCache;
+            }
+            PooledPaths *o = new (std::nothrow) PooledPaths();
+            size_t cls = 0;
+            char *blk = o ? (char *)e->host_pool->get(len_bytes + off_bytes + verts * 4 + 16, &cls) : nullptr;
+            if (!blk)
+            {
+                delete o;
+                fail(KK_ERR_OOM, "host allocation failed");
+            }
+            o->pool = e->host_pool;
+            o->block = blk;
+            o->cls = cls;
+            p->owner = o;
+            p->length = (uint32_t *)blk;
+            p->offset = (uint64_t *)(blk + len_bytes);
+            p->vertices = (uint32_t *)(blk + len_bytes + off_bytes);
+        };
+        if (one_epoch && n > 0 && custom == nullptr && e->into_stream && opts->app != KK_APP_METAPATH &&
+            stream_pays(opts) && graph_no_dead_ends(e))
+        {
+            /* the path lengths are known before the walk: its segments leave
+             * for the block as they end, as in kk_walk_into */
+            make_copy_stream(e);
+            struct Restore
+            {
+                kk_engine *e;
+                ~Restore()
+                {
+                    e->seg_sink = nullptr;
+                    cudaStreamSynchronize(e->copy_stream);
+                }
+            } restore{e};
+            StreamDest to;
+            SegmentSink sink;
+            sink.before = [&](const uint64_t *d_off, uint32_t num, uint64_t total) {
+                make_block(total);
+                to = StreamDest{p->length, p->offset, p->vertices, 0};
+                stream_before(e, 0, to, d_off, num);
+            };
+            sink.during = [&](const uint32_t *, const uint32_t *d_path, uint32_t, uint32_t, uint32_t nseg,
+                              const volatile uint32_t *flag, const volatile uint64_t *bound, cudaEvent_t walked) {
+                stream_during(e, to, d_path, nseg, flag, bound, walked);
+            };
+            e->seg_sink = &sink;
+            const uint32_t *d_start = upload_start(e, opts);
+            WalkResult r;
+            run_epoch(e, opts, d_start, opts->walker_begin, n, true, r);
+            p->total_steps = r.total_steps;
+            KK_CUDA_CHECK(cudaStreamSynchronize(e->copy_stream));
+            return;
+        }
         if (one_epoch || bounded)
         {
             uint64_t base = 0, vcap = 0;
             p->total_steps = walk_epochs(e, opts, custom, [&](uint32_t done, uint32_t num, const uint32_t *d_len,
                                                               const uint64_t *d_off, const uint32_t *d_verts,
                                                               uint64_t total) {
-                const size_t len_bytes = ((size_t)n * 4 + 15) & ~(size_t)15;
-                const size_t off_bytes = ((size_t)n * 8 + 15) & ~(size_t)15;
                 if (p->owner == nullptr)
                 {
-                    if (e->host_pool == nullptr)
-                    {
-                        e->host_pool = new HostPool();
-                        e->host_pool->limit = kBatchPoolCache;
-                    }
                     vcap = one_epoch ? total : (uint64_t)n * ((uint64_t)opts->walk_length + 1);
-                    PooledPaths *o = new (std::nothrow) PooledPaths();
-                    size_t cls = 0;
-                    char *blk = o ? (char *)e->host_pool->get(len_bytes + off_bytes + vcap * 4 + 16, &cls) : nullptr;
-                    if (!blk)
-                    {
-                        delete o;
-                        fail(KK_ERR_OOM, "host allocation failed");
-                    }
-                    o->pool = e->host_pool;
-                    o->block = blk;
-                    o->cls = cls;
-                    p->owner = o;
-                    p->length = (uint32_t *)blk;
-                    p->offset = (uint64_t *)(blk + len_bytes);
-                    p->vertices = (uint32_t *)(blk + len_bytes + off_bytes);
+                    make_block(vcap);
                 }
                 if (base + total > vcap)
                     fail(KK_ERR_PATH_CAPACITY, "a walk exceeded its path capacity");
