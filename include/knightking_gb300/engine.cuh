@@ -1038,9 +1038,18 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
             /* the extension bound; a walker on an isolated start gets its one
              * vertex here, with no draws (its walk ends there at once: a bound
              * that is exact, packed paths or not) */
-            constant_extension_bound_kernel<<<grid_for(e, n, 256), 256, 0, e->stream>>>(
-                g, true, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext, 1u << 24, caps,
-                d_status);
+            int resident = 0;
+            KK_CUDA_CHECK(
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, constant_extension_bound_kernel, 256, 0));
+            const uint32_t warps = (uint32_t)e->sm_count * (resident > 0 ? resident : 1) * 8u;
+            const uint32_t per = n / warps + (n % warps != 0 || n == 0);
+            /* lanes of their own do live / 32 of a warp's evaluations, together
+             * mean / (mean + 16) of them count */
+            const double mean = 1.0 / (1.0 - (double)rs.const_ext + 1e-9);
+            const uint32_t together = (uint32_t)(31.0 * mean / (mean + 16.0)) + 1u;
+            constant_extension_bound_kernel<<<(unsigned)(n / (per * 8ull) + 1), 256, 0, e->stream>>>(
+                g, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext, 1u << 24, per,
+                together < 31u ? together : 31u, caps, d_status);
             count_launch(e);
             KK_CUDA_CHECK(cudaGetLastError());
         }
