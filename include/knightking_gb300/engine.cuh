@@ -913,7 +913,11 @@ void walk_regrouped(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc
  * (walk_straight_kernel, in small blocks); beyond, the
  * walkers in turn and the paths in tiles (walk_stream_kernel; next: a zeroed
  * word).  R-MAT 10, 1,024 walkers of 80 steps: 33 us against 39 in tiles;
- * R-MAT 22 weighted, 2.4 M walkers: 4.95 ms against 4.72 in tiles. */
+ * R-MAT 22 weighted, 2.4 M walkers: 4.95 ms against 4.72 in tiles.  Uneven
+ * walks, which end by themselves and leave the SM to the next block, take turns
+ * only from three times that many on (PPR of mean 33 over R-MAT 20 at 1.03, 2, 3
+ * and 4 times: 324, 422, 550, 678 us a thread each, 332, 436, 510, 604 in turn;
+ * DeepWalk of 40 steps at 1.03 and 2 times 166 and 281 against 172 and 242). */
 template <typename S, typename WC, typename TC, typename Bucket>
 void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
                      const WalkLaunch &L, bool uneven, uint32_t *next)
@@ -930,7 +934,7 @@ void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &t
     KK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, walk_stream_kernel<S, WC, TC, Bucket>,
                                                                 (int)bs, smem));
     const unsigned hold = (unsigned)e->sm_count * (resident > 0 ? resident : 1), all = grid_for(e, n, bs);
-    if (all > hold && !segments)
+    if (all > (uneven ? 3u : 1u) * hold && !segments)
     {
         walk_stream_kernel<S, WC, TC, Bucket><<<hold, bs, smem, e->stream>>>(g, wc, tc, alias, L, next);
     }
