@@ -701,7 +701,7 @@ bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *a
     if (t[3] - t[0] > 4 * hold)
         return false;
     AliasSmall a;
-    a.first = t[0]; /* the hubs keep 1024 threads a row, on the side stream */
+    a.first = t[0]; /* the hubs keep 1024 threads a row, in a launch of their own */
     a.big = t[3];
     a.big_blocks = a.big - a.first < hold ? a.big - a.first : hold;
     const uint32_t per[kAliasSmallClasses] = {1, 2, 4, 8, 16};
@@ -715,20 +715,26 @@ bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *a
     }
     const uint32_t want = a.big_blocks + (sum_tasks + 7) / 8;
     const uint32_t grid = want < hold ? want : hold;
+    cudaStream_t small = e->stream;
     if (a.first)
     {
+        /* the hubs on the main stream, where they start at once, and the rest
+         * behind the event on the side stream: the other way round, the rest's
+         * resident blocks may take every SM first and the hubs, the longest
+         * rows, wait for one to leave (R-MAT 18: 192 us, or 315 when they did) */
+        small = e->side;
         KK_CUDA_CHECK(cudaEventRecord(e->ev_fork, e->stream));
-        KK_CUDA_CHECK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
         const uint32_t cap = (uint32_t)(e->sm_count > 1 ? e->sm_count / 2 : 1);
-        alias_build_hub_kernel<TC, Bucket><<<a.first < cap ? a.first : cap, 1024, 0, e->side>>>(
+        alias_build_hub_kernel<TC, Bucket><<<a.first < cap ? a.first : cap, 1024, 0, e->stream>>>(
             g, tc, alias, vcur, sum, scratch, (const uint32_t *)e->order.p, 0, a.first, next + 2);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
+        KK_CUDA_CHECK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
     }
     if (grid)
     {
-        alias_small_kernel<TC, Bucket><<<grid, 256, kAliasSmallSmem, e->stream>>>(g, tc, alias, vcur, sum, scratch,
-                                                                                 rows, a, next);
+        alias_small_kernel<TC, Bucket><<<grid, 256, kAliasSmallSmem, small>>>(g, tc, alias, vcur, sum, scratch, rows,
+                                                                              a, next);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
