@@ -276,8 +276,18 @@ struct SegmentSink
     std::function<void(const uint32_t *d_len, const uint32_t *d_path, uint32_t n, uint32_t shift, uint32_t nseg,
                        const volatile uint32_t *flag, const volatile uint64_t *bound, cudaEvent_t walked)>
         during;
+    /* or, without before and during: the walk is launched, and its packed
+     * paths may be queued for the host behind it */
+    std::function<void(const uint32_t *d_len, const uint64_t *d_off, const uint32_t *d_path, uint32_t n)> after;
     bool used = false;
 };
+
+/* Vertices (8 MB) up to which a walk of one length gets a path buffer for n
+ * whole paths, isolated starts or not, and kk_walk's copy follows it on its
+ * stream (host wall of a call, copied after the host knows the total / behind
+ * the walk: DeepWalk R-MAT 12 at 0.1, 1, 8 and 16 MB 76/65, 88/78, 157/147 and
+ * 223/227 us; node2vec R-MAT 14 at 1, 8 and 12 MB 160/146, 249/235 and 289/288). */
+constexpr uint64_t kBoundedVertices = 1u << 21;
 
 struct RunSpec
 {
@@ -375,6 +385,7 @@ struct kk_engine
     kk::DevBuf batch_small, batch_rel;
     kk::HostPool *host_pool = nullptr;
     cudaEvent_t ev_walked[3] = {nullptr, nullptr, nullptr}, ev_copied[3] = {nullptr, nullptr, nullptr};
+    cudaEvent_t ev_bound = nullptr;    /* after a walk's path offsets */
     cudaEvent_t ev_seg_copy = nullptr; /* after the last streamed segment copy issued */
     /* no walker can reach a vertex without out-edges except by starting on
      * one (every edge's target has out-edges); cached per graph */
@@ -549,6 +560,9 @@ void exclusive_scan_u64(kk_engine *e, const uint64_t *in, uint64_t *out, uint64_
 /* The same on stream st with temporary storage tmp. */
 void exclusive_scan_u64(kk_engine *e, const uint64_t *in, uint64_t *out, uint64_t n, cudaStream_t st,
                         kk::DevBuf &tmp);
+
+/* off[0..n]: the path offsets of c's walkers, on the engine's stream. */
+void exact_offsets(kk_engine *e, const ExactCap &c, uint64_t *off);
 
 /* Sorts n (key, value) pairs by the low `bits` bits of the key (stable), on
  * the engine's stream: the regrouped walk's records by vertex. */
@@ -986,6 +1000,89 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
     unsigned long long *d_steps = (unsigned long long *)((char *)d_status + 16);
     KK_CUDA_CHECK(cudaMemsetAsync(d_status, 0, 64, e->stream));
     KK_CUDA_CHECK(cudaEventRecord(e->ev[0], e->stream));
+    WalkLaunch L;
+    L.seed = rs.seed;
+    L.walker_begin = rs.walker_begin;
+    L.walker_num = n;
+    L.start = rs.d_start;
+    L.n_start = rs.n_start;
+    L.total_steps = d_steps;
+    L.status = d_status;
+    L.trial_limit = e->trial_limit;
+    L.stats = e->walk_stats ? (unsigned long long *)((char *)d_status + 24) : nullptr;
+    /* the walk's output set (two sets let a chunked kk_walk_into walk one
+     * chunk while the previous one is packed and copied out) */
+    const int ws = e->walk_set;
+    kk::DevBuf &b_length = ws ? e->length_x[ws - 1] : e->length, &b_caps = ws ? e->caps_x[ws - 1] : e->caps;
+    kk::DevBuf &b_off = ws ? e->path_off_x[ws - 1] : e->path_off, &b_path = ws ? e->path_x[ws - 1] : e->path;
+    L.length = b_length.as<uint32_t>(n);
+    uint64_t total_cap;
+    bool wait_total = false;
+    const bool exact = rs.exact && rs.packed_out && rs.want_paths && graph_no_dead_ends(e);
+    const bool stream_out = exact && e->seg_sink != nullptr && e->seg_sink->before && n > 0;
+    uint32_t seg_shift = 0, nseg = 0, *seg_count = nullptr;
+    if (rs.fixed_cap && !exact)
+    {
+        L.path_off = nullptr;
+        L.cap = rs.cap;
+        total_cap = (uint64_t)n * rs.cap;
+    }
+    else
+    {
+        uint64_t *off = b_off.as<uint64_t>((uint64_t)n + 1);
+        if (!rs.fixed_cap)
+        {
+            uint64_t *caps = b_caps.as<uint64_t>((uint64_t)n + 1);
+            KK_CUDA_CHECK(cudaMemsetAsync(caps + n, 0, sizeof(uint64_t), e->stream));
+            /* the extension bound; a walker on an isolated start gets its one
+             * vertex here, with no draws (its walk ends there at once: a bound
+             * that is exact, packed paths or not) */
+            int resident = 0;
+            KK_CUDA_CHECK(
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, constant_extension_bound_kernel, 256, 0));
+            const uint32_t warps = (uint32_t)e->sm_count * (resident > 0 ? resident : 1) * 8u;
+            const uint32_t per = n / warps + (n % warps != 0 || n == 0);
+            /* lanes of their own do live / 32 of a warp's evaluations, together
+             * mean / (mean + 16) of them count */
+            const double mean = 1.0 / (1.0 - (double)rs.const_ext + 1e-9);
+            const uint32_t together = (uint32_t)(31.0 * mean / (mean + 16.0)) + 1u;
+            constant_extension_bound_kernel<<<(unsigned)(n / (per * 8ull) + 1), 256, 0, e->stream>>>(
+                g, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext, 1u << 24, per,
+                together < 31u ? together : 31u, caps, d_status);
+            count_launch(e);
+            KK_CUDA_CHECK(cudaGetLastError());
+            exclusive_scan_u64(e, caps, off, (uint64_t)n + 1);
+        }
+        else
+        {
+            exact_offsets(e, ExactCap{g, rs.d_start, rs.n_start, rs.walker_begin, n, rs.cap}, off);
+        }
+        /* the paths' total sizes their buffer and its copy.  A small walk of one
+         * length takes the buffer for n paths of it, and nobody waits; else the
+         * host waits for the total while the tables are built (R-MAT 16, 65536
+         * node2vec walkers: 524 us a call, 543 to 557 with the wait behind them) */
+        total_cap = (uint64_t)n * rs.cap;
+        wait_total = stream_out || !rs.fixed_cap || total_cap > kBoundedVertices;
+        if (wait_total)
+            words_to_host(e, (const uint32_t *)(off + n), 32, 2); /* host words 32, 33 of the 64 */
+        if (stream_out)
+        {
+            /* streamed copy-out: segments of 2^shift >= 4096 walkers, at most
+             * kMaxSegments of them; flags cleared before the walk can set any */
+            seg_shift = 12;
+            while ((((uint64_t)n + (1ull << seg_shift) - 1) >> seg_shift) > kMaxSegments)
+                seg_shift++;
+            nseg = (uint32_t)(((uint64_t)n + (1ull << seg_shift) - 1) >> seg_shift);
+            memset((char *)e->h_status + kSegFlagAt, 0, (size_t)nseg * 4);
+            seg_count = e->seg_count.as<uint32_t>(kMaxSegments);
+            KK_CUDA_CHECK(cudaMemsetAsync(seg_count, 0, (size_t)nseg * 4, e->stream));
+            segment_bounds_to_host(e, off, n, seg_shift, nseg);
+        }
+        if (wait_total)
+            KK_CUDA_CHECK(cudaEventRecord(e->ev_bound, e->stream));
+        L.path_off = off;
+        L.cap = 0;
+    }
     const Bucket *alias = nullptr;
     const float *ra = nullptr;
     if constexpr (TC::has_static)
@@ -1012,88 +1109,14 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
         KK_CUDA_CHECK(cudaGetLastError());
         ra = rap;
     }
-    WalkLaunch L;
-    L.seed = rs.seed;
-    L.walker_begin = rs.walker_begin;
-    L.walker_num = n;
-    L.start = rs.d_start;
-    L.n_start = rs.n_start;
-    L.total_steps = d_steps;
     L.alias_sum = (const float *)e->sum.p;
-    L.status = d_status;
-    L.trial_limit = e->trial_limit;
-    L.stats = e->walk_stats ? (unsigned long long *)((char *)d_status + 24) : nullptr;
-    /* the walk's output set (two sets let a chunked kk_walk_into walk one
-     * chunk while the previous one is packed and copied out) */
-    const int ws = e->walk_set;
-    kk::DevBuf &b_length = ws ? e->length_x[ws - 1] : e->length, &b_caps = ws ? e->caps_x[ws - 1] : e->caps;
-    kk::DevBuf &b_off = ws ? e->path_off_x[ws - 1] : e->path_off, &b_path = ws ? e->path_x[ws - 1] : e->path;
-    L.length = b_length.as<uint32_t>(n);
-    uint64_t total_cap;
-    const bool exact = rs.exact && rs.packed_out && rs.want_paths && graph_no_dead_ends(e);
-    uint32_t seg_shift = 0, nseg = 0, *seg_count = nullptr;
-    if (rs.fixed_cap && !exact)
+    if (wait_total)
     {
-        L.path_off = nullptr;
-        L.cap = rs.cap;
-        total_cap = (uint64_t)n * rs.cap;
-    }
-    else
-    {
-        uint64_t *caps = b_caps.as<uint64_t>((uint64_t)n + 1);
-        uint64_t *off = b_off.as<uint64_t>((uint64_t)n + 1);
-        KK_CUDA_CHECK(cudaMemsetAsync(caps + n, 0, sizeof(uint64_t), e->stream));
-        if (!rs.fixed_cap)
-        {
-            /* the extension bound; a walker on an isolated start gets its one
-             * vertex here, with no draws (its walk ends there at once: a bound
-             * that is exact, packed paths or not) */
-            int resident = 0;
-            KK_CUDA_CHECK(
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, constant_extension_bound_kernel, 256, 0));
-            const uint32_t warps = (uint32_t)e->sm_count * (resident > 0 ? resident : 1) * 8u;
-            const uint32_t per = n / warps + (n % warps != 0 || n == 0);
-            /* lanes of their own do live / 32 of a warp's evaluations, together
-             * mean / (mean + 16) of them count */
-            const double mean = 1.0 / (1.0 - (double)rs.const_ext + 1e-9);
-            const uint32_t together = (uint32_t)(31.0 * mean / (mean + 16.0)) + 1u;
-            constant_extension_bound_kernel<<<(unsigned)(n / (per * 8ull) + 1), 256, 0, e->stream>>>(
-                g, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext, 1u << 24, per,
-                together < 31u ? together : 31u, caps, d_status);
-            count_launch(e);
-            KK_CUDA_CHECK(cudaGetLastError());
-        }
-        if (exact && rs.fixed_cap)
-        {
-            /* the full capacity, and one vertex for a walker on an isolated
-             * start */
-            exact_caps_kernel<<<grid_for(e, n, 256), 256, 0, e->stream>>>(g, rs.d_start, rs.n_start, rs.walker_begin,
-                                                                          n, rs.cap, caps);
-            count_launch(e);
-            KK_CUDA_CHECK(cudaGetLastError());
-        }
-        exclusive_scan_u64(e, caps, off, (uint64_t)n + 1);
-        words_to_host(e, (const uint32_t *)(off + n), 32, 2); /* host words 32, 33 of the 64 */
-        if (exact && e->seg_sink != nullptr && n > 0)
-        {
-            /* streamed copy-out: segments of 2^shift >= 4096 walkers, at most
-             * kMaxSegments of them; flags cleared before the walk can set any */
-            seg_shift = 12;
-            while ((((uint64_t)n + (1ull << seg_shift) - 1) >> seg_shift) > kMaxSegments)
-                seg_shift++;
-            nseg = (uint32_t)(((uint64_t)n + (1ull << seg_shift) - 1) >> seg_shift);
-            memset((char *)e->h_status + kSegFlagAt, 0, (size_t)nseg * 4);
-            seg_count = e->seg_count.as<uint32_t>(kMaxSegments);
-            KK_CUDA_CHECK(cudaMemsetAsync(seg_count, 0, (size_t)nseg * 4, e->stream));
-            segment_bounds_to_host(e, off, n, seg_shift, nseg);
-        }
-        KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
+        KK_CUDA_CHECK(cudaEventSynchronize(e->ev_bound));
         total_cap = ((volatile uint64_t *)e->h_status)[16];
-        L.path_off = off;
-        L.cap = 0;
         if (nseg > 0)
         {
-            e->seg_sink->before(off, n, total_cap);
+            e->seg_sink->before(L.path_off, n, total_cap);
             L.seg_count = seg_count;
             L.seg_flag = (volatile uint32_t *)((char *)e->d_status_host + kSegFlagAt);
             L.seg_shift = seg_shift;
@@ -1179,6 +1202,8 @@ launched:
                             (const volatile uint32_t *)((const char *)e->h_status + kSegFlagAt),
                             (const volatile uint64_t *)((const char *)e->h_status + kSegBoundAt), e->ev[2]);
     }
+    if (exact && e->seg_sink != nullptr && e->seg_sink->after)
+        e->seg_sink->after(L.length, L.path_off, L.path, n);
     words_to_host(e, (const uint32_t *)d_status, 0, 16);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     int h_small[16];

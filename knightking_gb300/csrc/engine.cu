@@ -87,6 +87,26 @@ __global__ void length_to_u64_kernel(const uint32_t *len, uint64_t *out, uint32_
         out[i] = i < n ? len[i] : 0;
 }
 
+/* A small walk's packed paths into the caller's pinned block, behind the walk
+ * on its stream: one launch, and no total for the host to wait for, in place of
+ * three copies after it (kBoundedVertices has the figures).  Writes to host
+ * memory bound it. */
+__global__ void paths_to_host_kernel(uint32_t n, const uint32_t *len, const uint64_t *off, const uint32_t *path,
+                                     uint32_t *h_len, uint64_t *h_off, uint32_t *h_vert)
+{
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t total = off[n], quads = total / 4;
+    for (uint64_t i = t; i < quads; i += step)
+        reinterpret_cast<uint4 *>(h_vert)[i] = reinterpret_cast<const uint4 *>(path)[i];
+    if (t < total % 4)
+        h_vert[quads * 4 + t] = path[quads * 4 + t];
+    for (uint64_t i = t; i < n; i += step)
+    {
+        h_len[i] = len[i];
+        h_off[i] = off[i];
+    }
+}
+
 __global__ void words_to_host_kernel(const uint32_t *src, volatile uint32_t *dst, int n)
 {
     if (threadIdx.x < (unsigned)n)
@@ -731,6 +751,7 @@ kk_status kk_engine_create(kk_engine **out, int device)
         for (int i = 0; i < 3; i++)
             KK_CUDA_CHECK(cudaEventCreate(&e->ev[i]));
         KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
+        KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_bound, cudaEventDisableTiming));
         KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
         KK_CUDA_CHECK(cudaEventCreateWithFlags(&e->ev_hub_join, cudaEventDisableTiming));
         /* mapped pinned words the walks' status and capacity reads land in:
@@ -770,6 +791,8 @@ void kk_engine_destroy(kk_engine *e)
             cudaEventDestroy(e->ev[i]);
     if (e->ev_fork)
         cudaEventDestroy(e->ev_fork);
+    if (e->ev_bound)
+        cudaEventDestroy(e->ev_bound);
     if (e->ev_join)
         cudaEventDestroy(e->ev_join);
     if (e->ev_hub_join)
@@ -1202,6 +1225,39 @@ kk_status walk_to_host(kk_engine *e, const kk_walk_opts *opts, kk_paths **out, c
             run_epoch(e, opts, d_start, opts->walker_begin, n, true, r);
             p->total_steps = r.total_steps;
             KK_CUDA_CHECK(cudaStreamSynchronize(e->copy_stream));
+            return;
+        }
+        const uint64_t vbound = (uint64_t)n * ((uint64_t)opts->walk_length + 1);
+        if (one_epoch && bounded && custom == nullptr && vbound <= kBoundedVertices && graph_no_dead_ends(e))
+        {
+            /* known lengths and few vertices: the paths follow the walk on its
+             * stream, into a block for n whole ones */
+            make_block(vbound);
+            struct Restore
+            {
+                kk_engine *e;
+                bool queued;
+                ~Restore()
+                {
+                    e->seg_sink = nullptr;
+                    if (queued)
+                        cudaStreamSynchronize(e->stream);
+                }
+            } restore{e, false};
+            SegmentSink sink;
+            sink.after = [&](const uint32_t *d_len, const uint64_t *d_off, const uint32_t *d_path, uint32_t num) {
+                restore.queued = true;
+                paths_to_host_kernel<<<grid_for(e, vbound / 4 + 1, 256), 256, 0, e->stream>>>(
+                    num, d_len, d_off, d_path, p->length, p->offset, p->vertices);
+                count_launch(e);
+                KK_CUDA_CHECK(cudaGetLastError());
+            };
+            e->seg_sink = &sink;
+            const uint32_t *d_start = upload_start(e, opts);
+            WalkResult r;
+            run_epoch(e, opts, d_start, opts->walker_begin, n, true, r);
+            restore.queued = false; /* the call has waited for the stream */
+            p->total_steps = r.total_steps;
             return;
         }
         if (one_epoch || bounded)

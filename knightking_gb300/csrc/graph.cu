@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
 #include <memory>
 #include <string>
@@ -51,6 +52,22 @@ void exclusive_scan_u64(kk_engine *e, const uint64_t *in, uint64_t *out, uint64_
 void exclusive_scan_u64(kk_engine *e, const uint64_t *in, uint64_t *out, uint64_t n)
 {
     exclusive_scan_u64(e, in, out, n, e->stream, e->cub_tmp);
+}
+
+void exact_offsets(kk_engine *e, const ExactCap &c, uint64_t *off)
+{
+    if (c.n < kOffsetBlocks * kOffsetWalkers)
+    {
+        exact_offsets_kernel<<<c.n / kOffsetWalkers + 1, 1024, 0, e->stream>>>(c, off);
+        count_launch(e);
+        KK_CUDA_CHECK(cudaGetLastError());
+        return;
+    }
+    const auto caps = thrust::make_transform_iterator(thrust::make_counting_iterator(0u), c);
+    size_t bytes = 0;
+    KK_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, caps, off, (int64_t)c.n + 1, e->stream));
+    void *tmp = e->cub_tmp.ensure(bytes);
+    KK_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(tmp, bytes, caps, off, (int64_t)c.n + 1, e->stream));
 }
 
 void sort_pairs_u32(kk_engine *e, const uint32_t *keys_in, uint32_t *keys_out, const uint32_t *vals_in,
