@@ -1374,10 +1374,23 @@ __device__ __forceinline__ void alias_q1_chain(float *F, uint16_t *Pq, uint16_t 
     }
 }
 
+/* Words from one row's probabilities to the next row's, and from one row's
+ * queues to the next's: the lanes of a group touch G consecutive words (G / 2 of
+ * a queue), so rows G words apart modulo 32 share no bank, where rows of DMAX
+ * words all began on one (the builds of R-MAT 22 and of 1 M vertices with 32
+ * edges each 1932 -> 1826 and 640 -> 515 us; shared memory was their busiest
+ * unit). */
+template <uint32_t G, uint32_t DMAX>
+struct AliasRowWords
+{
+    static constexpr uint32_t f = DMAX + (G < 32 ? G : 0), q = DMAX + (G < 32 ? (G + 1) / 2 : 0);
+    static constexpr uint32_t warp = (32 / G) * (f + q);
+};
+
 template <uint32_t G, uint32_t DMAX>
 constexpr size_t alias_group_smem_per_warp()
 {
-    return (size_t)(32 / G) * DMAX * 8;
+    return (size_t)AliasRowWords<G, DMAX>::warp * 4;
 }
 
 /* Warps per block of the lane-group kernels: each warp works alone (its own
@@ -1400,8 +1413,9 @@ __device__ __forceinline__ void alias_group_rows(const GraphView &g, const TC &t
     constexpr uint32_t gbits = G == 32 ? kFullMask : (1u << G) - 1u;
     const uint32_t lane = threadIdx.x & 31, grp = lane / G, gl = lane % G, gsh = grp * G;
     const uint32_t glt = (1u << gl) - 1u;
-    float *F = reinterpret_cast<float *>(smem) + (size_t)grp * DMAX;
-    uint16_t *Pq = reinterpret_cast<uint16_t *>(smem + (size_t)RPW * DMAX) + (size_t)grp * 2 * DMAX;
+    typedef AliasRowWords<G, DMAX> Row;
+    float *F = reinterpret_cast<float *>(smem) + (size_t)grp * Row::f;
+    uint16_t *Pq = reinterpret_cast<uint16_t *>(smem + (size_t)RPW * Row::f + (size_t)grp * Row::q);
     uint16_t *Qq = Pq + DMAX;
     const uint32_t v = d.v, deg = d.deg;
     const int64_t e0 = d.e0;
@@ -1538,8 +1552,7 @@ __global__ void __launch_bounds__(32 * kAliasGroupWarps) alias_group_kernel(Grap
 {
     constexpr uint32_t RPW = 32 / G;
     extern __shared__ uint32_t smem_all[];
-    /* this warp's slice: 8 B per edge of its RPW rows */
-    uint32_t *smem = smem_all + (size_t)(threadIdx.x >> 5) * RPW * DMAX * 2;
+    uint32_t *smem = smem_all + (size_t)(threadIdx.x >> 5) * AliasRowWords<G, DMAX>::warp; /* this warp's slice */
     const uint32_t lane = threadIdx.x & 31, grp = lane / G;
     /* the next vertices' counter value and row descriptors are fetched while
      * the current ones are processed */
@@ -1846,7 +1859,8 @@ __global__ void __launch_bounds__(1024) alias_build_hub_kernel(GraphView g, TC t
  * else alias_block_row); every block then takes warp tasks (the lane groups of
  * classes 4 to 8, 32 / G rows a task, largest first) until none is left. */
 constexpr uint32_t kAliasSmallClasses = 5;
-constexpr uint32_t kAliasSmallSmem = 8 * 1024 * 8; /* 8 warps' class-4 rows, 8 B an edge */
+constexpr uint32_t kAliasSmallSmem = 8 * AliasRowWords<16, 512>::warp * 4; /* 8 warps' rows of the widest class */
+static_assert(AliasRowWords<32, 1024>::warp <= AliasRowWords<16, 512>::warp, "a warp's rows fit");
 struct AliasSmall
 {
     uint32_t first, big, big_blocks;     /* rows [first, big) of more than 1024 edges, the blocks that take them */
