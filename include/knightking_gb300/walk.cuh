@@ -635,9 +635,9 @@ constexpr bool use_cursor_buckets()
  *        pairing, queues in the 16 B/edge scratch at 2*off[v]; batches of 64
  *        or fewer go to one warp (no block barrier); on a side stream;
  *   4097..16384: the same kernel with 256-thread blocks, several per SM;
- *   2049..4096: a block per vertex, the row and its queues in shared memory
- *        (alias_block_row_kernel);
- *   1..2048: groups of G lanes per vertex, 32/G vertices per warp, rows and
+ *   1025..4096: a block per vertex, of 256 threads above 2048, else 128, the
+ *        row and its queues in shared memory (alias_block_row_kernel);
+ *   1..1024: groups of G lanes per vertex, 32/G vertices per warp, rows and
  *        queues in shared memory (alias_group_kernel): G = 32 above 512,
  *        16 above 128, 8 above 32, 4 above 16, else 2.
  * A group's batches are at most G wide; the average batch of a FIFO pairing
@@ -1420,18 +1420,23 @@ __device__ __forceinline__ void alias_group_rows(const GraphView &g, const TC &t
     const uint32_t v = d.v, deg = d.deg;
     const int64_t e0 = d.e0;
     const uint32_t wdeg = __reduce_max_sync(kFullMask, deg);
-    /* stage the rows' probabilities, G consecutive edges per load */
+    /* stage the rows' probabilities, G consecutive edges per load, and zeros up
+     * to the warp's longest row */
+    const uint32_t wend = (wdeg + 3u) & ~3u;
 #pragma unroll 4
-    for (uint32_t i = gl; i < wdeg; i += G)
-        if (i < deg)
-            F[i] = static_at(g, tc, v, e0 + i);
+    for (uint32_t i = gl; i < wend; i += G)
+        F[i] = i < deg ? static_at(g, tc, v, e0 + i) : 0.0f;
+    /* the bucket pass reads the row's neighbours in pop order, each a miss
+     * unless the lines are on their way (R-MAT 22 1800 -> 1729 us) */
+    for (uint32_t i = gl * 32; i < deg; i += G * 32)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(g.nbr + e0 + i));
     __syncwarp();
     mid(); /* the rows are on their way: the caller fetches what comes next */
     /* the sum in edge order (:579-584), one lane per group */
     float sum = 0.0f;
     if constexpr (RPW == 1)
     {
-        /* rows of 513..2048 edges: the exact warp scan */
+        /* rows of 513..1024 edges: the exact warp scan */
         sum = warp_exact_sum<8>(F, deg);
         if (lane == 0 && deg != 0 && sum_out != nullptr)
             sum_out[v] = sum;
@@ -1439,16 +1444,29 @@ __device__ __forceinline__ void alias_group_rows(const GraphView &g, const TC &t
     else if (gl == 0)
     {
         /* a group past its row's end adds +0.0f, which leaves a sum of
-         * non-negative terms unchanged, so the FADD chain has no select */
-        uint32_t i = 0;
-        for (; i + 4 <= wdeg; i += 4)
+         * non-negative terms unchanged, so that the loop is a read of four (two
+         * where rows are 8 B aligned) and their FADDs */
+        if constexpr (G >= 4)
         {
-            const float a0 = i < deg ? F[i] : 0.0f, a1 = i + 1 < deg ? F[i + 1] : 0.0f;
-            const float a2 = i + 2 < deg ? F[i + 2] : 0.0f, a3 = i + 3 < deg ? F[i + 3] : 0.0f;
-            sum = fadd(fadd(fadd(fadd(sum, a0), a1), a2), a3);
+            for (uint32_t i = 0; i < wend; i += 4)
+            {
+                const float4 a = *reinterpret_cast<const float4 *>(F + i);
+                sum = fadd(fadd(fadd(fadd(sum, a.x), a.y), a.z), a.w);
+            }
         }
-        for (; i < wdeg; i++)
-            sum = fadd(sum, i < deg ? F[i] : 0.0f);
+        else if constexpr (G == 2)
+        {
+            for (uint32_t i = 0; i < wend; i += 4)
+            {
+                const float2 a = *reinterpret_cast<const float2 *>(F + i), b = *reinterpret_cast<const float2 *>(F + i + 2);
+                sum = fadd(fadd(fadd(fadd(sum, a.x), a.y), b.x), b.y);
+            }
+        }
+        else
+        {
+            for (uint32_t i = 0; i < wend; i++)
+                sum = fadd(sum, F[i]);
+        }
         if (deg != 0 && sum_out != nullptr)
             sum_out[v] = sum;
     }
@@ -1619,6 +1637,8 @@ __device__ __forceinline__ void alias_block_row(const GraphView &g, const TC &tc
 #pragma unroll 4
     for (uint32_t i = tid; i < deg; i += NT)
         F[i] = static_at(g, tc, v, e0 + i);
+    for (uint32_t i = tid * 32; i < deg; i += NT * 32)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(g.nbr + e0 + i));
     __syncthreads();
     /* the sum in edge order (:579-584), exact block scan */
     const float sum = block_exact_sum<4>([&](uint32_t i) { return F[i]; }, deg, sh.maps, &sh.f, &sh.u, nullptr);
