@@ -693,10 +693,10 @@ void launch_alias_class(kk_engine *e, K kern, unsigned nt, size_t smem, uint32_t
 /* The build in one launch beside the hubs', for graphs of up to
  * kAliasSmallEdges edges whose rows of 1025 to 16384 edges are at most four a
  * resident block (a block of 256 threads takes each; more of them, and the
- * classes' own launches fill the SMs better); false: left to those.  Classes
- * against one launch, us: R-MAT 8 48 / 19, 10 71 / 28, 14 151 / 45, 16 219 /
- * 95, 18 366 / 188, 19 384 / 296, 20 690 / 743 (3,000 such rows: classes); a
- * graph of 1 M vertices and 32 M edges with 200 such rows 691 / 559. */
+ * classes' own launches fill the SMs as well); false: left to those.  Classes
+ * against one launch, us: R-MAT 8 53 / 25, 10 64 / 34, 14 101 / 45, 16 145 / 75,
+ * 18 250 / 139, 19 334 / 229, 20 525 / 517 (6,000 such rows); a graph of 1 M
+ * vertices and 32 M edges with 200 such rows 540 / 494. */
 constexpr uint64_t kAliasSmallEdges = 40000000;
 
 template <typename TC, typename Bucket>
@@ -832,7 +832,20 @@ void build_alias(kk_engine *e, const TC &tc)
                                count_launch(e);
                            });
     }
-    /* 1..2048: lane groups, 32/G vertices per warp */
+    /* 1025..2048: the same in 128 threads; a warp each, at 16 KB a warp, filled a
+     * sixth of the SM (class launches of R-MAT 14, 18 and 20 133 -> 90, 281 -> 250
+     * and 532 -> 526 us) */
+    {
+        static int res = 0;
+        constexpr size_t smem = alias_block_row_smem<2048>();
+        launch_alias_class(e, alias_block_row_kernel<TC, Bucket, 128, 2048>, 128, smem, 1, t[2], t[3], res,
+                           [&](unsigned grid) {
+                               alias_block_row_kernel<TC, Bucket, 128, 2048>
+                                   <<<grid, 128, smem, st>>>(g, tc, alias, vcur, sum, order, t[2], t[3], next + 3);
+                               count_launch(e);
+                           });
+    }
+    /* 1..1024: lane groups, 32/G vertices per warp */
     auto group = [&](auto kern, uint32_t G, size_t smem_warp, int c, int &res, cudaStream_t s) {
         constexpr unsigned W = kAliasGroupWarps;
         const size_t smem = smem_warp * W;
@@ -853,8 +866,7 @@ void build_alias(kk_engine *e, const TC &tc)
             KK_CUDA_CHECK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
         light = e->side;
     }
-    static int r3 = 0, r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0;
-    group(alias_group_kernel<TC, Bucket, 32, 2048>, 32, alias_group_smem_per_warp<32, 2048>(), 3, r3, st);
+    static int r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0;
     group(alias_group_kernel<TC, Bucket, 32, 1024>, 32, alias_group_smem_per_warp<32, 1024>(), 4, r4, st);
     group(alias_group_kernel<TC, Bucket, 16, 512>, 16, alias_group_smem_per_warp<16, 512>(), 5, r5,
           e->alias_streams >= 3 ? light : st);
