@@ -444,9 +444,13 @@ bool graph_no_dead_ends(kk_engine *e)
         e->no_dead_ends = e->dead_ends_valid = true; /* every vertex has out-edges */
     if (!e->dead_ends_valid)
     {
-        int *flag = (int *)e->small.ensure(64) + 12; /* a word the walks' status does not use */
-        KK_CUDA_CHECK(cudaMemsetAsync(flag, 0, sizeof(int), e->stream));
-        dead_end_kernel<<<grid_for(e, e->E, 256), 256, 0, e->stream>>>(e->view(), flag);
+        int *flag = (int *)e->small.ensure(64) + 12; /* words the walks' status does not use */
+        uint32_t *some = (uint32_t *)flag + 1, *bits = (uint32_t *)e->cub_tmp.ensure(((size_t)e->V / 32 + 1) * 4);
+        KK_CUDA_CHECK(cudaMemsetAsync(flag, 0, 2 * sizeof(int), e->stream));
+        alive_bits_kernel<<<grid_for(e, e->V, 256), 256, 0, e->stream>>>(e->d_off, e->V, bits, some);
+        count_launch(e);
+        const unsigned grid = grid_for(e, e->E, 256), cap = 16u * (unsigned)e->sm_count;
+        dead_end_kernel<<<grid < cap ? grid : cap, 256, 0, e->stream>>>(e->d_nbr, e->E, bits, some, flag);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
         words_to_host(e, (const uint32_t *)flag, 40, 1);
@@ -810,14 +814,60 @@ __global__ void offsets_from_sorted_kernel(const uint32_t *s, uint64_t m, uint32
     }
 }
 
-__global__ void unpack_values_kernel(const uint64_t *val, uint64_t m, uint32_t *nbr, float *w)
+/* The CSR from records sorted by source: offsets where the source changes,
+ * neighbours and weights out of the values.  Four records a thread, 16 B a read
+ * and a write; bytes bound it (22 M weighted records 141 us in two passes of a
+ * record a thread, 63 in this one). */
+__global__ void csr_from_sorted_kernel(const uint32_t *key, const uint64_t *val, uint64_t m, uint32_t V, int64_t *off,
+                                       uint32_t *nbr, float *w)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q <= m / 4;
+         q += (uint64_t)gridDim.x * blockDim.x)
     {
-        const uint64_t x = val[i];
-        nbr[i] = (uint32_t)x;
-        if (w != nullptr)
-            w[i] = __uint_as_float((uint32_t)(x >> 32));
+        const uint64_t i = 4 * q;
+        uint32_t k[4] = {0, 0, 0, 0};
+        int64_t last = i == 0 ? -1 : (int64_t)key[i - 1];
+        const uint32_t n = m - i < 4 ? (uint32_t)(m - i) : 4u;
+        if (n == 4)
+        {
+            const uint4 kk = *reinterpret_cast<const uint4 *>(key + i);
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(val + i);
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(val + i + 2);
+            k[0] = kk.x, k[1] = kk.y, k[2] = kk.z, k[3] = kk.w;
+            *reinterpret_cast<uint4 *>(nbr + i) =
+                make_uint4((uint32_t)x.x, (uint32_t)x.y, (uint32_t)y.x, (uint32_t)y.y);
+            if (w != nullptr)
+                *reinterpret_cast<uint4 *>(w + i) = make_uint4((uint32_t)(x.x >> 32), (uint32_t)(x.y >> 32),
+                                                               (uint32_t)(y.x >> 32), (uint32_t)(y.y >> 32));
+        }
+        else
+        {
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+            {
+                if (j < n)
+                {
+                    const uint64_t x = val[i + j];
+                    k[j] = key[i + j];
+                    nbr[i + j] = (uint32_t)x;
+                    if (w != nullptr)
+                        w[i + j] = __uint_as_float((uint32_t)(x >> 32));
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++)
+        {
+            if (j < n)
+            {
+                for (int64_t v = last + 1; v <= (int64_t)k[j]; v++)
+                    off[v] = (int64_t)(i + j);
+                last = k[j];
+            }
+        }
+        if (n < 4) /* the last thread: the vertices past the last source */
+            for (int64_t v = last + 1; v <= (int64_t)V; v++)
+                off[v] = (int64_t)m;
     }
 }
 
@@ -877,12 +927,9 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
                                                   e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(e->cub_tmp.ensure(bytes), bytes, d_key, d_key2, d_val, d_val2,
                                                   (int64_t)m, 0, bits, e->stream));
-    offsets_from_sorted_kernel<<<grid_for(e, m + 1, 256), 256, 0, e->stream>>>(d_key2, m, V,
-                                                                               (int64_t *)e->gnext.off.p);
-    count_launch(e);
-    KK_CUDA_CHECK(cudaGetLastError());
-    unpack_values_kernel<<<grid_for(e, m ? m : 1, 256), 256, 0, e->stream>>>(
-        d_val2, m, (uint32_t *)e->gnext.nbr.p, weighted ? (float *)e->gnext.w.p : nullptr);
+    csr_from_sorted_kernel<<<grid_for(e, m / 4 + 1, 256), 256, 0, e->stream>>>(
+        d_key2, d_val2, m, V, (int64_t *)e->gnext.off.p, (uint32_t *)e->gnext.nbr.p,
+        weighted ? (float *)e->gnext.w.p : nullptr);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
     graph_commit(e, V, m, weighted, false, -1);
