@@ -1830,7 +1830,7 @@ __device__ __forceinline__ void alias_block_row(const GraphView &g, const TC &tc
 }
 
 template <typename TC, typename Bucket, uint32_t NT, uint32_t DMAX>
-__global__ void __launch_bounds__(NT) alias_block_row_kernel(GraphView g, TC tc, Bucket *out, const uint64_t *vcur,
+__global__ void __launch_bounds__(NT, 1536 / NT) alias_block_row_kernel(GraphView g, TC tc, Bucket *out, const uint64_t *vcur,
                                                              float *sum_out, const uint32_t *order, uint32_t lo,
                                                              uint32_t hi, uint32_t *next)
 {
