@@ -115,15 +115,14 @@ kk_status kk_engine_set_stream(kk_engine *e, void *stream);
  *                        lives: 32, 64, 128, or 0 for the value found (restored on destroy)
  *   "walk_stats"         1 counts trials, queries and probes (kk_last_walk_stats)
  *   "walk_multi"         walkers per thread (1, 2, 4) of first-order walks without a dynamic component
- *   "walk_park"          first-order walks with a dynamic component (rejection trials), one walker per
- *                        thread: once fewer than this many lanes of a warp are walking, its walkers stop
- *                        at their next step boundary and later launches resume them 32 to a warp
- *                        (0 off, 1..32; default 20)
+ *   "walk_park"          first-order walks with a dynamic component (rejection trials): 1..32 (default
+ *                        20; all alike) more walkers than the GPU holds at once take turns on the
+ *                        resident threads, 0 one walker per thread
  *   "alias_hub_grid"     blocks of the hub alias kernel (0: one per two SMs)
  *   "alias_streams"      1 the alias classes of degree <= 16384 in turn on the engine's stream,
  *                        2 those of degree <= 128 after the hubs on a second stream, beside the rest,
- *                        3 (default) those of degree <= 512, 4 those of degree <= 512 on the second
- *                        stream from the start and the hubs alone on a third
+ *                        3 (default) also those of degree 1025..16384 on a third, 4 those of degree
+ *                        <= 512 on the second stream from the start and the hubs alone on a third
  *   "alias_small_lanes"  0 (default) lane groups of 4 and 2 per row for the alias rows of degree
  *                        17..32 and 1..16; 1 groups of 2 and 1
  *   "into_stream"        1 (default): kk_walk_into walks whose path lengths are known before they

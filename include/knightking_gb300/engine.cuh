@@ -353,7 +353,7 @@ struct kk_engine
 
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     cudaStream_t side = nullptr; /* hub alias builds run here, joined by events */
-    cudaStream_t hub = nullptr;  /* alias_streams 4: the hubs alone on this stream */
+    cudaStream_t hub = nullptr;  /* alias_streams 4: the hubs alone on this stream; 3: rows of 1025..16384 */
     cudaEvent_t ev_hub_join = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     /* vertices by degree, descending (cached per graph), and the alias-build
@@ -458,8 +458,8 @@ struct kk_engine
      * SMs); fewer leave more of the SMs to the classes on the main stream */
     int alias_hub_grid = 0;
     /* alias_streams (option): 1 every class but the hubs on the main stream,
-     * 2 the classes of degree <= 128 after the hubs on the side stream, 3 the
-     * classes of degree <= 512 (S22 lognormal build 2.69 -> 2.50 ms); 4 the
+     * 2 the classes of degree <= 128 after the hubs on the side stream, 3 also
+     * the classes of degree 1025..16384 on a third stream; 4 the
      * hubs alone on a third stream, the classes of degree <= 512 on the side
      * stream from the start (a hub row's pairing is a long chain of rounds
      * that the small classes need not wait for) */
@@ -763,7 +763,7 @@ bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *a
 /* Builds alias tables in the Bucket layout into e->alias/e->sum for a
  * static functor: hubs on the side stream, the other classes in turn on the
  * main stream or (alias_streams) the small-row classes after the hubs on the
- * side stream, every class largest vertex first from its own counter. */
+ * side stream and the block classes on a third, every class largest vertex first from its own counter. */
 template <typename TC, typename Bucket = IndexBucket>
 void build_alias(kk_engine *e, const TC &tc)
 {
@@ -812,6 +812,18 @@ void build_alias(kk_engine *e, const TC &tc)
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
+    /* alias_streams 3: the block classes, 1025..16384, on the hub stream, where
+     * their last and longest rows share the SMs with the groups' (R-MAT 20, 21
+     * and 22 with those and the groups of 129 edges and more on the main stream
+     * and all others on the side stream 434, 880 and 1673 us, with everything
+     * above 512 on the main stream 524, 950 and 1694; lognormal weights 584, 1060
+     * and 1991, so 706, 1141 and 2018) */
+    const bool rows_beside = e->alias_streams == 3 && t[3] > t[0];
+    if (rows_beside)
+    {
+        KK_CUDA_CHECK(cudaStreamWaitEvent(e->hub, e->ev_fork, 0));
+        st = e->hub;
+    }
     /* 4097..16384: the hub kernel in 256-thread blocks */
     {
         static int res = 0;
@@ -845,6 +857,7 @@ void build_alias(kk_engine *e, const TC &tc)
                                count_launch(e);
                            });
     }
+    st = e->stream;
     /* 1..1024: lane groups, 32/G vertices per warp */
     auto group = [&](auto kern, uint32_t G, size_t smem_warp, int c, int &res, cudaStream_t s) {
         constexpr unsigned W = kAliasGroupWarps;
@@ -854,9 +867,9 @@ void build_alias(kk_engine *e, const TC &tc)
             count_launch(e);
         });
     };
-    /* alias_streams 2: the classes of degree <= 128 (2.5 to 5 KB of shared
+    /* alias_streams >= 2: the classes of degree <= 128 (2.5 to 5 KB of shared
      * memory per warp) follow the hubs on the side stream and share the SMs
-     * with the classes of large rows (10 to 48 KB per warp or block); 3: the
+     * with the classes of large rows (10 to 48 KB per warp or block); 4: the
      * class 129..512 with them */
     const bool split = e->alias_streams >= 2;
     cudaStream_t light = st;
@@ -869,7 +882,7 @@ void build_alias(kk_engine *e, const TC &tc)
     static int r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0;
     group(alias_group_kernel<TC, Bucket, 32, 1024>, 32, alias_group_smem_per_warp<32, 1024>(), 4, r4, st);
     group(alias_group_kernel<TC, Bucket, 16, 512>, 16, alias_group_smem_per_warp<16, 512>(), 5, r5,
-          e->alias_streams >= 3 ? light : st);
+          e->alias_streams == 4 ? light : st);
     group(alias_group_kernel<TC, Bucket, 8, 128>, 8, alias_group_smem_per_warp<8, 128>(), 6, r6, light);
     if (e->alias_small_lanes == 0)
     {
@@ -888,7 +901,7 @@ void build_alias(kk_engine *e, const TC &tc)
         KK_CUDA_CHECK(cudaEventRecord(e->ev_join, e->side));
         KK_CUDA_CHECK(cudaStreamWaitEvent(e->stream, e->ev_join, 0));
     }
-    if (hub_alone)
+    if (hub_alone || rows_beside)
     {
         KK_CUDA_CHECK(cudaEventRecord(e->ev_hub_join, e->hub));
         KK_CUDA_CHECK(cudaStreamWaitEvent(e->stream, e->ev_hub_join, 0));
