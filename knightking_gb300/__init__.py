@@ -538,11 +538,12 @@ class Server:
         paths = None
         total_steps = 0
         if r.paths:
-            try:
-                total_steps = r.paths.contents.total_steps
-                if keep_paths:
-                    paths = PathSet(*_capi.paths_to_numpy(r.paths.contents))
-            finally:
+            total_steps = r.paths.contents.total_steps
+            if keep_paths:
+                # views of the request's own pinned block, as batch_walk's are: copying them out of it took
+                # two thirds of a burst (16 requests, 42 MB of paths: 4.3 ms, 1.6 without)
+                paths = PathSet(*_capi.paths_to_numpy_owned(r.paths))
+            else:
                 self._lib.kk_paths_free(r.paths)
         res = ServeResult(paths, r.status, r.queue_ms, r.latency_ms, r.batch_jobs)
         res.total_steps = int(total_steps)
