@@ -693,10 +693,10 @@ void launch_alias_class(kk_engine *e, K kern, unsigned nt, size_t smem, uint32_t
 /* The build in one launch beside the hubs', for graphs of up to
  * kAliasSmallEdges edges whose rows of 1025 to 16384 edges are at most four a
  * resident block (a block of 256 threads takes each; more of them, and the
- * classes' own launches fill the SMs as well); false: left to those.  Classes
- * against one launch, us: R-MAT 8 53 / 25, 10 64 / 34, 14 101 / 45, 16 145 / 75,
- * 18 250 / 139, 19 334 / 229, 20 525 / 517 (6,000 such rows); a graph of 1 M
- * vertices and 32 M edges with 200 such rows 540 / 494. */
+ * classes' own launches fill the SMs better); false: left to those.  Classes
+ * against one launch, us: R-MAT 8 41 / 24, 10 43 / 37, 14 66 / 46, 16 104 / 77,
+ * 18 206 / 144, 19 262 / 231, 20 434 / 517 (6,000 such rows), 21 880 / 1015; a
+ * graph of 1 M vertices and 32 M edges with 200 such rows 526 / 497. */
 constexpr uint64_t kAliasSmallEdges = 40000000;
 
 template <typename TC, typename Bucket>
