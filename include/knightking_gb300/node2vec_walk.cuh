@@ -36,42 +36,6 @@ struct N2vParams
     step_t walk_length;
 };
 
-/* The same constants as the walk asks for them: in registers (or a launch's
- * constant bank), or read from the job's row, which L1 holds, at each use: a
- * batch's lanes have each their own, and eight registers more than the 64 of
- * four blocks an SM spill into the loop. */
-struct N2vInRegs
-{
-    N2vParams p;
-    __device__ __forceinline__ float upperbound() const { return p.upperbound; }
-    __device__ __forceinline__ float lowerbound() const { return p.lowerbound; }
-    __device__ __forceinline__ float overflow() const { return p.overflow; }
-    __device__ __forceinline__ float inv_p() const { return p.inv_p; }
-    __device__ __forceinline__ float inv_q() const { return p.inv_q; }
-    __device__ __forceinline__ float sure_below() const { return p.sure_below; }
-    __device__ __forceinline__ uint32_t walk_length() const { return p.walk_length; }
-};
-
-struct N2vInJob
-{
-    const BatchJob *job;
-    /* volatile: read here, not kept */
-    __device__ __forceinline__ static uint32_t word(const void *at)
-    {
-        uint32_t x;
-        asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(x) : "l"(at));
-        return x;
-    }
-    __device__ __forceinline__ float c(int k) const { return __uint_as_float(word(job->c + k)); }
-    __device__ __forceinline__ float upperbound() const { return c(0); }
-    __device__ __forceinline__ float lowerbound() const { return c(1); }
-    __device__ __forceinline__ float overflow() const { return c(2); }
-    __device__ __forceinline__ float inv_p() const { return c(3); }
-    __device__ __forceinline__ float inv_q() const { return c(4); }
-    __device__ __forceinline__ float sure_below() const { return fminf(c(4), 1.0f); }
-    __device__ __forceinline__ uint32_t walk_length() const { return word(&job->walk_length); }
-};
-
 /* What every walk of the launch reads. */
 template <typename Bucket>
 struct N2vTables
@@ -85,8 +49,8 @@ struct N2vTables
 /* Walks walker id from v to its end (the 32-bit offsets at hand), its path to
  * out (vertex 0 on; or nullptr); the path's length in len.  team: the warp's
  * lanes that call this together.  False when a step passed the trial limit. */
-template <bool Weighted, bool Outlier, typename Bucket, typename Params>
-__device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const Params &P,
+template <bool Weighted, bool Outlier, typename Bucket>
+__device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const N2vParams &P,
                                          walker_id_t id, vertex_id_t v, uint32_t *out, uint32_t trial_limit,
                                          unsigned long long *stats, unsigned team, Sampler &rng, uint32_t &len)
 {
@@ -111,15 +75,15 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
     uint64_t cand_cur = 0;
     float dart = 0.0f;
     /* q > 1: most candidates are no neighbours, and a no rejects */
-    const bool ahead = P.inv_q() < 1.0f;
+    const bool ahead = P.inv_q < 1.0f;
     auto begin_step = [&]() {
         rng.enter(id, step, 0);
         trials = 0;
         if constexpr (Outlier)
         {
-            const bool on = P.overflow() > 0.0f;
+            const bool on = P.overflow > 0.0f;
             find = Weighted && on;
-            ob = Weighted ? 0.0f : P.overflow();
+            ob = Weighted ? 0.0f : P.overflow;
             back_i = kNone;
             sec = kNone; /* find's first sector follows from the position */
             if (on)
@@ -134,7 +98,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
     begin_step();
     /* one way through the loop, and the warp's lanes (team) meet at its top:
      * they share the instructions of every pass */
-    bool alive = P.walk_length() > 0;
+    bool alive = P.walk_length > 0;
     while (__any_sync(team, alive))
     {
         if (alive)
@@ -184,9 +148,9 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                     if (Outlier && Weighted && look && !asked)
                     {
                         if (sec == kNone)
-                            sec = edge_set_sector(prev, edge_set_sectors(pe - pb, Weighted));
+                            sec = edge_set_sector(prev, edge_set_sectors(pe - pb, t.set.shift));
                         const uint4 *b = reinterpret_cast<const uint4 *>(
-                            t.set.keys + (edge_set_row(pb, v, Weighted) + sec) * kEdgeSectorWords);
+                            t.set.keys + (edge_set_row(pb, v, t.set.shift) + sec) * kEdgeSectorWords);
                         k0 = __ldg(b);
                         k1 = __ldg(b + 1);
                     }
@@ -201,13 +165,13 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                 if (m == 9)
                 {
                     /* undecided: the next sector, next time */
-                    sec = sec + 1 == (asked ? pn : edge_set_sectors(pe - pb, Weighted)) ? 0 : sec + 1;
+                    sec = sec + 1 == (asked ? pn : edge_set_sectors(pe - pb, t.set.shift)) ? 0 : sec + 1;
                     trial = false;
                 }
                 else if (asked)
                 {
                     query = false;
-                    taken = dart <= (m < 8 ? 1.0f : P.inv_q());
+                    taken = dart <= (m < 8 ? 1.0f : P.inv_q);
                     trial = trial && !taken;
                 }
                 else if constexpr (Outlier && Weighted)
@@ -222,7 +186,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                         if (edge)
                             back_w = gather(g.w + pb + back_i);
                     }
-                    ob = edge ? fmul(back_w, P.overflow()) : 0.0f;
+                    ob = edge ? fmul(back_w, P.overflow) : 0.0f;
                     find = false;
                 }
             }
@@ -230,7 +194,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
             {
                 back_i = 0;
                 back_w = gather(g.w + pb);
-                ob = fmul(back_w, P.overflow());
+                ob = fmul(back_w, P.overflow);
                 find = false;
             }
             if (trial)
@@ -243,7 +207,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                     {
                         float area = rav;
                         if (t.ra == nullptr)
-                            area = fmul(Weighted ? rav : u2f(pe - pb), P.upperbound());
+                            area = fmul(Weighted ? rav : u2f(pe - pb), P.upperbound);
                         const float r = fsub(map_gen_float(wd.x, fadd(fmul(ob, u2f(1u)), area)), area);
                         wd = make_uint4(wd.y, wd.z, wd.w, 0u);
                         drawn = 1;
@@ -267,7 +231,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                             }
                             cand = Weighted && at == kNone ? prev : some ? gather(g.nbr + pb + at) : 0;
                             cand_cur = ~0ull;
-                            dart = fadd(fdiv(fsub(r, fmul(u2f(oi), ob)), sc), P.upperbound());
+                            dart = fadd(fdiv(fsub(r, fmul(u2f(oi), ob)), sc), P.upperbound);
                         }
                     }
                 }
@@ -285,7 +249,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                             cand = first ? hi.x : hi.y;
                         if constexpr (Bucket::cursor)
                             cand_cur = first ? ((uint64_t)hi.y << 32) | hi.x : ((uint64_t)hi.w << 32) | hi.z;
-                        dart = map_gen_float(coin ? wd.z : wd.y, P.upperbound());
+                        dart = map_gen_float(coin ? wd.z : wd.y, P.upperbound);
                         drawn += coin ? 3u : 2u;
                     }
                     else
@@ -293,14 +257,14 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                         cand = lo.x;
                         if (g.adjc != nullptr)
                             cand_cur = ((uint64_t)lo.w << 32) | lo.z;
-                        dart = map_gen_float(wd.y, P.upperbound());
+                        dart = map_gen_float(wd.y, P.upperbound);
                         drawn += 2u;
                     }
-                    taken = dart <= P.lowerbound();
+                    taken = dart <= P.lowerbound;
                 }
                 rng.take(drawn, nxt);
                 const bool back = prev == cand;
-                if (!taken && some && step != 0 && !back && !(dart <= P.sure_below()))
+                if (!taken && some && step != 0 && !back && !(dart <= P.sure_below))
                 {
                     query = true;
                     if (stats != nullptr)
@@ -309,7 +273,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                 }
                 else if (!taken && some)
                 {
-                    taken = dart <= (step == 0 ? P.upperbound() : back ? P.inv_p() : P.inv_q());
+                    taken = dart <= (step == 0 ? P.upperbound : back ? P.inv_p : P.inv_q);
                 }
                 if (stats != nullptr)
                     atomicAdd(stats, 1ull);
@@ -319,8 +283,8 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
             if (taken)
             {
                 step++;
-                prow = (uint32_t)edge_set_row(pb, v, Weighted);
-                pn = edge_set_sectors(pe - pb, Weighted);
+                prow = (uint32_t)edge_set_row(pb, v, t.set.shift);
+                pn = edge_set_sectors(pe - pb, t.set.shift);
                 prev = v;
                 v = cand;
                 if (out != nullptr)
@@ -342,7 +306,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                     pe = gather(g.off32 + v + 1);
                 }
                 begin_step();
-                alive = step < P.walk_length();
+                alive = step < P.walk_length;
             }
         }
     }
@@ -365,7 +329,7 @@ __global__ void __launch_bounds__(256, 4) n2v_walk_kernel(GraphView g, N2vTables
         WalkerConfig<apps::Node2vecState> wc;
         walk_begin<apps::Node2vecState>(g, wc, L, i, run, rng);
         uint32_t len;
-        if (!n2v_walk<Weighted, Outlier, Bucket>(g, t, N2vInRegs{P}, run.w.id, run.v, run.out, L.trial_limit, L.stats, team, rng,
+        if (!n2v_walk<Weighted, Outlier, Bucket>(g, t, P, run.w.id, run.v, run.out, L.trial_limit, L.stats, team, rng,
                                                  len))
             atomicOr(L.status, KK_STATUS_TRIAL_LIMIT);
         L.length[i] = len;
@@ -450,19 +414,10 @@ __global__ void __launch_bounds__(256, MinBlocks)
         if (out != nullptr)
             out[0] = v;
         uint32_t len;
-        bool within;
-        if constexpr (MinBlocks >= 4)
-        {
-            within = n2v_walk<Weighted, true, Bucket>(g, t, N2vInJob{job}, id, v, out, trial_limit, stats, team, rng,
-                                                      len);
-        }
-        else
-        {
-            const N2vParams P{job->c[0], job->c[1], job->c[2], job->c[3], job->c[4], fminf(job->c[4], 1.0f),
-                              job->walk_length};
-            within = n2v_walk<Weighted, true, Bucket>(g, t, N2vInRegs{P}, id, v, out, trial_limit, stats, team, rng,
-                                                      len);
-        }
+        const N2vParams P{job->c[0], job->c[1], job->c[2], job->c[3], job->c[4], fminf(job->c[4], 1.0f),
+                          job->walk_length};
+        const bool within =
+            n2v_walk<Weighted, true, Bucket>(g, t, P, id, v, out, trial_limit, stats, team, rng, len);
         const uint32_t j = (uint32_t)(job - jobs);
         if (!within)
             atomicOr(nt.count != nullptr ? nt.status + j : status, KK_STATUS_TRIAL_LIMIT);

@@ -114,12 +114,11 @@ struct SecondOrderTransitionConfig
  * neighbour ids per row, in sectors of 32 B: eight ids, or in a weighted graph
  * four ids and their edges' weights (the weight of (u, v)'s first edge in u's
  * sorted adjacency, std::lower_bound's), so that either lookup is one read.
- * Row u of degree d at offset e0 has d / 4 + 1 sectors from sector e0 / 4 + u
- * on, weighted d / 2 + 1 from e0 / 2 + u (rows do not overlap: (e0 + d) / 4 >=
- * e0 / 4 + d / 4), so a lookup finds the row's table from its adjacency
- * position alone, the load is below 1/2, and the set takes 8 or 16 B an edge
- * and 32 B a vertex: it stays in L2 where a table of 64-bit (u, v) keys at
- * load 1/4 in 64 B buckets did not.  v's probe starts at sector
+ * Row u of degree d at offset e0 has (d >> shift) + 1 sectors from sector
+ * (e0 >> shift) + u on (rows do not overlap: (e0 + d) >> shift >= (e0 >> shift)
+ * + (d >> shift)), so a lookup finds the row's table from its adjacency position
+ * alone.  The shift sets the load, below 1/2 or 1/4: the set takes 8 B an edge
+ * unweighted, 16 or 32 weighted, and 32 B a vertex.  v's probe starts at sector
  * edge_set_sector(v) of the row and goes on in turn; an insert moves past a
  * sector only when its slots hold other ids, so a lookup that meets a free
  * slot may stop. */
@@ -130,20 +129,21 @@ struct EdgeSetView
     const uint32_t *keys; /* nullptr: no set */
     bool weighted;
     const int64_t *off;
+    uint32_t shift;
 };
 
-__host__ __device__ __forceinline__ uint64_t edge_set_row(int64_t e0, vertex_id_t u, bool weighted)
+__host__ __device__ __forceinline__ uint64_t edge_set_row(int64_t e0, vertex_id_t u, uint32_t shift)
 {
-    return ((uint64_t)e0 >> (weighted ? 1 : 2)) + u;
+    return ((uint64_t)e0 >> shift) + u;
 }
-__host__ __device__ __forceinline__ uint32_t edge_set_sectors(uint32_t deg, bool weighted)
+__host__ __device__ __forceinline__ uint32_t edge_set_sectors(uint32_t deg, uint32_t shift)
 {
-    return (deg >> (weighted ? 1 : 2)) + 1;
+    return (deg >> shift) + 1;
 }
 /* all rows' sectors */
-__host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t V, bool weighted)
+__host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t V, uint32_t shift)
 {
-    return (E >> (weighted ? 1 : 2)) + V + 1;
+    return (E >> shift) + V + 1;
 }
 /* where v's probe starts among a row's n sectors */
 __host__ __device__ __forceinline__ uint32_t edge_set_sector(vertex_id_t v, uint32_t n)
@@ -180,8 +180,8 @@ __device__ __forceinline__ uint32_t word_of(const uint4 &a, uint32_t j)
 __device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t u, int64_t e0, uint32_t deg,
                                               vertex_id_t v, float *weight)
 {
-    const uint64_t row = edge_set_row(e0, u, s.weighted);
-    const uint32_t n = edge_set_sectors(deg, s.weighted);
+    const uint64_t row = edge_set_row(e0, u, s.shift);
+    const uint32_t n = edge_set_sectors(deg, s.shift);
     uint32_t b = edge_set_sector(v, n);
     for (uint32_t probe = 0; probe < n; probe++)
     {
@@ -239,14 +239,15 @@ __device__ __forceinline__ void edge_set_fill(const GraphView &g, int64_t e0, ui
 /* The rows order[lo, hi), a block each (hubs): the row's table in global
  * memory. */
 static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g, uint32_t *keys,
-                                                                     const uint32_t *order, uint32_t lo, uint32_t hi)
+                                                                     const uint32_t *order, uint32_t lo, uint32_t hi,
+                                                                     uint32_t shift)
 {
     for (uint32_t k = lo + blockIdx.x; k < hi; k += gridDim.x)
     {
         const uint32_t u = order[k];
         const int64_t e0 = g.off[u];
-        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, g.w != nullptr);
-        uint32_t *row = keys + edge_set_row(e0, u, g.w != nullptr) * kEdgeSectorWords;
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, shift);
+        uint32_t *row = keys + edge_set_row(e0, u, shift) * kEdgeSectorWords;
         for (uint32_t i = threadIdx.x; i < n * kEdgeSectorWords; i += blockDim.x)
             row[i] = kNone;
         __syncthreads();
@@ -259,30 +260,31 @@ static __global__ void __launch_bounds__(1024) edge_set_block_kernel(GraphView g
  * in shared memory (its inserts are chains of atomics, ten times shorter there
  * than in L2), then out in one coalesced pass. */
 template <uint32_t DMAX>
-constexpr uint32_t edge_set_group_words(bool weighted)
+constexpr uint32_t edge_set_group_words(uint32_t shift)
 {
-    return (DMAX / (weighted ? 2 : 4) + 1) * kEdgeSectorWords;
+    return ((DMAX >> shift) + 1) * kEdgeSectorWords;
 }
 
 template <uint32_t G, uint32_t DMAX>
 static __global__ void __launch_bounds__(128) edge_set_group_kernel(GraphView g, uint32_t *keys,
-                                                                    const uint32_t *order, uint32_t lo, uint32_t hi)
+                                                                    const uint32_t *order, uint32_t lo, uint32_t hi,
+                                                                    uint32_t shift)
 {
     extern __shared__ uint32_t s_rows[];
     const uint32_t gl = threadIdx.x % G, grp = threadIdx.x / G, groups = blockDim.x / G;
     const unsigned mask = G == 32 ? kFullMask : ((1u << (G % 32)) - 1u) << (threadIdx.x % 32 / G * G);
-    uint32_t *row = s_rows + grp * edge_set_group_words<DMAX>(g.w != nullptr);
+    uint32_t *row = s_rows + grp * edge_set_group_words<DMAX>(shift);
     for (uint32_t k = lo + blockIdx.x * groups + grp; k < hi; k += gridDim.x * groups)
     {
         const uint32_t u = order[k];
         const int64_t e0 = g.off[u];
-        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, g.w != nullptr);
+        const uint32_t deg = (uint32_t)(g.off[u + 1] - e0), n = edge_set_sectors(deg, shift);
         for (uint32_t i = gl; i < n * kEdgeSectorWords; i += G)
             row[i] = kNone;
         __syncwarp(mask);
         edge_set_fill(g, e0, deg, row, n, gl, G);
         __syncwarp(mask);
-        const uint64_t at = edge_set_row(e0, u, g.w != nullptr) * kEdgeSectorWords;
+        const uint64_t at = edge_set_row(e0, u, shift) * kEdgeSectorWords;
         for (uint32_t i = gl; i < n * kEdgeSectorWords; i += G)
             keys[at + i] = row[i];
         __syncwarp(mask);

@@ -101,14 +101,15 @@ BatchPlan plan_batch(kk_engine *e, const kk_walk_opts *jobs, int n, bool longest
 namespace
 {
 
-/* node2vec batches of no more walkers than four blocks of 256 an SM wait on
- * latency: their kernel keeps a walk's state in registers at two blocks an SM
- * (20 jobs, 148,000 walkers, 32 M edges: walk 2.17 -> 1.55 ms); a larger batch
- * is bound by the reads of all SMs (512 jobs on R-MAT 22: 15.5 ms at four
- * blocks, 18.3 at two). */
+/* node2vec batches of up to 3072 walkers an SM wait on latency: their kernel
+ * has registers for a walk's state at two blocks of 256 an SM; a larger batch is
+ * bound by the reads of all SMs (two / three blocks, 1 M vertices, 32 M edges:
+ * 148,000 walkers 1.54 / 1.65 ms, 400,000 2.38 / 2.70, 540,000 3.77 / 3.62,
+ * 2.7 M 16.1 / 14.3; four blocks, whose walks spill, 1024 requests on R-MAT 20
+ * and 24 28.2 and 29.0 ms against 26.9 and 28.1 at three). */
 uint32_t batch_wide_limit(const kk_engine *e)
 {
-    return 1024u * (uint32_t)e->sm_count;
+    return 3072u * (uint32_t)e->sm_count;
 }
 bool batch_wide(const kk_engine *e, const BatchPlan &plan)
 {
@@ -168,7 +169,7 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
                 if (batch_wide(e, plan))
                     launch(n2v_batch_kernel<TC::has_static, Bucket, 2>);
                 else
-                    launch(n2v_batch_kernel<TC::has_static, Bucket, 4>);
+                    launch(n2v_batch_kernel<TC::has_static, Bucket, 3>);
                 launched = true;
             }
         }

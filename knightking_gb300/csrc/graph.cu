@@ -507,19 +507,34 @@ const uint4 *cursor_adjacency_of(kk_engine *e)
     return (const uint4 *)e->adjc.p;
 }
 
+/* Edges a sector, as a shift: an unweighted row's sectors, of eight ids, are
+ * half full; a weighted row's, of four, are a quarter full from 28 M edges on,
+ * where the set is far larger than L2 and a second sector costs a read of
+ * memory (of one in seven lookups that find nothing at half full, of one in
+ * fifty), and half full below, where the set's size counts.  Half / a quarter,
+ * walk: R-MAT 16, 65536 walkers 274 / 293 us; R-MAT 19, 300007 1155 / 1159;
+ * R-MAT 22, 2.4 M 7.78 / 7.37 ms; 20 jobs on 32 M edges 1.55 / 1.48; 1024
+ * requests on R-MAT 24 31.9 / 29.6.  24 M edges' load with the set 3.32 / 3.41. */
+static uint32_t edge_set_shift(const kk_engine *e)
+{
+    if (e->d_w == nullptr)
+        return 2;
+    return e->E >= 28000000 && e->E + e->V + 1 < (1ull << 32) ? 0 : 1; /* the walk counts sectors in 32 bits */
+}
+
 EdgeSetView node2vec_edge_set_built(const kk_engine *e)
 {
     if (e->n2v_adjacency != 0)
-        return EdgeSetView{nullptr, false, nullptr};
-    return EdgeSetView{(const uint32_t *)e->edge_set.p, e->d_w != nullptr, e->d_off};
+        return EdgeSetView{nullptr, false, nullptr, 0};
+    return EdgeSetView{(const uint32_t *)e->edge_set.p, e->d_w != nullptr, e->d_off, edge_set_shift(e)};
 }
 
 EdgeSetView node2vec_edge_set(kk_engine *e)
 {
     if (e->n2v_adjacency != 0 || e->edge_set_valid)
         return node2vec_edge_set_built(e);
-    const bool weighted = e->d_w != nullptr;
-    uint32_t *keys = e->edge_set.as<uint32_t>(edge_set_total(e->E, e->V, weighted) * kEdgeSectorWords);
+    const uint32_t shift = edge_set_shift(e);
+    uint32_t *keys = e->edge_set.as<uint32_t>(edge_set_total(e->E, e->V, shift) * kEdgeSectorWords);
     const uint32_t *order = vertex_order(e);
     const GraphView g = e->view();
     const uint32_t *t = e->tier;
@@ -530,7 +545,7 @@ EdgeSetView node2vec_edge_set(kk_engine *e)
         if (t[3] == 0)
             return;
         const uint32_t cap = 2u * (uint32_t)e->sm_count;
-        edge_set_block_kernel<<<t[3] < cap ? t[3] : cap, 1024, 0, st>>>(g, keys, order, 0, t[3]);
+        edge_set_block_kernel<<<t[3] < cap ? t[3] : cap, 1024, 0, st>>>(g, keys, order, 0, t[3], shift);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     };
@@ -539,7 +554,7 @@ EdgeSetView node2vec_edge_set(kk_engine *e)
             return;
         const size_t smem = (size_t)(128 / G) * row_words * sizeof(uint32_t);
         KK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid_for(e, hi - lo, 128 / G), 128, smem, st>>>(g, keys, order, lo, hi);
+        kern<<<grid_for(e, hi - lo, 128 / G), 128, smem, st>>>(g, keys, order, lo, hi, shift);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     };
@@ -547,7 +562,7 @@ EdgeSetView node2vec_edge_set(kk_engine *e)
     {
         /* a launch a class costs more than their lanes save */
         blocks();
-        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(weighted), t[3], e->n_nz);
+        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(shift), t[3], e->n_nz);
     }
     else
     {
@@ -558,11 +573,11 @@ EdgeSetView node2vec_edge_set(kk_engine *e)
         beside.fork();
         st = e->side;
         blocks();
-        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(weighted), t[3], t[4]);
+        group(edge_set_group_kernel<32, 1024>, 32, edge_set_group_words<1024>(shift), t[3], t[4]);
         st = e->stream;
-        group(edge_set_group_kernel<32, 512>, 32, edge_set_group_words<512>(weighted), t[4], t[5]);
-        group(edge_set_group_kernel<16, 128>, 16, edge_set_group_words<128>(weighted), t[5], t[6]);
-        group(edge_set_group_kernel<8, 32>, 8, edge_set_group_words<32>(weighted), t[6], e->n_nz);
+        group(edge_set_group_kernel<32, 512>, 32, edge_set_group_words<512>(shift), t[4], t[5]);
+        group(edge_set_group_kernel<16, 128>, 16, edge_set_group_words<128>(shift), t[5], t[6]);
+        group(edge_set_group_kernel<8, 32>, 8, edge_set_group_words<32>(shift), t[6], e->n_nz);
         beside.join();
     }
     e->edge_set_valid = true;

@@ -67,3 +67,30 @@ def test_node2vec_walks(engine, oracle_lib, p, q, length, kind, weighted, layout
         assert r.total_steps == steps
         np.testing.assert_array_equal(r.path_length, lens)
         np.testing.assert_array_equal(r.vertices, verts)
+
+
+@pytest.mark.parametrize("weighted", [True, False])
+@pytest.mark.parametrize("offsets32", [1, 0])
+def test_node2vec_batches(engine, oracle_lib, weighted, offsets32):
+    """Batches on both sides of the 3072 walkers an SM up to which the kernel has
+    two blocks an SM, and the kernel with the hooks (no 32-bit offsets)."""
+    csr = _graph("rows", weighted)
+    V = len(csr["off"]) - 1
+    engine.load_arrays(V, csr["off"], csr["nbr"], csr.get("w"))
+    ocsr = oracle_lib.CSR(V, csr["off"], csr["nbr"], csr.get("w")).sorted_copy()
+    engine.set_option("compact_offsets", offsets32)
+    try:
+        for sizes in ((33, 4000, 1), (500001, 5, 120000)):
+            jobs = [dict(walker_num=n, seed=9 + k, walker_begin=10 * k, walk_length=3 + 5 * k, p=(0.25, 2.0, 1.0)[k],
+                         q=(3.0, 0.5, 1.0)[k], weighted=weighted) for k, n in enumerate(sizes)]
+            got = engine.batch_walk("node2vec", jobs)
+            one = engine.walk("node2vec", sizes[2], **{k: v for k, v in jobs[2].items() if k != "walker_num"})
+            np.testing.assert_array_equal(got[2].vertices, one.vertices)
+            for job, paths in zip(jobs, got):
+                lens, verts, steps = oracle_lib.walk(ocsr, oracle_lib.make_params("node2vec", **job),
+                                                     cap=job["walk_length"] + 1)
+                assert paths.total_steps == steps
+                np.testing.assert_array_equal(paths.path_length, lens)
+                np.testing.assert_array_equal(paths.vertices, verts)
+    finally:
+        engine.set_option("compact_offsets", 1)
