@@ -111,9 +111,16 @@ uint32_t batch_wide_limit(const kk_engine *e)
 {
     return 3072u * (uint32_t)e->sm_count;
 }
-bool batch_wide(const kk_engine *e, const BatchPlan &plan)
+/* A serving slot shares the SMs with the other slots' batches, so that fewer
+ * walkers fill them (a burst of 16 requests, 108,000 walkers, on two slots: 1.61 ms
+ * with the line at 256 walkers an SM, 1.73 at 1024, 1.90 at none). */
+uint32_t slot_wide_limit(const kk_engine *e)
 {
-    return plan.app == KK_APP_NODE2VEC && plan.total <= batch_wide_limit(e);
+    return 256u * (uint32_t)e->sm_count;
+}
+bool batch_wide(const kk_engine *e, const BatchPlan &plan, bool slot)
+{
+    return plan.app == KK_APP_NODE2VEC && plan.total <= (slot ? slot_wide_limit(e) : batch_wide_limit(e));
 }
 
 /* Launches the batch on the slot, reading alias tables in the Bucket layout
@@ -153,7 +160,8 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
     unsigned long long *st = e->walk_stats ? steps + 1 : nullptr;
     if (e->walk_schedule == 0)
     {
-        unsigned grid = grid_for(e, hdr && batch_wide(e, plan) ? std::min(walkers, batch_wide_limit(e)) : walkers, bs);
+        const bool wide = batch_wide(e, plan, hdr != nullptr || slot.notify.count != nullptr);
+        unsigned grid = grid_for(e, hdr && wide ? std::min(walkers, slot_wide_limit(e)) : walkers, bs);
         if (hdr && grid > 64u * (unsigned)e->sm_count)
             grid = 64u * (unsigned)e->sm_count; /* grid-stride over whatever the header holds */
         bool launched = false;
@@ -166,7 +174,7 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
                     kern<<<grid, bs, 0, slot.stream>>>(gv, t, d_jobs, nj, plan.total, *path, length, steps, status,
                                                        e->trial_limit, st, hdr, slot.notify);
                 };
-                if (batch_wide(e, plan))
+                if (wide)
                     launch(n2v_batch_kernel<TC::has_static, Bucket, 2>);
                 else
                     launch(n2v_batch_kernel<TC::has_static, Bucket, 3>);
@@ -417,7 +425,7 @@ static void launch_batch_graph(kk_engine *e, BatchPlan &plan, BatchSlot &slot)
     h.hdr[0] = nj;
     h.hdr[1] = plan.total;
     /* one graph per kernel a batch's size may ask for */
-    cudaGraphExec_t &exec = slot.exec[batch_wide(e, plan) ? 1 : 0];
+    cudaGraphExec_t &exec = slot.exec[batch_wide(e, plan, true) ? 1 : 0];
     if (exec == nullptr)
     {
         cudaGraph_t graph = nullptr;
