@@ -391,7 +391,9 @@ def walk_kernel_name(app, best):
         return "walk_pool_kernel"
     if best.get("walk_multi", 1) > 1 and app in ("deepwalk", "ppr"):
         return "walk_multi_kernel<%d>" % best["walk_multi"]
-    return "walk_static_kernel"
+    if app == "node2vec":
+        return "n2v_walk_kernel"
+    return "walk_turns_kernel" if app == "metapath" else "walk_stream_kernel"
 
 
 def run_reference(args, wl, world, rank, local):
@@ -713,7 +715,7 @@ def run_serve_bench(args, wl, world, rank, local):
     achieved = steps_per_launch * b_step / (mean_launch_ms / 1e3) / 1e9
     kernel_rate = k_steps / (k_ms / 1e3)
     ceiling = engine.gather_ceiling(4 << 30)
-    traffic = traffic_for(args.workload, "walk_batch_kernel", steps_per_launch)
+    traffic = traffic_for(args.workload, "n2v_batch_kernel", steps_per_launch)
 
     parity = cpu = None
     if rank == 0:
@@ -785,7 +787,7 @@ def run_serve_bench(args, wl, world, rank, local):
                      "bytes_per_step": b_step, "design_bytes_per_step": design_b,
                      "access_counts": {"trials_per_step": T, "queries_per_step": Q, "probes_per_step": P,
                                        "return_edge_lookups_per_step": R},
-                     "kernel": "walk_batch_kernel (second order)", "kernel_ms": mean_launch_ms,
+                     "kernel": "n2v_batch_kernel (second order)", "kernel_ms": mean_launch_ms,
                      "launches": len(launch_steps), "steps_per_launch": steps_per_launch,
                      "gather": {"ceiling_reads_per_s": ceiling, "reads_per_step": T + Q + R,
                                 "achieved_reads_per_s": kernel_rate * (T + Q + R),
