@@ -47,15 +47,19 @@ struct N2vTables
 };
 
 /* Walks walker id from v to its end (the 32-bit offsets at hand), its path to
- * out (vertex 0 on; or nullptr); the path's length in len.  team: the warp's
- * lanes that call this together.  False when a step passed the trial limit. */
+ * out (vertex 0 on, with room for cap vertices; or nullptr); the path's length
+ * in len.  team: the warp's lanes that call this together.  Returns status
+ * flags: a step passed the trial limit, or the path's room.  The start's slot
+ * need not fit the walk (one vertex for a start outside the graph, whose walker
+ * stands on vertex 0 until the host refuses the call). */
 template <bool Weighted, bool Outlier, typename Bucket>
-__device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const N2vParams &P,
-                                         walker_id_t id, vertex_id_t v, uint32_t *out, uint32_t trial_limit,
-                                         unsigned long long *stats, unsigned team, Sampler &rng, uint32_t &len)
+__device__ __forceinline__ int n2v_walk(const GraphView &g, const N2vTables<Bucket> &t, const N2vParams &P,
+                                        walker_id_t id, vertex_id_t v, uint32_t *out, uint32_t cap,
+                                        uint32_t trial_limit, unsigned long long *stats, unsigned team, Sampler &rng,
+                                        uint32_t &len)
 {
     uint32_t step = 0, prev = 0, trials = 0;
-    bool within = true;
+    int status = KK_STATUS_OK;
     /* v's adjacency as read, its first edge and the one past its last: what
      * follows from them is computed where it is used, or the walk would wait
      * for them here */
@@ -278,7 +282,16 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
                 if (stats != nullptr)
                     atomicAdd(stats, 1ull);
                 if (++trials > trial_limit)
-                    alive = taken = within = false; /* this trial was one too many */
+                {
+                    /* this trial was one too many */
+                    alive = taken = false;
+                    status = KK_STATUS_TRIAL_LIMIT;
+                }
+            }
+            if (taken && path_full(out, step + 1, cap))
+            {
+                alive = taken = false;
+                status = KK_STATUS_PATH_CAPACITY;
             }
             if (taken)
             {
@@ -311,7 +324,7 @@ __device__ __forceinline__ bool n2v_walk(const GraphView &g, const N2vTables<Buc
         }
     }
     len = step + 1;
-    return within;
+    return status;
 }
 
 /* One thread per walker for its whole walk. */
@@ -329,9 +342,10 @@ __global__ void __launch_bounds__(256, 4) n2v_walk_kernel(GraphView g, N2vTables
         WalkerConfig<apps::Node2vecState> wc;
         walk_begin<apps::Node2vecState>(g, wc, L, i, run, rng);
         uint32_t len;
-        if (!n2v_walk<Weighted, Outlier, Bucket>(g, t, P, run.w.id, run.v, run.out, L.trial_limit, L.stats, team, rng,
-                                                 len))
-            atomicOr(L.status, KK_STATUS_TRIAL_LIMIT);
+        const int status = n2v_walk<Weighted, Outlier, Bucket>(g, t, P, run.w.id, run.v, run.out, run.cap,
+                                                               L.trial_limit, L.stats, team, rng, len);
+        if (status != KK_STATUS_OK)
+            atomicOr(L.status, status);
         L.length[i] = len;
         segment_done(L, i);
         my_steps = len - 1;
@@ -416,11 +430,11 @@ __global__ void __launch_bounds__(256, MinBlocks)
         uint32_t len;
         const N2vParams P{job->c[0], job->c[1], job->c[2], job->c[3], job->c[4], fminf(job->c[4], 1.0f),
                           job->walk_length};
-        const bool within =
-            n2v_walk<Weighted, true, Bucket>(g, t, P, id, v, out, trial_limit, stats, team, rng, len);
+        const int failed =
+            n2v_walk<Weighted, true, Bucket>(g, t, P, id, v, out, cap, trial_limit, stats, team, rng, len);
         const uint32_t j = (uint32_t)(job - jobs);
-        if (!within)
-            atomicOr(nt.count != nullptr ? nt.status + j : status, KK_STATUS_TRIAL_LIMIT);
+        if (failed != KK_STATUS_OK)
+            atomicOr(nt.count != nullptr ? nt.status + j : status, failed);
         length[job->first_task + i] = len;
         my_steps += len - 1;
         WalkLaunch L;

@@ -2050,6 +2050,14 @@ __global__ void regular_area_kernel(GraphView g, TC tc, const float *sum, float 
 #define KK_STATUS_PATH_CAPACITY 8
 #define KK_STATUS_BAD_START 16
 
+/* Whether a path of len vertices has no room for another: out holds cap of
+ * them (nullptr: no path is stored).  Every walk kernel asks before it takes an
+ * accepted step, and fails the call with KK_STATUS_PATH_CAPACITY. */
+__device__ __forceinline__ bool path_full(const uint32_t *out, uint32_t len, uint32_t cap)
+{
+    return out != nullptr && len >= cap;
+}
+
 struct WalkLaunch
 {
     uint64_t seed;
@@ -2376,15 +2384,13 @@ __device__ __forceinline__ bool straight_trial(const GraphView &g, const WC &wc,
     w.step++;
     if constexpr (is_hook<decltype(wc.walker_update_state)>())
         wc.walker_update_state(w, v, AdjUnit{ac.nbr, (edge_id_t)(pos.e0 + ac.idx)});
-    if (run.out)
+    if (path_full(run.out, run.len, run.cap))
     {
-        if (run.len >= run.cap)
-        {
-            atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
-            return false;
-        }
-        run.out[run.len] = ac.nbr;
+        atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
+        return false;
     }
+    if (run.out)
+        run.out[run.len] = ac.nbr;
     run.len++;
     run.pv = v;
     run.ppos = pos;
@@ -2595,15 +2601,13 @@ __device__ __forceinline__ bool rejection_trial(const GraphView &g, const WC &wc
     w.step++;
     if constexpr (is_hook<decltype(wc.walker_update_state)>())
         wc.walker_update_state(w, v, AdjUnit{ac.nbr, (edge_id_t)(e0 + ac.idx)});
-    if (run.out)
+    if (path_full(run.out, run.len, run.cap))
     {
-        if (run.len >= run.cap)
-        {
-            atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
-            return false;
-        }
-        run.out[run.len] = ac.nbr;
+        atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
+        return false;
     }
+    if (run.out)
+        run.out[run.len] = ac.nbr;
     run.len++;
     run.pv = v;
     run.ppos = pos;
@@ -2681,7 +2685,7 @@ __device__ __forceinline__ bool straight_step(const GraphView &g, const WC &wc, 
         if (!ends && ext < 1.0f)
             ends = map_gen_float(rng.primed_word(), 1.0f) > ext;
     }
-    const bool full = run.out != nullptr && run.len >= run.cap;
+    const bool full = path_full(run.out, run.len, run.cap);
     if (ends || full)
     {
         if (!ends)
@@ -3228,19 +3232,11 @@ __global__ void __launch_bounds__(256, 4) walk_multi_kernel(GraphView g, WC wc, 
             r.w.step++;
             if constexpr (is_hook<decltype(wc.walker_update_state)>())
                 wc.walker_update_state(r.w, v, AdjUnit{ac.nbr, (edge_id_t)(pos.e0 + ac.idx), ac.tag});
-            bool over = false;
-            if (r.out)
-            {
-                if (r.len >= r.cap)
-                {
-                    atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
-                    over = true;
-                }
-                else
-                {
-                    r.out[r.len] = ac.nbr;
-                }
-            }
+            const bool over = path_full(r.out, r.len, r.cap);
+            if (over)
+                atomicOr(L.status, KK_STATUS_PATH_CAPACITY);
+            else if (r.out)
+                r.out[r.len] = ac.nbr;
             if (over)
             {
                 L.length[idx[k]] = r.len;
