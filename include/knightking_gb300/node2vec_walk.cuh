@@ -165,7 +165,8 @@ __device__ __forceinline__ int n2v_walk(const GraphView &g, const N2vTables<Buck
             if (look && alive)
             {
                 const vertex_id_t x = asked ? cand : prev;
-                const uint32_t m = Weighted ? edge_set_match(k0, x) : edge_set_match(k0, k1, x);
+                /* a weighted walk's set is weighted; an unweighted walk's may be too */
+                const uint32_t m = Weighted ? edge_set_match(k0, x) : edge_set_match(t.set, k0, k1, x);
                 if (m == 9)
                 {
                     /* undecided: the next sector, next time */

@@ -169,6 +169,13 @@ __device__ __forceinline__ uint32_t edge_set_match(const uint4 &a, const uint4 &
     const uint32_t m = edge_set_match(b, v), l = edge_set_match(a, v);
     return l < 4 ? l : m < 4 ? m + 4 : m;
 }
+/* The sector's halves x and y as the set holds them: y is four more ids, or the
+ * weights of x's.  That is the graph's choice, whatever the walk's weighting. */
+__device__ __forceinline__ uint32_t edge_set_match(const EdgeSetView &s, const uint4 &x, const uint4 &y,
+                                                   vertex_id_t v)
+{
+    return s.weighted ? edge_set_match(x, v) : edge_set_match(x, y, v);
+}
 __device__ __forceinline__ uint32_t word_of(const uint4 &a, uint32_t j)
 {
     const uint32_t lo = j & 1 ? a.y : a.x, hi = j & 1 ? a.w : a.z;
@@ -187,7 +194,7 @@ __device__ __forceinline__ bool edge_set_find(const EdgeSetView &s, vertex_id_t 
     {
         const uint4 *p = reinterpret_cast<const uint4 *>(s.keys + (row + b) * kEdgeSectorWords);
         const uint4 x = __ldg(p), y = __ldg(p + 1);
-        const uint32_t m = s.weighted ? edge_set_match(x, v) : edge_set_match(x, y, v);
+        const uint32_t m = edge_set_match(s, x, y, v);
         if (m < 8)
         {
             if (weight != nullptr)
