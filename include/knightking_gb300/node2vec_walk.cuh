@@ -100,9 +100,10 @@ __device__ __forceinline__ int n2v_walk(const GraphView &g, const N2vTables<Buck
         }
     };
     begin_step();
+    const step_t last = path_steps(out, cap, P.walk_length);
     /* one way through the loop, and the warp's lanes (team) meet at its top:
      * they share the instructions of every pass */
-    bool alive = P.walk_length > 0;
+    bool alive = last > 0;
     while (__any_sync(team, alive))
     {
         if (alive)
@@ -289,11 +290,6 @@ __device__ __forceinline__ int n2v_walk(const GraphView &g, const N2vTables<Buck
                     status = KK_STATUS_TRIAL_LIMIT;
                 }
             }
-            if (taken && path_full(out, step + 1, cap))
-            {
-                alive = taken = false;
-                status = KK_STATUS_PATH_CAPACITY;
-            }
             if (taken)
             {
                 step++;
@@ -320,11 +316,13 @@ __device__ __forceinline__ int n2v_walk(const GraphView &g, const N2vTables<Buck
                     pe = gather(g.off32 + v + 1);
                 }
                 begin_step();
-                alive = step < P.walk_length;
+                alive = step < last;
             }
         }
     }
     len = step + 1;
+    if (step == last && last < P.walk_length && pe != pb && status == KK_STATUS_OK)
+        status = KK_STATUS_PATH_CAPACITY; /* another step was due */
     return status;
 }
 

@@ -2059,10 +2059,15 @@ __global__ void regular_area_kernel(GraphView g, TC tc, const float *sum, float 
 
 /* Whether a path of len vertices has no room for another: out holds cap of
  * them (nullptr: no path is stored).  Every walk kernel asks before it takes an
- * accepted step, and fails the call with KK_STATUS_PATH_CAPACITY. */
+ * accepted step, and fails the call with KK_STATUS_PATH_CAPACITY; one whose
+ * walks have a length of their own asks once, for the steps that fit. */
 __device__ __forceinline__ bool path_full(const uint32_t *out, uint32_t len, uint32_t cap)
 {
     return out != nullptr && len >= cap;
+}
+__device__ __forceinline__ step_t path_steps(const uint32_t *out, uint32_t cap, step_t walk_length)
+{
+    return path_full(out, walk_length, cap) ? cap - 1 : walk_length;
 }
 
 struct WalkLaunch
