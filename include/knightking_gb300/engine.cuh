@@ -991,14 +991,15 @@ void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &t
 }
 
 /* Node2vec walks: over the edge set, or with the hooks where the engine asks
- * the sorted adjacency (node2vec_adjacency 1) or has no 32-bit offsets. */
+ * the sorted adjacency (node2vec_adjacency 1) or has no 32-bit offsets, or the
+ * hooks hold arrays or bounds of the caller's. */
 template <typename S, typename WC, typename TC, typename Bucket>
 void launch_node2vec(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
                      const float *ra, const WalkLaunch &L)
 {
     const uint32_t n = L.walker_num;
     const unsigned bs = (unsigned)e->walk_block;
-    if (tc.respond_query.set.keys == nullptr || g.off32 == nullptr)
+    if (!n2v_reads_graph(g, tc))
     {
         walk_static_kernel<S, WC, TC, Bucket><<<grid_for(e, n, bs), bs, 0, e->stream>>>(g, wc, tc, alias, ra, L);
         return;
@@ -1193,7 +1194,7 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
         {
             launch_straight<S, WC, TC, Bucket>(e, g, wc, tc, alias, L, !rs.fixed_cap, (uint32_t *)d_status + 14);
         }
-        else if constexpr (is_node2vec<TC>::value)
+        else if constexpr (is_node2vec<WC, TC>())
         {
             launch_node2vec<S, WC, TC, Bucket>(e, g, wc, tc, alias, ra, L);
         }

@@ -352,17 +352,45 @@ __global__ void __launch_bounds__(256, 4) n2v_walk_kernel(GraphView g, N2vTables
     flush_steps(L.total_steps, my_steps);
 }
 
-/* Whether a transition is node2vec's, with its outlier or without. */
-template <typename TC, typename = void>
-struct is_node2vec
+/* Whether a walk's hooks are node2vec's own, every one of them (apps.cuh),
+ * weighted or not, with its outlier or without: the kernels here restate them,
+ * so a walk with another hook among them, or another walker config, is the
+ * general kernels'. */
+template <typename WC, typename TC>
+constexpr bool is_node2vec()
 {
-    static constexpr bool value = false;
-};
+    if constexpr (TC::order == 2)
+    {
+        using namespace apps;
+        constexpr bool weighted = TC::has_static, outlier = TC::has_outlier;
+        typedef SecondOrderTransitionConfig<
+            Node2vecState, vertex_id_t, bool, FixedLengthExt<Node2vecState>,
+            typename std::conditional<weighted, WeightStatic, NoHook>::type, Node2vecPostQuery, Node2vecRespond,
+            Node2vecDyn, ConstBound, ConstBound,
+            typename std::conditional<outlier, Node2vecOutlierUB<weighted>, NoHook>::type,
+            typename std::conditional<outlier, Node2vecOutlierSearch, NoHook>::type>
+            Plain;
+        return std::is_same<TC, Plain>::value &&
+               std::is_same<WC, WalkerConfig<Node2vecState, NoHook, NoHook, Node2vecUpdate>>::value;
+    }
+    return false;
+}
+
+/* Whether the hooks read what the kernels here do: the graph's arrays, the
+ * edge set and the 32-bit offsets, and at step 0 the bound that is the dart's. */
 template <typename TC>
-struct is_node2vec<TC, std::enable_if_t<std::is_same<decltype(TC::dynamic_comp), apps::Node2vecDyn>::value>>
+bool n2v_reads_graph(const GraphView &g, const TC &tc)
 {
-    static constexpr bool value = true;
-};
+    bool same = tc.respond_query.set.keys != nullptr && g.off32 != nullptr && tc.respond_query.nbr == g.nbr &&
+                tc.dynamic_comp.upperbound == tc.dcomp_upperbound.value;
+    if constexpr (TC::has_static)
+        same = same && tc.static_comp.w == g.w;
+    if constexpr (TC::has_outlier)
+        same = same && tc.outlier_upperbound.set.keys == tc.respond_query.set.keys &&
+               tc.outlier_search.nbr == g.nbr &&
+               (!TC::has_static || (tc.outlier_upperbound.w == g.w && tc.outlier_upperbound.nbr == g.nbr));
+    return same;
+}
 
 template <typename TC>
 N2vParams n2v_params(const TC &tc)

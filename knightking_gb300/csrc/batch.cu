@@ -165,7 +165,7 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
         if (hdr && grid > 64u * (unsigned)e->sm_count)
             grid = 64u * (unsigned)e->sm_count; /* grid-stride over whatever the header holds */
         bool launched = false;
-        if constexpr (is_node2vec<TC>::value)
+        if constexpr (is_node2vec<typename App::WC, TC>())
         {
             if (app.set.keys != nullptr && gv.off32 != nullptr)
             {
