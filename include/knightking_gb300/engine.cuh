@@ -992,7 +992,8 @@ void launch_straight(kk_engine *e, const GraphView &g, const WC &wc, const TC &t
 
 /* Node2vec walks: over the edge set, or with the hooks where the engine asks
  * the sorted adjacency (node2vec_adjacency 1) or has no 32-bit offsets, or the
- * hooks hold arrays or bounds of the caller's. */
+ * set has too many sectors for the kernel, or the hooks hold arrays or bounds of
+ * the caller's. */
 template <typename S, typename WC, typename TC, typename Bucket>
 void launch_node2vec(kk_engine *e, const GraphView &g, const WC &wc, const TC &tc, const Bucket *alias,
                      const float *ra, const WalkLaunch &L)

@@ -376,12 +376,19 @@ constexpr bool is_node2vec()
     return false;
 }
 
+/* Whether the kernels here can walk g over the set: they find positions in the
+ * 32-bit offsets and count sectors in 32 bits. */
+inline bool n2v_over_edge_set(const GraphView &g, const EdgeSetView &set)
+{
+    return set.keys != nullptr && g.off32 != nullptr && edge_set_in_32_bits(g.E, g.V, set.shift);
+}
+
 /* Whether the hooks read what the kernels here do: the graph's arrays, the
  * edge set and the 32-bit offsets, and at step 0 the bound that is the dart's. */
 template <typename TC>
 bool n2v_reads_graph(const GraphView &g, const TC &tc)
 {
-    bool same = tc.respond_query.set.keys != nullptr && g.off32 != nullptr && tc.respond_query.nbr == g.nbr &&
+    bool same = n2v_over_edge_set(g, tc.respond_query.set) && tc.respond_query.nbr == g.nbr &&
                 tc.dynamic_comp.upperbound == tc.dcomp_upperbound.value;
     if constexpr (TC::has_static)
         same = same && tc.static_comp.w == g.w;

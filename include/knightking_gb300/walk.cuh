@@ -145,6 +145,11 @@ __host__ __device__ __forceinline__ uint64_t edge_set_total(uint64_t E, uint32_t
 {
     return (E >> shift) + V + 1;
 }
+/* whether a walk may count them in 32 bits */
+__host__ __device__ __forceinline__ bool edge_set_in_32_bits(uint64_t E, uint32_t V, uint32_t shift)
+{
+    return edge_set_total(E, V, shift) <= 1ull << 32;
+}
 /* where v's probe starts among a row's n sectors */
 __host__ __device__ __forceinline__ uint32_t edge_set_sector(vertex_id_t v, uint32_t n)
 {

@@ -167,7 +167,7 @@ void launch_batch_with(kk_engine *e, const App &app, const BatchPlan &plan, Batc
         bool launched = false;
         if constexpr (is_node2vec<typename App::WC, TC>())
         {
-            if (app.set.keys != nullptr && gv.off32 != nullptr)
+            if (n2v_over_edge_set(gv, app.set))
             {
                 const N2vTables<Bucket> t{alias, (const float *)e->sum.p, nullptr, app.set};
                 auto launch = [&](auto kern) {

@@ -519,7 +519,7 @@ static uint32_t edge_set_shift(const kk_engine *e)
 {
     if (e->d_w == nullptr)
         return 2;
-    return e->E >= 28000000 && e->E + e->V + 1 < (1ull << 32) ? 0 : 1; /* the walk counts sectors in 32 bits */
+    return e->E >= 28000000 && edge_set_in_32_bits(e->E, e->V, 0) ? 0 : 1;
 }
 
 EdgeSetView node2vec_edge_set_built(const kk_engine *e)
