@@ -500,6 +500,7 @@ class Server:
     def __init__(self, engine, app, weighted=None, slots=2, max_jobs=256, slot_bytes=1 << 30, graphs=True):
         self._engine = engine
         self._lib = engine._lib
+        self._kept = set()  # the small results that hold their blocks
         self.app = app
         if weighted is None:
             weighted = engine.info()[2]
@@ -528,7 +529,14 @@ class Server:
     def poll(self, ticket, timeout_ms=-1, keep_paths=True):
         """The request's ServeResult, or None if it is not done within
         timeout_ms.  keep_paths=False frees the paths unread (result.paths is
-        then None and result.total_steps still counts them)."""
+        then None and result.total_steps still counts them).
+
+        The paths are views of the request's own block of pinned host memory
+        (64 KiB or a larger power of two), which goes back to the server when
+        the last array viewing it is gone: copy what is kept for long.  Copying
+        every result out of its block took two thirds of a burst (16 requests,
+        42 MB of paths: 4.3 ms, 1.6 without).  Of results below 256 KiB, at most
+        256 hold their blocks at a time; further ones are copies."""
         r = _capi.KKServeResult()
         st = self._lib.kk_serve_poll(self._h, ctypes.c_uint64(ticket), int(timeout_ms), ctypes.byref(r))
         if st == _capi.KK_ERR_TIMEOUT:
@@ -540,9 +548,7 @@ class Server:
         if r.paths:
             total_steps = r.paths.contents.total_steps
             if keep_paths:
-                # views of the request's own pinned block, as batch_walk's are: copying them out of it took
-                # two thirds of a burst (16 requests, 42 MB of paths: 4.3 ms, 1.6 without)
-                paths = PathSet(*_capi.paths_to_numpy_owned(r.paths))
+                paths = PathSet(*_capi.paths_to_numpy_served(r.paths, self._kept))
             else:
                 self._lib.kk_paths_free(r.paths)
         res = ServeResult(paths, r.status, r.queue_ms, r.latency_ms, r.batch_jobs)
