@@ -41,6 +41,35 @@ namespace kk
 /* Memory a load leaves for the next one: up to this much is kept. */
 constexpr size_t kKeepBytes = (size_t)1 << 30;
 
+/* A load or a sort in gnext's arrays: whatever its end, of what stands there
+ * afterwards (nothing of use: the graph before, or a refused one) no more than
+ * that is left. */
+struct NextArrays
+{
+    kk_engine *e;
+    ~NextArrays()
+    {
+        if (e->gnext.bytes() > kKeepBytes)
+            e->gnext.release();
+    }
+};
+
+/* A load's temporaries in the memory of the walks' alias tables and queues: of
+ * a weighted graph loaded (keep), they are the next walk's; a refused load, or
+ * an unweighted graph's, whose walks use neither, gives large ones back. */
+struct LoadTemps
+{
+    kk_engine *e;
+    bool keep = false;
+    ~LoadTemps()
+    {
+        if (keep || e->alias.bytes + e->scratch.bytes <= kKeepBytes)
+            return;
+        e->alias.release();
+        e->scratch.release();
+    }
+};
+
 /* Between fork() and join(), what is launched on the side stream runs beside
  * the engine's; a call that fails in between waits for it. */
 struct SideWork
@@ -647,8 +676,6 @@ void graph_commit(kk_engine *e, uint32_t V, uint64_t E, bool w, bool type, int s
     e->E = E;
     graph_offsets32(e);
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    if (e->gnext.bytes() > kKeepBytes)
-        e->gnext.release();
     e->has_graph = true;
     e->sorted = sorted;
 }
@@ -673,6 +700,7 @@ void graph_sort_adjacency(kk_engine *e)
     vertex_order(e);
     const RowDesc *rows = (const RowDesc *)e->rows.p;
     const uint32_t *t = e->tier;
+    NextArrays next{e};
     next_arrays(e, e->V, E, false, e->d_w != nullptr, e->d_type != nullptr, false);
     uint32_t *nbr_out = (uint32_t *)e->gnext.nbr.p;
     float *w_out = (float *)e->gnext.w.p;
@@ -756,8 +784,6 @@ void graph_sort_adjacency(kk_engine *e)
         std::swap(e->gb.type, e->gnext.type);
         e->d_type = (uint8_t *)e->gb.type.p;
     }
-    if (e->gnext.bytes() > kKeepBytes)
-        e->gnext.release();
     e->sorted = 1;
 }
 
@@ -787,6 +813,7 @@ void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off,
         fail(KK_ERR_INVALID_CONFIG, "graph needs V > 0, off and nbr");
     if (off[0] != 0 || (uint64_t)off[V] != E)
         fail(KK_ERR_INVALID_CONFIG, "off[0] must be 0 and off[V] must be E");
+    NextArrays next{e};
     bool checked = false;
     try
     {
@@ -932,16 +959,6 @@ __global__ void csr_from_sorted_kernel(const uint32_t *key, const uint64_t *val,
 
 } // namespace
 
-/* After a load: an unweighted graph's walks use neither of the buffers the
- * load's temporaries stood in; large ones are given back. */
-static void load_temps_done(kk_engine *e, bool weighted)
-{
-    if (weighted || e->alias.bytes + e->scratch.bytes <= kKeepBytes)
-        return;
-    e->alias.release();
-    e->scratch.release();
-}
-
 /* CSR in HBM from the raw records of an untyped binary edge file (8-byte
  * src/dst or 12-byte src/dst/weight, include/storage.hpp:35-55), which
  * fill(d) puts into device memory at d as they are; they are split (and mirrored,
@@ -958,6 +975,8 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
     const bool weighted = rec == 12;
     /* the records and the sort's keys and values stand where the walks' alias
      * tables and queues will: both are rebuilt for the new graph */
+    NextArrays next{e};
+    LoadTemps temps{e};
     e->alias_cached = -1;
     const uint64_t m1 = (m + 64) & ~(uint64_t)63; /* every array aligned */
     uint64_t *d_val = e->scratch.as<uint64_t>(2 * m1), *d_val2 = d_val + m1;
@@ -992,7 +1011,7 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
     graph_commit(e, V, m, weighted, false, -1);
-    load_temps_done(e, weighted);
+    temps.keep = weighted;
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
@@ -1005,6 +1024,8 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
     if (m >= 0xffffffffull)
         fail(KK_ERR_INVALID_CONFIG, "edge lists are limited to 2^32 - 1 edges");
     const auto t0 = std::chrono::steady_clock::now();
+    NextArrays next{e};
+    LoadTemps temps{e};
     e->alias_cached = -1; /* the sort's arrays stand in the tables' memory */
     const uint64_t m1 = (m + 64) & ~(uint64_t)63; /* every array aligned */
     uint32_t *d_src = e->alias.as<uint32_t>(4 * m1), *d_src2 = d_src + m1, *d_idx = d_src2 + m1, *d_perm = d_idx + m1;
@@ -1048,7 +1069,7 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
         KK_CUDA_CHECK(cudaGetLastError());
     }
     graph_commit(e, V, m, h_w != nullptr, h_t != nullptr, -1);
-    load_temps_done(e, h_w != nullptr);
+    temps.keep = h_w != nullptr;
     e->load_device_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
@@ -1484,6 +1505,7 @@ void graph_generate_rmat(kk_engine *e, uint32_t scale, uint32_t ef, double a, do
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, bytes, mir, mir_sorted, E, 0, 64, e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(e->cub_tmp.ensure(bytes), bytes, mir, mir_sorted, E, 0, 64, e->stream));
     cudaFree(mir);
+    NextArrays next{e};
     next_arrays(e, V, E, true, weights != 0, types != 0, true);
     GraphBufs &nx = e->gnext;
     unsigned int *deg = nullptr;
