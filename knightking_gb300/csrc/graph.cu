@@ -432,7 +432,32 @@ void graph_offsets32(kk_engine *e)
 {
     if (e->E > 0xffffffffull)
         return;
-    uint32_t *o = e->off32.as<uint32_t>((uint64_t)e->V + 1);
+    uint32_t *o = nullptr;
+    try
+    {
+        o = e->off32.as<uint32_t>((uint64_t)e->V + 1);
+    }
+    catch (const Error &x)
+    {
+        if (x.status != KK_ERR_OOM)
+            throw;
+        /* in the place of the graph before; without them the walks read the
+         * 64-bit ones */
+        cudaGetLastError();
+        KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
+        e->gnext.release();
+        try
+        {
+            o = e->off32.as<uint32_t>((uint64_t)e->V + 1);
+        }
+        catch (const Error &y)
+        {
+            if (y.status != KK_ERR_OOM)
+                throw;
+            cudaGetLastError();
+            return;
+        }
+    }
     offsets32_kernel<<<grid_for(e, (uint64_t)e->V + 1, 256), 256, 0, e->stream>>>(e->d_off, e->V, o);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
@@ -633,27 +658,18 @@ void graph_check_sorted(kk_engine *e)
     e->sorted = words[kScanDescents] == words[kScanBetween];
 }
 
-/* Room for a graph in gnext's arrays.  When the device is full, the graph the
- * engine holds goes first (drop: the caller has checked the new one, which
- * will replace it). */
-static void next_arrays(kk_engine *e, uint32_t V, uint64_t E, bool off, bool w, bool type, bool drop)
+/* What make() allocates for a checked graph.  When the device is full, the graph
+ * the engine holds, which the new one will replace, goes first. */
+template <typename F>
+static void in_place_of_graph(kk_engine *e, F make)
 {
-    auto make = [&]() {
-        if (off)
-            e->gnext.off.as<int64_t>((uint64_t)V + 1);
-        e->gnext.nbr.as<uint32_t>(E + 1);
-        if (w)
-            e->gnext.w.as<float>(E + 1);
-        if (type)
-            e->gnext.type.as<uint8_t>(E + 4);
-    };
     try
     {
         make();
     }
     catch (const Error &x)
     {
-        if (x.status != KK_ERR_OOM || !drop)
+        if (x.status != KK_ERR_OOM)
             throw;
         cudaGetLastError();
         e->gnext.release();
@@ -662,6 +678,18 @@ static void next_arrays(kk_engine *e, uint32_t V, uint64_t E, bool off, bool w, 
         e->gb.release();
         make();
     }
+}
+
+/* Room for a graph in gnext's arrays. */
+static void next_arrays(kk_engine *e, uint32_t V, uint64_t E, bool off, bool w, bool type)
+{
+    if (off)
+        e->gnext.off.as<int64_t>((uint64_t)V + 1);
+    e->gnext.nbr.as<uint32_t>(E + 1);
+    if (w)
+        e->gnext.w.as<float>(E + 1);
+    if (type)
+        e->gnext.type.as<uint8_t>(E + 4);
 }
 
 void graph_commit(kk_engine *e, uint32_t V, uint64_t E, bool w, bool type, int sorted)
@@ -701,7 +729,7 @@ void graph_sort_adjacency(kk_engine *e)
     const RowDesc *rows = (const RowDesc *)e->rows.p;
     const uint32_t *t = e->tier;
     NextArrays next{e};
-    next_arrays(e, e->V, E, false, e->d_w != nullptr, e->d_type != nullptr, false);
+    next_arrays(e, e->V, E, false, e->d_w != nullptr, e->d_type != nullptr);
     uint32_t *nbr_out = (uint32_t *)e->gnext.nbr.p;
     float *w_out = (float *)e->gnext.w.p;
     uint8_t *type_out = (uint8_t *)e->gnext.type.p;
@@ -817,7 +845,7 @@ void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off,
     bool checked = false;
     try
     {
-        next_arrays(e, V, E, true, w != nullptr, type != nullptr, false);
+        next_arrays(e, V, E, true, w != nullptr, type != nullptr);
     }
     catch (const Error &x)
     {
@@ -826,7 +854,7 @@ void graph_load_arrays(kk_engine *e, uint32_t V, uint64_t E, const int64_t *off,
         cudaGetLastError();
         check_arrays(V, E, off, nbr, type);
         checked = true;
-        next_arrays(e, V, E, true, w != nullptr, type != nullptr, true);
+        in_place_of_graph(e, [&]() { next_arrays(e, V, E, true, w != nullptr, type != nullptr); });
     }
     GraphBufs &n = e->gnext;
     KK_CUDA_CHECK(cudaMemcpyAsync(n.off.p, off, ((size_t)V + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, e->stream));
@@ -996,13 +1024,16 @@ void csr_from_records(kk_engine *e, uint32_t V, uint64_t n, size_t rec, bool und
     KK_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     if (((volatile uint32_t *)e->h_status)[41] != 0)
         fail(KK_ERR_INVALID_CONFIG, "edge endpoint >= v_num"); /* the engine keeps its graph */
-    next_arrays(e, V, m, true, weighted, false, true);
     int bits = 1;
     while (bits < 32 && ((uint64_t)1 << bits) < V)
         bits++;
     size_t bytes = 0;
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, d_key, d_key2, d_val, d_val2, (int64_t)m, 0, bits,
                                                   e->stream));
+    in_place_of_graph(e, [&]() {
+        next_arrays(e, V, m, true, weighted, false);
+        e->cub_tmp.ensure(bytes);
+    });
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(e->cub_tmp.ensure(bytes), bytes, d_key, d_key2, d_val, d_val2,
                                                   (int64_t)m, 0, bits, e->stream));
     csr_from_sorted_kernel<<<grid_for(e, m / 4 + 1, 256), 256, 0, e->stream>>>(
@@ -1028,20 +1059,26 @@ void csr_from_edges(kk_engine *e, uint32_t V, uint64_t m, const uint32_t *h_src,
     LoadTemps temps{e};
     e->alias_cached = -1; /* the sort's arrays stand in the tables' memory */
     const uint64_t m1 = (m + 64) & ~(uint64_t)63; /* every array aligned */
-    uint32_t *d_src = e->alias.as<uint32_t>(4 * m1), *d_src2 = d_src + m1, *d_idx = d_src2 + m1, *d_perm = d_idx + m1;
-    uint32_t *d_in = e->scratch.as<uint32_t>(m1);
-    next_arrays(e, V, m, true, h_w != nullptr, h_t != nullptr, true);
+    int bits = 1;
+    while (bits < 32 && ((uint64_t)1 << bits) < V)
+        bits++;
+    size_t bytes = 0;
+    KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, (uint32_t *)nullptr, (uint32_t *)nullptr,
+                                                  (uint32_t *)nullptr, (uint32_t *)nullptr, (int64_t)m, 0, bits,
+                                                  e->stream));
+    uint32_t *d_src = nullptr, *d_in = nullptr;
+    in_place_of_graph(e, [&]() {
+        d_src = e->alias.as<uint32_t>(4 * m1);
+        d_in = e->scratch.as<uint32_t>(m1);
+        next_arrays(e, V, m, true, h_w != nullptr, h_t != nullptr);
+        e->cub_tmp.ensure(bytes);
+    });
+    uint32_t *d_src2 = d_src + m1, *d_idx = d_src2 + m1, *d_perm = d_idx + m1;
     GraphBufs &nx = e->gnext;
     KK_CUDA_CHECK(cudaMemcpyAsync(d_src, h_src, m * 4, cudaMemcpyHostToDevice, e->stream));
     iota_u32_kernel<<<grid_for(e, m, 256), 256, 0, e->stream>>>(d_idx, m);
     count_launch(e);
     KK_CUDA_CHECK(cudaGetLastError());
-    int bits = 1;
-    while (bits < 32 && ((uint64_t)1 << bits) < V)
-        bits++;
-    size_t bytes = 0;
-    KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, d_src, d_src2, d_idx, d_perm, (int64_t)m, 0, bits,
-                                                  e->stream));
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(e->cub_tmp.ensure(bytes), bytes, d_src, d_src2, d_idx, d_perm,
                                                   (int64_t)m, 0, bits, e->stream));
     offsets_from_sorted_kernel<<<grid_for(e, m + 1, 256), 256, 0, e->stream>>>(d_src2, m, V, (int64_t *)nx.off.p);
@@ -1506,7 +1543,7 @@ void graph_generate_rmat(kk_engine *e, uint32_t scale, uint32_t ef, double a, do
     KK_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(e->cub_tmp.ensure(bytes), bytes, mir, mir_sorted, E, 0, 64, e->stream));
     cudaFree(mir);
     NextArrays next{e};
-    next_arrays(e, V, E, true, weights != 0, types != 0, true);
+    in_place_of_graph(e, [&]() { next_arrays(e, V, E, true, weights != 0, types != 0); });
     GraphBufs &nx = e->gnext;
     unsigned int *deg = nullptr;
     uint64_t *deg64 = nullptr;
