@@ -118,12 +118,15 @@ kk_status kk_engine_set_stream(kk_engine *e, void *stream);
  *   "walk_park"          first-order walks with a dynamic component (rejection trials): 1..32 (default
  *                        20; all alike) more walkers than the GPU holds at once take turns on the
  *                        resident threads, 0 one walker per thread
- *   "alias_hub_grid"     blocks of the hub alias kernel (0: one per two SMs)
- *   "alias_streams"      1 the alias classes of degree <= 16384 in turn on the engine's stream,
+ *   "alias_one_launch"   1 (default): the rows of degree <= 16384 in one launch beside the hubs' on
+ *                        graphs of up to 40 M edges with few rows of degree above 1024; 0 a launch
+ *                        a degree class whatever the size
+ *   "alias_hub_grid"     blocks of the hub alias kernel, degree > 16384 (0: one per two SMs)
+ *   "alias_streams"      (a launch a class) 1 the alias classes of degree <= 16384 in turn on the engine's stream,
  *                        2 those of degree <= 128 after the hubs on a second stream, beside the rest,
  *                        3 (default) also those of degree 1025..16384 on a third, 4 those of degree
  *                        <= 512 on the second stream from the start and the hubs alone on a third
- *   "alias_small_lanes"  0 (default) lane groups of 4 and 2 per row for the alias rows of degree
+ *   "alias_small_lanes"  (a launch a class) 0 (default) lane groups of 4 and 2 per row for the alias rows of degree
  *                        17..32 and 1..16; 1 groups of 2 and 1
  *   "into_stream"        1 (default): kk_walk_into walks whose path lengths are known before they
  *                        run (DeepWalk, PPR, node2vec on graphs without reachable dead ends) in one

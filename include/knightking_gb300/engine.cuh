@@ -690,6 +690,14 @@ void launch_alias_class(kk_engine *e, K kern, unsigned nt, size_t smem, uint32_t
     KK_CUDA_CHECK(cudaGetLastError());
 }
 
+/* Blocks for n hub rows: the alias_hub_grid option's, or one per two SMs. */
+inline uint32_t alias_hub_blocks(const kk_engine *e, uint32_t n)
+{
+    const uint32_t cap =
+        e->alias_hub_grid > 0 ? (uint32_t)e->alias_hub_grid : (uint32_t)(e->sm_count > 1 ? e->sm_count / 2 : 1);
+    return n < cap ? n : cap;
+}
+
 /* The build in one launch beside the hubs', for graphs of up to
  * kAliasSmallEdges edges whose rows of 1025 to 16384 edges are at most four a
  * resident block (a block of 256 threads takes each; more of them, and the
@@ -738,8 +746,7 @@ bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *a
          * rows, wait for one to leave (R-MAT 18: 192 us, or 315 when they did) */
         small = e->side;
         KK_CUDA_CHECK(cudaEventRecord(e->ev_fork, e->stream));
-        const uint32_t cap = (uint32_t)(e->sm_count > 1 ? e->sm_count / 2 : 1);
-        alias_build_hub_kernel<TC, Bucket><<<a.first < cap ? a.first : cap, 1024, 0, e->stream>>>(
+        alias_build_hub_kernel<TC, Bucket><<<alias_hub_blocks(e, a.first), 1024, 0, e->stream>>>(
             g, tc, alias, vcur, sum, scratch, (const uint32_t *)e->order.p, 0, a.first, next + 2);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
@@ -804,11 +811,8 @@ void build_alias(kk_engine *e, const TC &tc)
         KK_CUDA_CHECK(cudaStreamWaitEvent(hub_st, e->ev_fork, 0));
         /* half the SMs by default: the hubs' serial sums and short batches use
          * few lanes, and the classes on the main stream get the other half */
-        const uint32_t cap =
-            e->alias_hub_grid > 0 ? (uint32_t)e->alias_hub_grid : (uint32_t)(e->sm_count > 1 ? e->sm_count / 2 : 1);
-        const unsigned grid = e->n_hub < cap ? e->n_hub : cap;
-        alias_build_hub_kernel<TC, Bucket><<<grid, 1024, 0, hub_st>>>(g, tc, alias, vcur, sum, scratch, order, 0,
-                                                                      e->n_hub, next);
+        alias_build_hub_kernel<TC, Bucket><<<alias_hub_blocks(e, e->n_hub), 1024, 0, hub_st>>>(
+            g, tc, alias, vcur, sum, scratch, order, 0, e->n_hub, next);
         count_launch(e);
         KK_CUDA_CHECK(cudaGetLastError());
     }
