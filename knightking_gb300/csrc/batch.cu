@@ -112,11 +112,15 @@ uint32_t batch_wide_limit(const kk_engine *e)
     return 3072u * (uint32_t)e->sm_count;
 }
 /* A serving slot shares the SMs with the other slots' batches, so that fewer
- * walkers fill them (a burst of 16 requests, 108,000 walkers, on two slots: 1.61 ms
- * with the line at 256 walkers an SM, 1.73 at 1024, 1.90 at none). */
+ * walkers fill them.  Bursts on 1 M vertices, 32 M edges, ms with the line at 256 /
+ * 1024 / 3072 walkers an SM: 16 requests, 113,000 walkers, on one slot 2.17 / 1.98 /
+ * 1.98, on two 2.02 / 1.89 / 1.90, on four 1.78 / 1.61 / 1.66; 218,000 walkers 2.76 /
+ * 2.63 / 2.92, 2.55 / 2.57 / 2.48, 2.47 / 2.29 / 2.27; 48 requests, 302,000 walkers
+ * 3.51 / 3.50 / 3.65, 3.22 / 3.21 / 3.14, 2.85 / 2.80 / 2.96; below 40,000 walkers
+ * the three are within 5%, as is no such kernel for slots. */
 uint32_t slot_wide_limit(const kk_engine *e)
 {
-    return 256u * (uint32_t)e->sm_count;
+    return 1024u * (uint32_t)e->sm_count;
 }
 bool batch_wide(const kk_engine *e, const BatchPlan &plan, bool slot)
 {
