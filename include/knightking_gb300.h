@@ -139,8 +139,11 @@ kk_status kk_engine_set_stream(kk_engine *e, void *stream);
  *                        paths out while the next chunk walks (default 6; 1 = whole)
  *   "cursor_adjacency"   1 uniform picks read a per-graph adjacency copy holding each neighbour's
  *                        position (16 B/edge, built on first use): one dependent read per step
+ *   "compact_offsets"    1 (default): walks read 32-bit copies of the offsets (graphs of fewer than
+ *                        2^32 edges), and node2vec the edge set in the kernel laid out for it; 0 the
+ *                        64-bit offsets, and node2vec in the general kernels
  *   "regroup_interval"   0 (default) off; k > 0: single-job walks of the one-walker-per-thread schedule
- *                        that do not park run in phases of k steps, and each phase takes its walkers
+ *                        that do not take turns run in phases of k steps, and each phase takes its walkers
  *                        sorted by the vertex they stand on (0..4096) */
 kk_status kk_engine_set_option(kk_engine *e, const char *name, int64_t value);
 /* Message of the last failed call on this engine ("" if none). */

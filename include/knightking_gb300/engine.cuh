@@ -703,8 +703,11 @@ inline uint32_t alias_hub_blocks(const kk_engine *e, uint32_t n)
  * resident block (a block of 256 threads takes each; more of them, and the
  * classes' own launches fill the SMs better); false: left to those.  Classes
  * against one launch, us: R-MAT 8 41 / 24, 10 43 / 37, 14 66 / 46, 16 104 / 77,
- * 18 206 / 144, 19 262 / 231, 20 434 / 517 (6,000 such rows), 21 880 / 1015; a
- * graph of 1 M vertices and 32 M edges with 200 such rows 526 / 497. */
+ * 18 206 / 144, 19 262 / 231, 20 434 / 517 (6,000 such rows), 21 880 / 1015; random
+ * graphs with 100 to 600 such rows, uniform and lognormal weights: 24 M edges 324 /
+ * 314 and 366 / 332, 32 M 399 / 395 and 460 / 427, 38 M 462 / 473 and 532 / 511, 45 M
+ * 525 / 552 and 592 / 595, 64 M 710 / 790 and 795 / 849, 96 M 1024 / 1188 and 1130 /
+ * 1278: the line lies between where the two families cross. */
 constexpr uint64_t kAliasSmallEdges = 40000000;
 
 template <typename TC, typename Bucket>
@@ -770,7 +773,8 @@ bool build_alias_small(kk_engine *e, const GraphView &g, const TC &tc, Bucket *a
 /* Builds alias tables in the Bucket layout into e->alias/e->sum for a
  * static functor: hubs on the side stream, the other classes in turn on the
  * main stream or (alias_streams) the small-row classes after the hubs on the
- * side stream and the block classes on a third, every class largest vertex first from its own counter. */
+ * side stream and the block classes on a third, every class largest vertex
+ * first from its own counter. */
 template <typename TC, typename Bucket = IndexBucket>
 void build_alias(kk_engine *e, const TC &tc)
 {

@@ -415,8 +415,8 @@ struct StreamDest
     uint64_t base = 0;
 };
 
-/* SegmentSink::before: the offsets are final (the engine's stream has been
- * synchronised), and so are the lengths, which the walk fills exactly: both
+/* SegmentSink::before: the offsets are final (the host has waited for the event
+ * behind them), and so are the lengths, which the walk fills exactly: both
  * out at once, while the walk's first segments are still walking.  s: the
  * output set whose buffers they pass through. */
 void stream_before(kk_engine *e, int s, const StreamDest &to, const uint64_t *d_off, uint32_t n)

@@ -562,13 +562,17 @@ const uint4 *cursor_adjacency_of(kk_engine *e)
 }
 
 /* Edges a sector, as a shift: an unweighted row's sectors, of eight ids, are
- * half full; a weighted row's, of four, are a quarter full from 28 M edges on,
- * where the set is far larger than L2 and a second sector costs a read of
- * memory (of one in seven lookups that find nothing at half full, of one in
- * fifty), and half full below, where the set's size counts.  Half / a quarter,
- * walk: R-MAT 16, 65536 walkers 274 / 293 us; R-MAT 19, 300007 1155 / 1159;
- * R-MAT 22, 2.4 M 7.78 / 7.37 ms; 20 jobs on 32 M edges 1.55 / 1.48; 1024
- * requests on R-MAT 24 31.9 / 29.6.  24 M edges' load with the set 3.32 / 3.41. */
+ * half full; a weighted row's, of four, are half full below 28 M edges and a
+ * quarter full from there on.  Of the lookups that find nothing one in seven
+ * needs a second sector at half full, one in fifty at a quarter; the set takes
+ * twice the memory and twice the writes.  The line lies where one walk of a
+ * million walkers at q > 1, 40 steps each, wins back what the build loses.  Half /
+ * a quarter, ms, such a walk at q 0.5, at q 3, and a load, sort and first short
+ * walk: random graphs of 13 M edges 1.35 / 1.32, 3.14 / 3.30, 1.42 / 1.44; 24 M
+ * 1.44 / 1.40, 3.91 / 3.88, 2.41 / 2.49; 27 M 1.46 / 1.42, 4.13 / 4.03, 2.67 / 2.74;
+ * 29 M 1.48 / 1.44, 4.27 / 4.15, 2.86 / 2.98; 32 M 1.51 / 1.46, 4.44 / 4.27, 3.15 / 3.30;
+ * 64 M 1.56 / 1.55, 4.92 / 4.66, 6.05 / 6.35; walks on R-MAT of 7.6 M edges 1.13 / 1.09,
+ * 2.71 / 2.62; 25.7 M 1.19 / 1.14, 3.20 / 3.00; 63.5 M 1.29 / 1.23, 3.91 / 3.59. */
 static uint32_t edge_set_shift(const kk_engine *e)
 {
     if (e->d_w == nullptr)
