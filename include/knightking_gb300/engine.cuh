@@ -1071,7 +1071,9 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
             KK_CUDA_CHECK(cudaMemsetAsync(caps + n, 0, sizeof(uint64_t), e->stream));
             /* the extension bound; a walker on an isolated start gets its one
              * vertex here, with no draws (its walk ends there at once: a bound
-             * that is exact, packed paths or not) */
+             * that is exact, packed paths or not).  Extension 0 ends a walk
+             * without a draw (src/apps/ppr.hpp:55-58): -1, which every draw is
+             * above, a draw of 0 too. */
             int resident = 0;
             KK_CUDA_CHECK(
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, constant_extension_bound_kernel, 256, 0));
@@ -1082,8 +1084,8 @@ void run_walk_with(kk_engine *e, const WC &wc, const TC &tc, const RunSpec &rs, 
             const double mean = 1.0 / (1.0 - (double)rs.const_ext + 1e-9);
             const uint32_t together = (uint32_t)(31.0 * mean / (mean + 16.0)) + 1u;
             constant_extension_bound_kernel<<<(unsigned)(n / (per * 8ull) + 1), 256, 0, e->stream>>>(
-                g, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext, 1u << 24, per,
-                together < 31u ? together : 31u, caps, d_status);
+                g, rs.d_start, rs.n_start, rs.seed, rs.walker_begin, n, rs.const_ext > 0.0f ? rs.const_ext : -1.0f,
+                1u << 24, per, together < 31u ? together : 31u, caps, d_status);
             count_launch(e);
             KK_CUDA_CHECK(cudaGetLastError());
             exclusive_scan_u64(e, caps, off, (uint64_t)n + 1);
